@@ -188,22 +188,7 @@ void place_phase1(Job& j, Carver& c) {
     j.list = c.take<long long>((size_t)j.list_cap * 8);
     j.recheck = c.take<long long>((size_t)j.list_cap * 8);
     j.ds = c.take<DevState>(sizeof(DevState));
-    j.fwn.g = fwn_grid(L, T);
-    const long long nc = j.fwn.g.cells;
-    const long long ncap = std::max<long long>(1, std::min<long long>(nc, T));
-    j.fwn.cells = c.take<FwnCell>((size_t)ncap * sizeof(FwnCell));
-    j.fwn.tri = c.take<unsigned>((size_t)T * 4);
-    j.fwn.cell_of = c.take<unsigned>((size_t)T * 4);
-    j.fwn.counts = c.take<unsigned>((size_t)nc * 4);
-    j.fwn.cursor = c.take<unsigned>((size_t)nc * 4);
-    j.fwn.flag = c.take<unsigned>((size_t)nc * 4);
-    j.fwn.off = c.take<unsigned long long>((size_t)nc * 8);
-    j.fwn.cidx = c.take<unsigned long long>((size_t)nc * 8);
-    j.fwn.scan = c.take<unsigned long long>((size_t)fwn_scan_elems(j.fwn.g) * 8);
-    j.fwn.fb = c.take<long long>((size_t)j.list_cap * 8);
-    j.fwn.fb_cap = j.list_cap;
-    void* sup = c.take<char>(fwn_super_bytes(j.fwn.g, T, j.list_cap));
-    if (sup) fwn_super_carve(j.fwn, sup, T, j.list_cap);
+    if (void* fw = c.take<char>(fwn_bytes(T, j.list_cap))) j.fwn = fwn_carve(fw, T, j.list_cap);
 }
 
 void place_phase2(Job& j, Carver& c) {
@@ -238,7 +223,7 @@ void enqueue_build(gbsdf_batch& b, Job& j, cudaStream_t st) {
     cudaMemsetAsync(j.bcur, 0, (size_t)L.nbricks * 4, st);
     cudaMemsetAsync(j.scur, 0, (size_t)L.nstrips * 4, st);
     launch_bin_fill(j.stt, j.ptt, T, L, j.boff, j.bcur, j.blist, j.soff, j.scur, j.slist, st, j.ds, j.cap_b, j.cap_s);
-    launch_fwn_build(j.t9, T, L, j.fwn, j.ds, st);
+    launch_fwn_build(j.t9, T, L, j.fwn, st);
     // [init] + [A]: one CTA per brick of the lattice, the surplus over the active count exits
     launch_fill(j.A, N, kFarSentinel, st);
     launch_splat(j.stt, j.boff, j.bcount, j.blist, j.active, -1, -1, L, j.A, j.ds, st);
@@ -249,15 +234,14 @@ void enqueue_build(gbsdf_batch& b, Job& j, cudaStream_t st) {
     // voxels decided exactly in E, a feature of the sign-risk model)
     const bool learned = learned_mode(b);
     if (learned) cudaMemsetAsync(j.E, 0, (size_t)L.nwords * 4, st);
-    const long long passes = std::min<long long>(64, (N + j.list_cap - 1) / j.list_cap + 1);
+    // (a lattice of at most the list's capacity cannot leave more than the list holds)
+    const long long passes = N <= j.list_cap ? 1 : std::min<long long>(64, (N + j.list_cap - 1) / j.list_cap + 1);
     auto fixup_passes = [&](uint32_t* ebits) {
         for (long long p = 0; p < passes; ++p) {
-            cudaMemsetAsync(&j.ds->listed, 0, sizeof(unsigned long long), st);
-            cudaMemsetAsync(&j.ds->list_overflow, 0, sizeof(unsigned long long), st);
-            cudaMemsetAsync(&j.ds->recheck_n, 0, sizeof(unsigned long long), st);
-            launch_list_unknown(j.U, j.S, L, j.list, j.list_cap, j.ds, 0, st, ebits);
-            launch_winding(&j.fwn, j.t9, T, L, j.list, j.list_cap, kGwnFixup, 0, j.S, j.recheck, j.list_cap, j.A, 0,
-                           stol, j.ds, b.num_sms, st);
+            cudaMemsetAsync(&j.ds->listed, 0, kPassCounters, st);
+            launch_list_blocks(j.U, L, j.list, j.list_cap, j.ds, 0, st);
+            launch_winding_blocks(j.fwn, j.t9, T, L, j.U, j.S, ebits, j.list, j.list_cap, 0, j.recheck, j.list_cap,
+                                  j.A, 0, stol, j.ds, b.num_sms, st);
             launch_gwn_recheck(j.t9, T, L, j.recheck, j.list_cap, kGwnFixup, j.S, j.ds, b.num_sms, st);
         }
     };
@@ -291,9 +275,9 @@ void enqueue_build(gbsdf_batch& b, Job& j, cudaStream_t st) {
         launch_verify_plan(gen, j.ds, st, learned ? 1 : 0);
         if (gen == kProbeGens - 1) break;
         launch_patch_mark(L, j.U, j.ds, st);
-        launch_list_unknown(j.U, j.S, L, j.list, j.list_cap, j.ds, 1, st, learned ? j.E : nullptr);
-        launch_winding(&j.fwn, j.t9, T, L, j.list, j.list_cap, kGwnFixup, 1, j.S, j.recheck, j.list_cap, j.A, 0,
-                       stol, j.ds, b.num_sms, st);
+        launch_list_blocks(j.U, L, j.list, j.list_cap, j.ds, 1, st);
+        launch_winding_blocks(j.fwn, j.t9, T, L, j.U, j.S, learned ? j.E : nullptr, j.list, j.list_cap, 1, j.recheck,
+                              j.list_cap, j.A, 0, stol, j.ds, b.num_sms, st);
         launch_gwn_recheck(j.t9, T, L, j.recheck, j.list_cap, kGwnFixup, j.S, j.ds, b.num_sms, st);
     }
     // learned mode, as in the single-mesh path: the signed-crossing pass (its unknown

@@ -65,8 +65,8 @@ struct Workspace {
     cudaEvent_t ev[14] = {};
     std::mutex mu;
     Buf A, B, S, U, t12, t9, stt, ptt, bcount, bcur, boff, active, blist, scount, scur, soff, slist, scan, list,
-        recheck, hb, verts, idx, flags, fpos, S2, U2, fbase, fX, logits, opencnt, ekeys, ecnt, mparts, mlossp, phist, E, fwc, fwt, fwo, fwn, fwu, fwf, fwoff,
-        fwci, fwscan, fwfb, fws;
+        recheck, hb, verts, idx, flags, fpos, S2, U2, fbase, fX, logits, opencnt, ekeys, ecnt, mparts, mlossp, phist, E, fw, etab,
+        caps, cfw, cross;
     DevState* ds = nullptr;
     DevState* hs = nullptr;  // pinned host mirror
 };
@@ -164,7 +164,7 @@ void free_ws(Workspace& w) {
                    &w.active, &w.blist, &w.scount, &w.scur, &w.soff, &w.slist, &w.scan, &w.list, &w.recheck,
                    &w.hb, &w.verts, &w.idx, &w.flags, &w.fpos, &w.S2, &w.U2, &w.fbase, &w.fX, &w.logits,
                    &w.opencnt, &w.ekeys, &w.ecnt, &w.mparts, &w.mlossp, &w.phist, &w.E,
-                   &w.fwc, &w.fwt, &w.fwo, &w.fwn, &w.fwu, &w.fwf, &w.fwoff, &w.fwci, &w.fwscan, &w.fwfb, &w.fws};
+                   &w.fw, &w.etab, &w.caps, &w.cfw, &w.cross};
     for (Buf* b : bufs) {
         if (b->p) cudaFree(b->p);
         *b = Buf{};
@@ -197,54 +197,84 @@ constexpr long long kListCap = 8ll * 1024 * 1024;  // >= 64 patch boxes of 49^3 
 // Clusters of the hierarchical winding evaluation for the packed triangles (w.t9).
 int build_fwn(Workspace& w, const Lattice& L, long long T, Fwn& f, Err& e) {
     cudaStream_t st = w.st;
-    const FwnGrid g = fwn_grid(L, T);
-    const long long ncap = std::max<long long>(1, std::min<long long>(g.cells, T));
-    GB_CK(ensure(w.fwc, (size_t)ncap * sizeof(FwnCell)));
-    GB_CK(ensure(w.fwt, (size_t)T * 4));
-    GB_CK(ensure(w.fwo, (size_t)T * 4));
-    GB_CK(ensure(w.fwn, (size_t)g.cells * 4));
-    GB_CK(ensure(w.fwu, (size_t)g.cells * 4));
-    GB_CK(ensure(w.fwf, (size_t)g.cells * 4));
-    GB_CK(ensure(w.fwoff, (size_t)g.cells * 8));
-    GB_CK(ensure(w.fwci, (size_t)g.cells * 8));
-    GB_CK(ensure(w.fwscan, (size_t)fwn_scan_elems(g) * 8));
-    GB_CK(ensure(w.fwfb, (size_t)kListCap * 8));
-    f = Fwn{g, P<FwnCell>(w.fwc), P<unsigned>(w.fwt), P<unsigned>(w.fwo), P<unsigned>(w.fwn), P<unsigned>(w.fwu),
-            P<unsigned>(w.fwf), P<unsigned long long>(w.fwoff), P<unsigned long long>(w.fwci),
-            P<unsigned long long>(w.fwscan), P<long long>(w.fwfb), kListCap};
-    GB_CK(ensure(w.fws, fwn_super_bytes(g, T, kListCap)));
-    fwn_super_carve(f, w.fws.p, T, kListCap);
-    launch_fwn_build(P<float>(w.t9), T, L, f, w.ds, st);
+    GB_CK(ensure(w.fw, fwn_bytes(T, kListCap)));
+    f = fwn_carve(w.fw.p, T, kListCap);
+    launch_fwn_build(P<float>(w.t9), T, L, f, st);
     GB_CK(cudaGetLastError());
     return GBSDF_OK;
 }
 
-int fixup_unknown(Workspace& w, const Lattice& L, long long T, float stol, Err& e, uint32_t* ebits = nullptr,
-                  const Fwn* fwn = nullptr) {
+// The crossings and caps of one build, made when a pass first has enough marked voxels.
+struct Capped {
+    bool tried = false, on = false;
+    long long B = 0;
+    Fwn f{};
+    Crossings x{};
+};
+
+// The integer grid is w.B, which holds nothing while winding numbers are decided. Meshes whose
+// boundary is long (unwelded soups: more than one unmatched edge for every four triangles) keep
+// to the clusters of the mesh: their caps would be as many as its triangles. So does a build
+// that finds no memory for the table.
+int make_capped(Workspace& w, const Lattice& L, long long T, Capped& c, Err& e) {
+    cudaStream_t st = w.st;
+    c.tried = true;
+    if (T > (1ll << 26)) return GBSDF_OK;  // the table is 12 bytes a slot, over six slots a triangle
+    if (ensure(w.etab, edge_table_bytes(T)) != cudaSuccess) return GBSDF_OK;
+    launch_edge_table(P<float>(w.t9), T, w.etab.p, st);
+    unsigned long long counts[2] = {0, 0};
+    GB_CK(cudaMemcpyAsync(counts, w.etab.p, sizeof(counts), cudaMemcpyDeviceToHost, st));
+    GB_CK(cudaStreamSynchronize(st));
+    c.B = (long long)counts[0];
+    if (counts[1] || c.B > T / 4) return GBSDF_OK;
+    const float* caps9 = nullptr;
+    if (c.B > 0) {
+        if (ensure(w.caps, caps_bytes(c.B)) != cudaSuccess || ensure(w.cfw, fwn_bytes(c.B, 1)) != cudaSuccess)
+            return GBSDF_OK;
+        caps9 = launch_caps(P<float>(w.t9), T, w.etab.p, c.B, w.caps.p, st);
+        c.f = fwn_carve(w.cfw.p, c.B, 1);
+        launch_fwn_build(caps9, c.B, L, c.f, st);
+    }
+    if (ensure(w.cross, crossing_bytes(L)) != cudaSuccess) return GBSDF_OK;
+    c.x = launch_crossings(P<float>(w.t9), T, caps9, c.B, L, P<int>(w.B), w.cross.p, st);
+    GB_CK(cudaGetLastError());
+    c.on = true;
+    return GBSDF_OK;
+}
+
+int fixup_unknown(Workspace& w, const Lattice& L, long long T, float stol, Err& e, uint32_t* ebits, const Fwn* fwn,
+                  Capped& cap, int dist_sq = 0) {
+    const float* dist = P<float>(w.A);
     cudaStream_t st = w.st;
     for (int pass = 0; pass < 1 << 20; ++pass) {
-        GB_CK(cudaMemsetAsync(&w.ds->listed, 0, sizeof(unsigned long long), st));
-        GB_CK(cudaMemsetAsync(&w.ds->list_overflow, 0, sizeof(unsigned long long), st));
-        GB_CK(cudaMemsetAsync(&w.ds->recheck_n, 0, sizeof(unsigned long long), st));
-        launch_list_unknown(P<uint32_t>(w.U), P<uint32_t>(w.S), L, P<long long>(w.list), kListCap, w.ds, 0, st,
-                            ebits);
+        GB_CK(cudaMemsetAsync(&w.ds->listed, 0, kPassCounters, st));
+        if (fwn) launch_list_blocks(P<uint32_t>(w.U), L, P<long long>(w.list), kListCap, w.ds, 0, st);
+        else launch_list_unknown(P<uint32_t>(w.U), P<uint32_t>(w.S), L, P<long long>(w.list), kListCap, w.ds, 0, st,
+                                 ebits);
         GB_CK(cudaMemcpyAsync(w.hs, w.ds, sizeof(DevState), cudaMemcpyDeviceToHost, st));
         GB_CK(cudaStreamSynchronize(st));
         long long n = std::min<long long>((long long)w.hs->listed, kListCap);
         if (n <= 0) return GBSDF_OK;
+        if (fwn && !cap.tried && w.hs->listed_voxels >= (unsigned long long)kCapsMinVoxels)
+            if (int rcc = make_capped(w, L, T, cap, e)) return rcc;
+        if (fwn && cap.on)
+            launch_capped_blocks(cap.f, cap.B, L, cap.x, P<uint32_t>(w.U), P<uint32_t>(w.S), ebits,
+                                 P<long long>(w.list), kListCap, dist, dist_sq, stol, w.ds, w.num_sms, st);
         if (fwn)
-            launch_winding(fwn, P<float>(w.t9), T, L, P<long long>(w.list), kListCap, kGwnFixup, 0, P<uint32_t>(w.S),
-                           P<long long>(w.recheck), kListCap, P<float>(w.A), 0, stol, w.ds, w.num_sms, st);
+            launch_winding_blocks(*fwn, P<float>(w.t9), T, L, P<uint32_t>(w.U), P<uint32_t>(w.S), ebits,
+                                  P<long long>(w.list), kListCap, 0, P<long long>(w.recheck), kListCap, dist, dist_sq,
+                                  stol, w.ds, w.num_sms, st);
         else if (n < 64 * 1024)
             launch_gwn_small(P<float>(w.t9), T, L, P<long long>(w.list), kListCap, kGwnFixup, P<uint32_t>(w.S),
-                             P<long long>(w.recheck), kListCap, P<float>(w.A), 0, stol, w.ds, n, st);
+                             P<long long>(w.recheck), kListCap, dist, dist_sq, stol, w.ds, n, st);
         else
             launch_gwn(P<float>(w.t9), T, L, P<long long>(w.list), kListCap, kGwnFixup, 0, P<uint32_t>(w.S),
-                       P<long long>(w.recheck), kListCap, P<float>(w.A), 0, stol, w.ds, w.num_sms, st);
+                       P<long long>(w.recheck), kListCap, dist, dist_sq, stol, w.ds, w.num_sms, st);
         launch_gwn_recheck(P<float>(w.t9), T, L, P<long long>(w.recheck), kListCap, kGwnFixup, P<uint32_t>(w.S),
                            w.ds, w.num_sms, st);
         GB_CK(cudaGetLastError());
-        if (w.hs->list_overflow == 0) return GBSDF_OK;
+        // blocks: the leftovers of a pass can outgrow their list too (their voxels stay marked)
+        if (w.hs->list_overflow == 0 && (!fwn || w.hs->listed_voxels <= (unsigned long long)kListCap)) return GBSDF_OK;
     }
     return e.set(GBSDF_ECUDA, "unknown-voxel fixup did not drain");
 }
@@ -425,7 +455,8 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
     }
     GB_CK(cudaEventRecord(w.ev[4], st));
     // ---- [C]
-    int rc = fixup_unknown(w, L, T, stol, e, ebits, fwn);
+    Capped cap;
+    int rc = fixup_unknown(w, L, T, stol, e, ebits, fwn, cap);
     if (rc != GBSDF_OK) return rc;
     GB_CK(cudaEventRecord(w.ev[5], st));
     // ---- [D]
@@ -529,10 +560,17 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
         launch_verify_plan(gen, w.ds, st, learned ? 1 : 0);
         if (gen == kProbeGens - 1) break;  // the last generation never patches
         launch_patch_mark(L, P<uint32_t>(w.U), w.ds, st);
-        launch_list_unknown(P<uint32_t>(w.U), P<uint32_t>(w.S), L, P<long long>(w.list), kListCap, w.ds, 1, st,
-                            ebits);
-        launch_winding(fwn, P<float>(w.t9), T, L, P<long long>(w.list), kListCap, kGwnFixup, 1, P<uint32_t>(w.S),
+        if (fwn) {
+            launch_list_blocks(P<uint32_t>(w.U), L, P<long long>(w.list), kListCap, w.ds, 1, st);
+            launch_winding_blocks(*fwn, P<float>(w.t9), T, L, P<uint32_t>(w.U), P<uint32_t>(w.S), ebits,
+                                  P<long long>(w.list), kListCap, 1, P<long long>(w.recheck), kListCap, P<float>(w.A),
+                                  0, stol, w.ds, w.num_sms, st);
+        } else {
+            launch_list_unknown(P<uint32_t>(w.U), P<uint32_t>(w.S), L, P<long long>(w.list), kListCap, w.ds, 1, st,
+                                ebits);
+            launch_gwn(P<float>(w.t9), T, L, P<long long>(w.list), kListCap, kGwnFixup, 1, P<uint32_t>(w.S),
                        P<long long>(w.recheck), kListCap, P<float>(w.A), 0, stol, w.ds, w.num_sms, st);
+        }
         launch_gwn_recheck(P<float>(w.t9), T, L, P<long long>(w.recheck), kListCap, kGwnFixup, P<uint32_t>(w.S),
                            w.ds, w.num_sms, st);
     }
@@ -549,7 +587,7 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
             launch_escalate(w.ds, P<uint32_t>(w.S), P<uint32_t>(w.U), P<uint32_t>(w.S2), P<uint32_t>(w.U2), L,
                             w.num_sms, st);
             GB_CK(cudaGetLastError());
-            int rce = fixup_unknown(w, L, T, stol, e, ebits, fwn);
+            int rce = fixup_unknown(w, L, T, stol, e, ebits, fwn, cap);
             if (rce != GBSDF_OK) return rce;
         }
         int rcf = brick_features(w, T, L, e);
@@ -573,7 +611,7 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
         GB_CK(ensure(w.phist, (size_t)kPropBins * 4));
         launch_propose_dev(logits, L, lthr, budget, P<unsigned>(w.phist), w.ds, P<uint32_t>(w.U), st);
         GB_CK(cudaGetLastError());
-        int rcp = fixup_unknown(w, L, T, stol, e, nullptr, fwn);
+        int rcp = fixup_unknown(w, L, T, stol, e, nullptr, fwn, cap);
         if (rcp != GBSDF_OK) return rcp;
     }
     GB_CK(cudaEventRecord(w.ev[7], st));
@@ -667,18 +705,17 @@ int run_legacy(Workspace& w, long long T, const Lattice& L, float* out, bool out
     GB_CK(ensure(w.B, (size_t)N * 4));
     GB_CK(ensure(w.S, (size_t)L.nwords * 4));
     GB_CK(ensure(w.t9, (size_t)T * 36));
-    GB_CK(ensure(w.hb, (size_t)ntiles * 24));
     GB_CK(ensure(w.list, (size_t)kListCap * 8));
     GB_CK(ensure(w.recheck, (size_t)kListCap * 8));
     GB_CK(cudaMemsetAsync(w.ds, 0, sizeof(DevState), st));
     GB_CK(cudaMemsetAsync(w.S.p, 0, (size_t)L.nwords * 4, st));
     launch_pack_tri9(P<float>(w.t12), T, P<float>(w.t9), st);
+    GB_CK(ensure(w.hb, (size_t)ntiles * 24));
     launch_tile_bounds(P<float>(w.t12), T, P<float>(w.hb), st);
     GB_CK(cudaEventRecord(w.ev[2], st));
     launch_legacy_dist(P<float>(w.t9), T, P<float>(w.hb), L, P<float>(w.A), st);
     GB_CK(cudaGetLastError());
     GB_CK(cudaEventRecord(w.ev[3], st));
-    // exact winding sign of every voxel, in list-sized chunks
     Fwn fwn_s{};
     const Fwn* fwn = nullptr;
     if (winding_eval == 0) {
@@ -686,17 +723,25 @@ int run_legacy(Workspace& w, long long T, const Lattice& L, float* out, bool out
         if (rcw != GBSDF_OK) return rcw;
         fwn = &fwn_s;
     }
-    for (long long v0 = 0; v0 < N; v0 += kListCap) {
-        long long n = std::min(kListCap, N - v0);
-        launch_iota(P<long long>(w.list), n, v0, st);
-        unsigned long long nn = (unsigned long long)n;
-        GB_CK(cudaMemcpyAsync(&w.ds->listed, &nn, sizeof(nn), cudaMemcpyHostToDevice, st));
-        GB_CK(cudaMemsetAsync(&w.ds->recheck_n, 0, sizeof(unsigned long long), st));
-        launch_winding(fwn, P<float>(w.t9), T, L, P<long long>(w.list), kListCap, kGwnFixup, 0, P<uint32_t>(w.S),
+    // exact winding sign of every voxel
+    if (fwn) {
+        GB_CK(ensure(w.U, (size_t)L.nwords * 4));
+        GB_CK(cudaMemsetAsync(w.U.p, 0xff, (size_t)L.nwords * 4, st));
+        Capped cap;
+        if (int rcx = fixup_unknown(w, L, T, kSurfaceTolVoxels, e, nullptr, fwn, cap, 1)) return rcx;
+    } else {
+        for (long long v0 = 0; v0 < N; v0 += kListCap) {
+            long long n = std::min(kListCap, N - v0);
+            launch_iota(P<long long>(w.list), n, v0, st);
+            unsigned long long nn = (unsigned long long)n;
+            GB_CK(cudaMemcpyAsync(&w.ds->listed, &nn, sizeof(nn), cudaMemcpyHostToDevice, st));
+            GB_CK(cudaMemsetAsync(&w.ds->recheck_n, 0, sizeof(unsigned long long), st));
+            launch_gwn(P<float>(w.t9), T, L, P<long long>(w.list), kListCap, kGwnFixup, 0, P<uint32_t>(w.S),
                        P<long long>(w.recheck), kListCap, P<float>(w.A), 1, kSurfaceTolVoxels, w.ds, w.num_sms, st);
-        launch_gwn_recheck(P<float>(w.t9), T, L, P<long long>(w.recheck), kListCap, kGwnFixup, P<uint32_t>(w.S),
-                           w.ds, w.num_sms, st);
-        GB_CK(cudaStreamSynchronize(st));  // `nn` lives on the host stack
+            launch_gwn_recheck(P<float>(w.t9), T, L, P<long long>(w.recheck), kListCap, kGwnFixup, P<uint32_t>(w.S),
+                               w.ds, w.num_sms, st);
+            GB_CK(cudaStreamSynchronize(st));  // `nn` lives on the host stack
+        }
     }
     GB_CK(cudaGetLastError());
     GB_CK(cudaEventRecord(w.ev[4], st));

@@ -60,7 +60,8 @@ struct ParTri {
 };
 static_assert(sizeof(ParTri) == 80, "ParTri layout");
 
-// Pipeline state kept in device memory; read back once at the end of a build.
+// Pipeline state kept in device memory; read back once at the end of a build. The six
+// counters from `listed` to `recheck_n` are one pass's, and are cleared together.
 struct DevState {
     unsigned long long brick_pairs;    // (triangle, brick) pairs of the splat
     unsigned long long strip_pairs;    // (triangle, strip) pairs of the parity pass
@@ -76,21 +77,20 @@ struct DevState {
     unsigned long long band_err_n;     // band voxels sampled for it
     unsigned long long listed;         // voxels listed for an exact winding evaluation
     unsigned long long list_overflow;
+    unsigned long long listed_voxels;  // marked voxels of the listed blocks
+    unsigned long long fwn_left;       // voxels the blocks left to the refining query
+    unsigned long long fwn_sum;        // voxels left to the sum over every triangle
+    unsigned long long recheck_n;      // entries in the FP64 re-check list
     unsigned long long fixup_voxels;
     unsigned long long gwn_pairs;      // point-triangle solid-angle evaluations (FP32)
-    unsigned long long recheck_n;      // entries in the FP64 re-check list
     unsigned long long fp64_rechecks;  // cumulative
     unsigned long long far_residual;
     unsigned long long safe_clamped;
     unsigned long long patched_voxels;
     unsigned long long overflow;       // a list outgrew the capacity planned for it (batches)
     unsigned long long wait_timeouts;  // bounded waits (TMA tiles) that gave up
-    unsigned long long fwn_cells;      // clusters of the hierarchical winding evaluation
     unsigned long long fwn_certified;  // voxels whose side the cluster bound decided
-    unsigned long long fwn_fallback;   // voxels handed to the exact sum (current pass)
     unsigned long long fwn_fallback_total;
-    unsigned long long fwn_supers;     // super-clusters (4^3 cluster cubes) of the first stage
-    unsigned long long fwn_fallback2;  // voxels the super-cluster stage left to the cluster stage
     int changed[64];                   // per eikonal round
     int stop;                          // eikonal converged flag
     int rounds;
@@ -176,79 +176,93 @@ void launch_list_unknown(uint32_t* ubits, uint32_t* sbits, const Lattice& L, lon
 void launch_gwn(const float* tri9, long long T, const Lattice& L, const long long* list, long long list_cap,
                 int consumer, int only_if, uint32_t* sbits, long long* recheck, long long recheck_cap,
                 const float* dist, int dist_sq, float surf_tol_vox, DevState* ds, int num_sms, cudaStream_t st);
-// Persistent exact-winding pass over a device-sized list, 32 threads per voxel (any list
-// length, no host round trip); `only_if`: skip unless a patch round is in flight.
+constexpr size_t kPassCounters = 6 * sizeof(unsigned long long);
+// Persistent exact-winding pass over the DevState::fwn_sum voxels of a list, 32 threads per
+// voxel (any list length, no host round trip); `only_if`: skip unless a patch round is in flight.
 void launch_gwn_team(const float* tri9, long long T, const Lattice& L, long long* list, long long list_cap,
                      int consumer, uint32_t* sbits, long long* recheck, long long recheck_cap, const float* dist,
                      int dist_sq, float surf_tol_vox, DevState* ds, int num_sms, cudaStream_t st, int only_if = 0);
 
-// ---- hierarchical winding numbers --------------------------------------------------
-// Triangles clustered by the grid cube of their centroid; each cluster keeps its
+// ---- hierarchical winding numbers (k_fwn.cu) ----------------------------------------
+// The triangles in Hilbert order of their centroids, kFwnLeaf consecutive ones a cluster,
+// kFwnFan consecutive clusters a cluster of the next level (three levels). A cluster keeps its
 // area-weighted centroid c, area vector D = sum(a_i n_i), first moment M = sum(a_i n_i
-// (g_i - c)^T) (g_i the triangle centroids; exact for flat triangles), area A and radius r
-// (every vertex within r of c). Seen from q at distance d > beta r, with y = c - q, the
-// kernel K(x) = (x - q) / |x - q|^3 expanded to second order gives the cluster's solid
-// angle D . y / d^3 + (tr M - 3 y^T M y / d^2) / d^3 within 3 r^2 A / (d - r)^4 (the second
-// derivative of K has norm at most 6 / |x - q|^4); nearer clusters are summed exactly. A voxel whose |w| clears 0.5
-// by more than the summed bound (plus rounding slack) is decided; the others go to the
-// exact per-triangle sum. Decisions therefore equal the exact path's.
+// (g_i - c)^T) (g_i the triangle centroids; exact for flat triangles), area A, second moment
+// Q = sum of the integrals of |x - c|^2 and radius r (every vertex within r of c). Seen from
+// q at distance d > beta r, with y = c - q, the kernel K(x) = (x - q) / |x - q|^3 expanded to
+// second order gives the cluster's solid angle D . y / d^3 + (tr M - 3 y^T M y / d^2) / d^3
+// within 3 Q / (d - r)^4 (the second derivative of K has norm at most 6 / |x - q|^4; a
+// triangle by itself: M = 0 and Q = a (sum of its squared sides) / 36). A voxel whose |w|
+// clears 0.5 by more than the summed bound (plus rounding slack) is decided; the others go to
+// the exact per-triangle sum. Decisions therefore equal the exact path's.
+constexpr int kFwnLeaf = 8;   // triangles of a cluster
+constexpr int kFwnFan = 16;   // clusters of a cluster of the next level
 struct FwnCell {
     float cx, cy, cz, r;      // centroid, radius
     float ax, ay, az, area;   // area vector, area
     float m[9];               // first moment sum_t D_t,i (g_t - c)_j, row-major (i, j)
-    unsigned off, cnt, pad0;
+    float q;                  // second moment
+    float pad[2];
 };
 static_assert(sizeof(FwnCell) == 80, "FwnCell layout");
-// The cluster grid: cubes of s voxels (s = 8, halved down to 2 while the triangles would
-// average more than 16 per cube), covering the lattice; triangles are binned by centroid
-// (clamped to the grid).
-struct FwnGrid {
-    int s;
-    int n[3];
-    long long cells;
-};
-FwnGrid fwn_grid(const Lattice& L, long long T);
 struct Fwn {
-    FwnGrid g;
-    FwnCell* cells;           // capacity: min(grid cells, triangles)
-    unsigned* tri;            // triangles by cluster
-    unsigned* cell_of;        // cluster brick of each triangle
-    unsigned* counts;         // per grid cell
-    unsigned* cursor;         // per grid cell
-    unsigned* flag;           // per grid cell: non-empty
-    unsigned long long* off;  // per grid cell
-    unsigned long long* cidx; // per grid cell: cluster index
-    unsigned long long* scan; // scan scratch
-    long long* fb;            // voxels left to the exact sum
+    long long n[3];              // clusters per level: ceil(T / 8), / 16, / 16
+    FwnCell* cells[3];
+    float4* leaf;                // per triangle, Hilbert order, five float4: (g, r) (D, Q) (v0 v1 v2)
+    unsigned *key[2], *idx[2];   // the sort's ping-pong
+    unsigned *hist, *offs;       // its tile histograms and their scan
+    long long* fb;               // voxels left to the exact sum
+    long long* fb2;              // voxels left to the refining stage
     long long fb_cap;
-    // super-clusters: the clusters of each cube of 4^3 cluster cubes, with aggregated
-    // moments; a first query stage uses them for far super-clusters and hands the voxels
-    // it cannot decide to the cluster stage (fb2)
-    long long scells = 0;            // super grid cubes
-    int sn[3] = {0, 0, 0};
-    FwnCell* supers = nullptr;       // capacity: min(super cubes, clusters)
-    unsigned* sup_of = nullptr;      // per cluster: its super cube
-    unsigned* sup_counts = nullptr;  // per super cube
-    unsigned* sup_cursor = nullptr;
-    unsigned* sup_flag = nullptr;
-    unsigned long long* sup_off = nullptr;
-    unsigned long long* sup_cidx = nullptr;
-    unsigned* sup_child = nullptr;   // clusters by super cube, ascending within a cube
-    long long* fb2 = nullptr;        // voxels left to the cluster stage (capacity fb_cap)
 };
-long long fwn_scan_elems(const FwnGrid& g);
-// Bytes of the super-cluster arrays of `g` (T triangles, list capacity `cap`), and their
-// carving from one 256-byte aligned allocation into f (sets scells, sn and the pointers).
-size_t fwn_super_bytes(const FwnGrid& g, long long T, long long cap);
-void fwn_super_carve(Fwn& f, void* base, long long T, long long cap);
+// Bytes of the arrays above for T triangles and leftover lists of `cap` voxels, and their
+// carving from one 256-byte aligned allocation.
+size_t fwn_bytes(long long T, long long cap);
+Fwn fwn_carve(void* base, long long T, long long cap);
 // Builds the clusters of the packed triangles (device only, no host round trip).
-void launch_fwn_build(const float* tri9, long long T, const Lattice& L, const Fwn& f, DevState* ds, cudaStream_t st);
+void launch_fwn_build(const float* tri9, long long T, const Lattice& L, const Fwn& f, cudaStream_t st);
 // Decides the listed voxels (as launch_gwn does) by the cluster bound, then sums the rest
 // exactly; the FP64 re-check pass (launch_gwn_recheck) follows as after launch_gwn.
 void launch_winding(const Fwn* f, const float* tri9, long long T, const Lattice& L, const long long* list,
                     long long list_cap, int consumer, int only_if, uint32_t* sbits, long long* recheck,
                     long long recheck_cap, const float* dist, int dist_sq, float surf_tol_vox, DevState* ds,
                     int num_sms, cudaStream_t st);
+// Whole blocks of bricks at once. launch_list_blocks lists the blocks that hold a voxel
+// marked in U (DevState::listed; listed_voxels counts the marks); launch_winding_blocks
+// decides their marked voxels (U, S and E as launch_list_unknown treats them; a voxel that
+// finds no room in the leftover list stays marked and counts in list_overflow) and hands the
+// undecided ones to the refining stage and the exact sum. ubits null: every voxel.
+void launch_list_blocks(const uint32_t* ubits, const Lattice& L, long long* list, long long cap, DevState* ds,
+                        int only_if, cudaStream_t st);
+void launch_winding_blocks(const Fwn& f, const float* tri9, long long T, const Lattice& L, uint32_t* ubits,
+                           uint32_t* sbits, uint32_t* ebits, const long long* list, long long list_cap, int only_if,
+                           long long* recheck, long long recheck_cap, const float* dist, int dist_sq,
+                           float surf_tol_vox, DevState* ds, int num_sms, cudaStream_t st);
+// ---- winding numbers from crossings and caps (k_caps.cu) ------------------------------
+// launch_edge_table matches the mesh's edges in `table` (edge_table_bytes) and counts its
+// boundary there: [0] the unmatched edges B, [1] nonzero when a vertex is not finite.
+// launch_caps builds their B caps in `scratch` (caps_bytes) and returns them, nine floats each.
+// launch_crossings sums the crossings of mesh and caps (`grid`: an int per voxel, scratch;
+// `scratch`: crossing_bytes). launch_capped_blocks then decides what marked voxels of the listed
+// blocks it can (as launch_winding_blocks does; f: the caps' clusters) and leaves the others
+// marked.
+struct Crossings {
+    const uint32_t* k;    // the voxels with a nonzero crossing number (sign-word layout)
+    const unsigned* bad;  // the columns to leave out, a bit per column (x fastest)
+};
+constexpr long long kCapsMinVoxels = 32768;  // marked voxels from which the pass pays off
+size_t edge_table_bytes(long long T);
+void launch_edge_table(const float* tri9, long long T, void* table, cudaStream_t st);
+size_t caps_bytes(long long B);
+const float* launch_caps(const float* tri9, long long T, const void* table, long long B, void* scratch,
+                         cudaStream_t st);
+size_t crossing_bytes(const Lattice& L);
+Crossings launch_crossings(const float* tri9, long long T, const float* caps9, long long B, const Lattice& L,
+                           int* grid, void* scratch, cudaStream_t st);
+void launch_capped_blocks(const Fwn& f, long long B, const Lattice& L, const Crossings& X, uint32_t* ubits,
+                          uint32_t* sbits, uint32_t* ebits, const long long* list, long long list_cap,
+                          const float* dist, int dist_sq, float surf_tol_vox, DevState* ds, int num_sms,
+                          cudaStream_t st);
 // Batches: decides on the device whether the build passed its checks (valid triangles,
 // the reference's CSR guard when `csr_guard`, no list overflow); sets ds->abort_ if not.
 void launch_batch_finalize(DevState* ds, int csr_guard, cudaStream_t st);
