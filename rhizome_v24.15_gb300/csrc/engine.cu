@@ -710,19 +710,21 @@ int run_legacy(Workspace& w, long long T, const Lattice& L, float* out, bool out
     GB_CK(cudaMemsetAsync(w.ds, 0, sizeof(DevState), st));
     GB_CK(cudaMemsetAsync(w.S.p, 0, (size_t)L.nwords * 4, st));
     launch_pack_tri9(P<float>(w.t12), T, P<float>(w.t9), st);
-    GB_CK(ensure(w.hb, (size_t)ntiles * 24));
-    launch_tile_bounds(P<float>(w.t12), T, P<float>(w.hb), st);
-    GB_CK(cudaEventRecord(w.ev[2], st));
-    launch_legacy_dist(P<float>(w.t9), T, P<float>(w.hb), L, P<float>(w.A), st);
-    GB_CK(cudaGetLastError());
-    GB_CK(cudaEventRecord(w.ev[3], st));
     Fwn fwn_s{};
     const Fwn* fwn = nullptr;
     if (winding_eval == 0) {
         int rcw = build_fwn(w, L, T, fwn_s, e);
         if (rcw != GBSDF_OK) return rcw;
         fwn = &fwn_s;
+    } else {
+        GB_CK(ensure(w.hb, (size_t)ntiles * 24));
+        launch_tile_bounds(P<float>(w.t12), T, P<float>(w.hb), st);
     }
+    GB_CK(cudaEventRecord(w.ev[2], st));
+    if (fwn) launch_nearest(*fwn, T, L, P<float>(w.A), st);
+    else launch_legacy_dist(P<float>(w.t9), T, P<float>(w.hb), L, P<float>(w.A), st);
+    GB_CK(cudaGetLastError());
+    GB_CK(cudaEventRecord(w.ev[3], st));
     // exact winding sign of every voxel
     if (fwn) {
         GB_CK(ensure(w.U, (size_t)L.nwords * 4));

@@ -208,7 +208,8 @@ static_assert(sizeof(FwnCell) == 80, "FwnCell layout");
 struct Fwn {
     long long n[3];              // clusters per level: ceil(T / 8), / 16, / 16
     FwnCell* cells[3];
-    float4* leaf;                // per triangle, Hilbert order, five float4: (g, r) (D, Q) (v0 v1 v2)
+    float4* box[3];              // their bounding boxes, two float4 each
+    float4* leaf;                // per triangle, Hilbert order, five float4: (g, r) (D, Q) (v0 v1 v2, a^2)
     unsigned *key[2], *idx[2];   // the sort's ping-pong
     unsigned *hist, *offs;       // its tile histograms and their scan
     long long* fb;               // voxels left to the exact sum
@@ -227,6 +228,8 @@ void launch_winding(const Fwn* f, const float* tri9, long long T, const Lattice&
                     long long list_cap, int consumer, int only_if, uint32_t* sbits, long long* recheck,
                     long long recheck_cap, const float* dist, int dist_sq, float surf_tol_vox, DevState* ds,
                     int num_sms, cudaStream_t st);
+// Squared distance of every voxel to its nearest triangle (legacy path).
+void launch_nearest(const Fwn& f, long long T, const Lattice& L, float* d2, cudaStream_t st);
 // Whole blocks of bricks at once. launch_list_blocks lists the blocks that hold a voxel
 // marked in U (DevState::listed; listed_voxels counts the marks); launch_winding_blocks
 // decides their marked voxels (U, S and E as launch_list_unknown treats them; a voxel that
