@@ -130,10 +130,11 @@ typedef struct gbsdf_options {
     int32_t winding_eval;   /* exact winding decisions: 0 = clustered (far clusters by a dipole
                                with a rigorous error bound, undecided voxels summed exactly;
                                same decisions), 1 = every voxel summed triangle by triangle */
-    int32_t splat_dense_cut; /* binned triangles per 8^3 brick above which the band splat takes the
-                                brick with its sub-brick kernel: 0 = autotuned per lattice class
-                                (gbsdf_stats.splat_dense_cut reports it), > 0 = that cut.
-                                Identical results at every cut. */
+    int32_t splat_dense_cut; /* binned triangles (eight to a cluster) per 8^3 brick above which the
+                                band splat takes the brick before the others, so that the longest
+                                work starts first: 0 = 256, > 0 = that cut
+                                (gbsdf_stats.splat_dense_cut reports it). Identical results at
+                                every cut. */
 } gbsdf_options;
 
 /* Learned sign-risk model: parameter count and brick feature count. */
@@ -151,7 +152,7 @@ typedef struct gbsdf_stats {
     int32_t sites;
     int32_t patch_rounds;
     int32_t splat_dense_cut; /* binned triangles per 8^3 brick above which the band splat takes the
-                                brick with its sub-brick kernel (autotuned per lattice class) */
+                                brick first */
     int64_t unknown_columns;
     int64_t fixup_voxels;
     int64_t far_residual;
@@ -161,7 +162,7 @@ typedef struct gbsdf_stats {
     int64_t band_voxels;
     int64_t splat_evals;   /* exact point-triangle distance evaluations */
     int64_t gwn_pairs;     /* point-triangle solid-angle evaluations */
-    int64_t brick_pairs;   /* (triangle, brick) pairs binned for the splat */
+    int64_t brick_pairs;   /* (cluster of eight triangles, brick) pairs binned for the splat */
     int64_t csr_entries;   /* entries of the reference's supercell CSR */
     int64_t kernel_launches; /* CUDA kernels this call launched */
     int64_t proposed;      /* learned mode: bricks the network proposed for the exact winding number */

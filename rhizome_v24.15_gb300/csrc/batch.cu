@@ -71,11 +71,10 @@ struct Job {
     float* out = nullptr;
     Lattice L{};
     int pre_status = GBSDF_OK;  // argument checks (the mesh is left out of the graph)
-    unsigned dense_cut = kDenseCutDefault;  // the splat's tile cut: the class's tuned value if timed
+    unsigned dense_cut = kDenseCutDefault;  // gbsdf_options.splat_dense_cut or the default
     // device buffers (offsets into the arenas)
     float *A = nullptr, *B = nullptr, *t12 = nullptr, *t9 = nullptr;
     uint32_t *S = nullptr, *U = nullptr;
-    SplatTri* stt = nullptr;
     ParTri* ptt = nullptr;
     unsigned *bcount = nullptr, *bcur = nullptr, *active = nullptr, *scount = nullptr, *scur = nullptr;
     unsigned long long *boff = nullptr, *soff = nullptr, *scan = nullptr;
@@ -99,7 +98,7 @@ struct Job {
     // the open-edge table, the network's logits and the proposal histogram
     uint32_t *S2 = nullptr, *U2 = nullptr, *E = nullptr;
     float *fbase = nullptr, *fX = nullptr, *logits = nullptr;
-    unsigned *opencnt = nullptr, *ecnt = nullptr, *phist = nullptr;
+    unsigned *opencnt = nullptr, *btris = nullptr, *ecnt = nullptr, *phist = nullptr;
     unsigned long long* ekeys = nullptr;
     long long ecap = 0;
 };
@@ -158,6 +157,7 @@ void place_learned(Job& j, Carver& c) {
     j.fX = c.take<float>((size_t)L.nbricks * kMlpIn * 4);
     j.logits = c.take<float>((size_t)L.nbricks * 4);
     j.opencnt = c.take<unsigned>((size_t)L.nbricks * 4);
+    j.btris = c.take<unsigned>((size_t)L.nbricks * 4);
     j.phist = c.take<unsigned>((size_t)kPropBins * 4);
     j.ecap = edge_table_cap(j.T);
     j.ekeys = c.take<unsigned long long>((size_t)j.ecap * 8);
@@ -174,7 +174,6 @@ void place_phase1(Job& j, Carver& c) {
     j.U = c.take<uint32_t>((size_t)L.nwords * 4);
     j.t12 = c.take<float>((size_t)T * 48);
     j.t9 = c.take<float>((size_t)T * 36);
-    j.stt = c.take<SplatTri>((size_t)T * sizeof(SplatTri));
     j.ptt = c.take<ParTri>((size_t)T * sizeof(ParTri));
     j.bcount = c.take<unsigned>((size_t)L.nbricks * 4);
     j.bcur = c.take<unsigned>((size_t)L.nbricks * 4);
@@ -207,11 +206,13 @@ void enqueue_counts(gbsdf_batch& b, Job& j, cudaStream_t st) {
     cudaMemsetAsync(j.ds, 0, sizeof(DevState), st);
     cudaMemsetAsync(j.bcount, 0, (size_t)L.nbricks * 4, st);
     cudaMemsetAsync(j.scount, 0, (size_t)L.nstrips * 4, st);
-    launch_prep(j.t12, T, L, j.stt, j.ptt, j.bcount, j.scount, j.ds, st);
+    launch_prep(j.t12, T, L, j.ptt, j.scount, j.ds, st);
+    launch_pack_tri9(j.t12, T, j.t9, st);
+    launch_fwn_build(j.t9, T, L, j.fwn, st);
+    launch_brick_bins(j.fwn, T, L, j.bcount, nullptr, nullptr, j.ds, st);
     launch_exclusive_scan(j.bcount, j.boff, L.nbricks, j.scan, 0, st);
     launch_exclusive_scan(j.scount, j.soff, L.nstrips, j.scan, 0, st);
     launch_active_bricks(j.bcount, L.nbricks, j.active, j.ds, st, j.dense_cut);
-    launch_pack_tri9(j.t12, T, j.t9, st);
 }
 
 // The rest of a build, with no host round trip.
@@ -222,12 +223,12 @@ void enqueue_build(gbsdf_batch& b, Job& j, cudaStream_t st) {
     const float stol = xs ? kSurfaceTolExactSigns : kSurfaceTolVoxels;
     cudaMemsetAsync(j.bcur, 0, (size_t)L.nbricks * 4, st);
     cudaMemsetAsync(j.scur, 0, (size_t)L.nstrips * 4, st);
-    launch_bin_fill(j.stt, j.ptt, T, L, j.boff, j.bcur, j.blist, j.soff, j.scur, j.slist, st, j.ds, j.cap_b, j.cap_s);
-    launch_fwn_build(j.t9, T, L, j.fwn, st);
-    // [init] + [A]: one CTA per brick of the lattice, the surplus over the active count exits
+    launch_strip_fill(j.ptt, T, L, j.soff, j.scur, j.slist, st, j.ds, j.cap_b, j.cap_s);
+    launch_brick_bins(j.fwn, T, L, j.bcur, j.boff, j.blist, j.ds, st, j.cap_b, j.cap_s);
+    // [init] + [A]
     launch_fill(j.A, N, kFarSentinel, st);
-    launch_splat(j.stt, j.boff, j.bcount, j.blist, j.active, -1, -1, L, j.A, j.ds, st);
-    launch_band_error(j.stt, j.boff, j.bcount, j.blist, L, j.A, j.ds, st);
+    launch_splat(j.fwn, T, j.boff, j.bcount, j.blist, j.active, -1, L, j.A, j.ds, st);
+    launch_band_error(j.fwn, T, j.boff, j.bcount, j.blist, L, j.A, j.ds, st);
     // [B]
     launch_parity(j.ptt, j.soff, j.scount, j.slist, L, j.S, j.U, j.ds, xs ? 1 : 0, st);
     // [C]: enough list passes to drain every voxel of the lattice (learned mode records the
@@ -293,7 +294,9 @@ void enqueue_build(gbsdf_batch& b, Job& j, cudaStream_t st) {
         cudaMemsetAsync(j.ecnt, 0, (size_t)j.ecap * 4, st);
         cudaMemsetAsync(j.opencnt, 0, (size_t)L.nbricks * 4, st);
         launch_open_edges(j.t12, T, L, j.ekeys, j.ecnt, j.ecap, j.opencnt, st);
-        launch_brick_features(j.A, j.S, j.E, j.S2, j.U2, j.bcount, j.opencnt, L, j.fbase, j.fX, st);
+        cudaMemsetAsync(j.btris, 0, (size_t)L.nbricks * 4, st);
+        launch_brick_tris(j.t12, T, L, j.btris, st);
+        launch_brick_features(j.A, j.S, j.E, j.S2, j.U2, j.btris, j.opencnt, L, j.fbase, j.fX, st);
         launch_mlp_forward(b.mlp_params, j.fX, L.nbricks, j.logits, st);
         const unsigned budget = b.budget > 0 ? b.budget : (unsigned)std::max<long long>(1, L.nbricks / 16);
         launch_propose_dev(j.logits, L, b.logit_thr, budget, j.phist, j.ds, j.U, st);
@@ -339,8 +342,7 @@ int plan(gbsdf_batch& b, BErr& e) {
             const SweepPlan plan1 = tuned_sweep_plan(b.device, Lp, j.A, j.B, &j.map_a, j.ds, b.origin, false, 1);
             j.xsched = plan.x;
             j.wsched = plan.w;
-            if (const unsigned cut = b.dense_cut > 0 ? (unsigned)b.dense_cut : tuned_dense_cut(b.device, j.L, j.T))
-                j.dense_cut = cut;
+            if (b.dense_cut > 0) j.dense_cut = (unsigned)b.dense_cut;
             j.xsched1 = plan1.x;
             j.wsched1 = plan1.w;
             const int xs_opt = b.sweep_schedule % 10, ws_opt = b.sweep_schedule / 10;

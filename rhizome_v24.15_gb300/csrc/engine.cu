@@ -64,7 +64,7 @@ struct Workspace {
     cudaStream_t st = nullptr;
     cudaEvent_t ev[14] = {};
     std::mutex mu;
-    Buf A, B, S, U, t12, t9, stt, ptt, bcount, bcur, boff, active, blist, scount, scur, soff, slist, scan, list,
+    Buf A, B, S, U, t12, t9, ptt, btris, bcount, bcur, boff, active, blist, scount, scur, soff, slist, scan, list,
         recheck, hb, verts, idx, flags, fpos, S2, U2, fbase, fX, logits, opencnt, ekeys, ecnt, mparts, mlossp, phist, E, fw, etab,
         caps, cfw, cross;
     DevState* ds = nullptr;
@@ -160,7 +160,7 @@ int init_ws(Workspace& w, int device, Err& e) {
 void free_ws(Workspace& w) {
     if (w.device < 0) return;
     cudaSetDevice(w.device);
-    Buf* bufs[] = {&w.A, &w.B, &w.S, &w.U, &w.t12, &w.t9, &w.stt, &w.ptt, &w.bcount, &w.bcur, &w.boff,
+    Buf* bufs[] = {&w.A, &w.B, &w.S, &w.U, &w.t12, &w.t9, &w.ptt, &w.btris, &w.bcount, &w.bcur, &w.boff,
                    &w.active, &w.blist, &w.scount, &w.scur, &w.soff, &w.slist, &w.scan, &w.list, &w.recheck,
                    &w.hb, &w.verts, &w.idx, &w.flags, &w.fpos, &w.S2, &w.U2, &w.fbase, &w.fX, &w.logits,
                    &w.opencnt, &w.ekeys, &w.ecnt, &w.mparts, &w.mlossp, &w.phist, &w.E,
@@ -310,10 +310,13 @@ int brick_features(Workspace& w, long long T, const Lattice& L, Err& e) {
     GB_CK(cudaMemsetAsync(w.ekeys.p, 0, (size_t)cap * 8, st));
     GB_CK(cudaMemsetAsync(w.ecnt.p, 0, (size_t)cap * 4, st));
     GB_CK(cudaMemsetAsync(w.opencnt.p, 0, (size_t)L.nbricks * 4, st));
+    GB_CK(ensure(w.btris, (size_t)L.nbricks * 4));
+    GB_CK(cudaMemsetAsync(w.btris.p, 0, (size_t)L.nbricks * 4, st));
+    launch_brick_tris(P<float>(w.t12), T, L, P<unsigned>(w.btris), st);
     launch_open_edges(P<float>(w.t12), T, L, P<unsigned long long>(w.ekeys), P<unsigned>(w.ecnt), cap,
                       P<unsigned>(w.opencnt), st);
     launch_brick_features(P<float>(w.A), P<uint32_t>(w.S), P<uint32_t>(w.E), P<uint32_t>(w.S2), P<uint32_t>(w.U2),
-                          P<unsigned>(w.bcount), P<unsigned>(w.opencnt), L, P<float>(w.fbase), P<float>(w.fX), st);
+                          P<unsigned>(w.btris), P<unsigned>(w.opencnt), L, P<float>(w.fbase), P<float>(w.fX), st);
     GB_CK(cudaGetLastError());
     return GBSDF_OK;
 }
@@ -333,7 +336,6 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
     GB_CK(ensure(w.S, (size_t)L.nwords * 4));
     GB_CK(ensure(w.U, (size_t)L.nwords * 4));
     GB_CK(ensure(w.t9, (size_t)T * 36));
-    GB_CK(ensure(w.stt, (size_t)T * sizeof(SplatTri)));
     GB_CK(ensure(w.ptt, (size_t)T * sizeof(ParTri)));
     GB_CK(ensure(w.bcount, (size_t)L.nbricks * 4));
     GB_CK(ensure(w.bcur, (size_t)L.nbricks * 4));
@@ -355,17 +357,18 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
     }
     GB_CK(cudaMemsetAsync(w.bcount.p, 0, (size_t)L.nbricks * 4, st));
     GB_CK(cudaMemsetAsync(w.scount.p, 0, (size_t)L.nstrips * 4, st));
-    launch_prep(P<float>(w.t12), T, L, P<SplatTri>(w.stt), P<ParTri>(w.ptt), P<unsigned>(w.bcount),
-                P<unsigned>(w.scount), w.ds, st);
+    launch_prep(P<float>(w.t12), T, L, P<ParTri>(w.ptt), P<unsigned>(w.scount), w.ds, st);
+    launch_pack_tri9(P<float>(w.t12), T, P<float>(w.t9), st);
+    Fwn clusters{};
+    if (int rcw = build_fwn(w, L, T, clusters, e)) return rcw;
+    const Fwn* fwn = (o.winding_eval == 0) ? &clusters : nullptr;
+    launch_brick_bins(clusters, T, L, P<unsigned>(w.bcount), nullptr, nullptr, w.ds, st);
     launch_exclusive_scan(P<unsigned>(w.bcount), P<unsigned long long>(w.boff), L.nbricks,
                           P<unsigned long long>(w.scan), 0, st);
     launch_exclusive_scan(P<unsigned>(w.scount), P<unsigned long long>(w.soff), L.nstrips,
                           P<unsigned long long>(w.scan), 0, st);
-    // the splat's tile cut: the class's tuned value, else the default (and timed below)
-    const unsigned cut_known = o.splat_dense_cut > 0 ? (unsigned)o.splat_dense_cut : tuned_dense_cut(w.device, L, T);
-    unsigned dense_cut = cut_known ? cut_known : kDenseCutDefault;
+    const unsigned dense_cut = o.splat_dense_cut > 0 ? (unsigned)o.splat_dense_cut : kDenseCutDefault;
     launch_active_bricks(P<unsigned>(w.bcount), L.nbricks, P<unsigned>(w.active), w.ds, st, dense_cut);
-    launch_pack_tri9(P<float>(w.t12), T, P<float>(w.t9), st);
     GB_CK(cudaGetLastError());
     GB_CK(cudaMemcpyAsync(w.hs, w.ds, sizeof(DevState), cudaMemcpyDeviceToHost, st));
     GB_CK(cudaStreamSynchronize(st));
@@ -378,65 +381,21 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
                      (unsigned long long)w.hs->csr_entries);
     const long long brick_pairs = (long long)w.hs->brick_pairs;
     const long long strip_pairs = (long long)w.hs->strip_pairs;
-    long long n_active = (long long)w.hs->active_bricks;
-    long long n_dense = (long long)w.hs->dense_bricks;
+    const long long n_bricks = (long long)(w.hs->active_bricks + w.hs->dense_bricks);
     GB_CK(ensure(w.blist, (size_t)std::max<long long>(brick_pairs, 1) * 4));
     GB_CK(ensure(w.slist, (size_t)std::max<long long>(strip_pairs, 1) * 4));
-    Fwn fwn_s{};
-    const Fwn* fwn = nullptr;
-    if (o.winding_eval == 0) {
-        int rcw = build_fwn(w, L, T, fwn_s, e);
-        if (rcw != GBSDF_OK) return rcw;
-        fwn = &fwn_s;
-    }
     GB_CK(cudaMemsetAsync(w.bcur.p, 0, (size_t)L.nbricks * 4, st));
     GB_CK(cudaMemsetAsync(w.scur.p, 0, (size_t)L.nstrips * 4, st));
-    launch_bin_fill(P<SplatTri>(w.stt), P<ParTri>(w.ptt), T, L, P<unsigned long long>(w.boff), P<unsigned>(w.bcur),
-                    P<unsigned>(w.blist), P<unsigned long long>(w.soff), P<unsigned>(w.scur), P<unsigned>(w.slist),
-                    st);
-    if (!cut_known && o.sweep_schedule == 0) {
-        // the class's first autotuned build: time the splat stage at each candidate cut on
-        // this build's own lists (identical results at every cut), keep the fastest
-        auto split = [&](unsigned cut) -> int {
-            GB_CK(cudaMemsetAsync(&w.ds->active_bricks, 0, 2 * sizeof(unsigned long long), st));
-            launch_active_bricks(P<unsigned>(w.bcount), L.nbricks, P<unsigned>(w.active), w.ds, st, cut);
-            GB_CK(cudaMemcpyAsync(&w.hs->active_bricks, &w.ds->active_bricks, 2 * sizeof(unsigned long long),
-                                  cudaMemcpyDeviceToHost, st));
-            GB_CK(cudaStreamSynchronize(st));
-            n_active = (long long)w.hs->active_bricks;
-            n_dense = (long long)w.hs->dense_bricks;
-            return (int)GBSDF_OK;
-        };
-        float best_ms = 1e30f;
-        unsigned best = dense_cut;
-        for (unsigned cut : {128u, 256u, 512u, 1024u}) {
-            if (int rcs = split(cut)) return rcs;
-            launch_fill(P<float>(w.A), N, kFarSentinel, st);
-            GB_CK(cudaEventRecord(w.ev[10], st));  // events 10 and 11: the tuner's own
-            launch_splat(P<SplatTri>(w.stt), P<unsigned long long>(w.boff), P<unsigned>(w.bcount),
-                         P<unsigned>(w.blist), P<unsigned>(w.active), n_active, n_dense, L, P<float>(w.A), w.ds, st);
-            GB_CK(cudaEventRecord(w.ev[11], st));
-            GB_CK(cudaEventSynchronize(w.ev[11]));
-            float ms = 0.0f;
-            GB_CK(cudaEventElapsedTime(&ms, w.ev[10], w.ev[11]));
-            if (ms < best_ms) {
-                best_ms = ms;
-                best = cut;
-            }
-        }
-        set_tuned_dense_cut(w.device, L, T, best);
-        dense_cut = best;
-        if (int rcs = split(best)) return rcs;
-        // the timed splats counted into the build's statistics: start them again
-        GB_CK(cudaMemsetAsync(&w.ds->band_voxels, 0, sizeof(unsigned long long), st));
-        GB_CK(cudaMemsetAsync(&w.ds->splat_evals, 0, sizeof(unsigned long long), st));
-    }
+    launch_brick_bins(clusters, T, L, P<unsigned>(w.bcur), P<unsigned long long>(w.boff), P<unsigned>(w.blist), w.ds,
+                      st);
+    launch_strip_fill(P<ParTri>(w.ptt), T, L, P<unsigned long long>(w.soff), P<unsigned>(w.scur), P<unsigned>(w.slist),
+                      st);
     GB_CK(cudaEventRecord(w.ev[2], st));
     // ---- [init] + [A]
     launch_fill(P<float>(w.A), N, kFarSentinel, st);
-    launch_splat(P<SplatTri>(w.stt), P<unsigned long long>(w.boff), P<unsigned>(w.bcount), P<unsigned>(w.blist),
-                 P<unsigned>(w.active), n_active, n_dense, L, P<float>(w.A), w.ds, st);
-    launch_band_error(P<SplatTri>(w.stt), P<unsigned long long>(w.boff), P<unsigned>(w.bcount), P<unsigned>(w.blist), L,
+    launch_splat(clusters, T, P<unsigned long long>(w.boff), P<unsigned>(w.bcount), P<unsigned>(w.blist),
+                 P<unsigned>(w.active), n_bricks, L, P<float>(w.A), w.ds, st);
+    launch_band_error(clusters, T, P<unsigned long long>(w.boff), P<unsigned>(w.bcount), P<unsigned>(w.blist), L,
                       P<float>(w.A), w.ds, st);
     GB_CK(cudaGetLastError());
     GB_CK(cudaEventRecord(w.ev[3], st));

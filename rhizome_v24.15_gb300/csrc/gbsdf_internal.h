@@ -39,18 +39,6 @@ inline Lattice padded(const Lattice& L) {
 }
 inline long long padded_voxels(const Lattice& L) { return (long long)padded_pitch(L.dims[0]) * L.dims[1] * L.dims[2]; }
 
-// Per-triangle record of the band splat (96 bytes): vertices, AABB, the
-// reference's clamped XY footprint and a conservative z range.
-struct SplatTri {
-    float v[9];
-    float bb[6];  // tx0, tx1, ty0, ty1, tz0, tz1
-    int fx0, fx1, fy0, fy1;
-    int z0, z1;
-    int valid;
-    int pad[2];
-};
-static_assert(sizeof(SplatTri) == 96, "SplatTri layout");
-
 // Per-triangle record of the parity pass (80 bytes).
 struct ParTri {
     float xyab[4];  // minx, miny, maxx, maxy
@@ -63,7 +51,7 @@ static_assert(sizeof(ParTri) == 80, "ParTri layout");
 // Pipeline state kept in device memory; read back once at the end of a build. The six
 // counters from `listed` to `recheck_n` are one pass's, and are cleared together.
 struct DevState {
-    unsigned long long brick_pairs;    // (triangle, brick) pairs of the splat
+    unsigned long long brick_pairs;    // (cluster, brick) pairs of the splat
     unsigned long long strip_pairs;    // (triangle, strip) pairs of the parity pass
     unsigned long long csr_entries;    // entries of the reference's supercell CSR (guard)
     unsigned long long invalid_tris;   // non-finite or out-of-range coordinates
@@ -125,45 +113,45 @@ unsigned long long& launch_counter();
 #define GBSDF_COUNT_LAUNCH() (++::gbsdf::launch_counter())
 
 // ---- launchers (each enqueues on `st`) ------------------------------------------
-void launch_prep(const float* tris12, long long T, const Lattice& L, SplatTri* st_out, ParTri* pt_out,
-                 unsigned* brick_count, unsigned* strip_count, DevState* ds, cudaStream_t st);
+void launch_prep(const float* tris12, long long T, const Lattice& L, ParTri* pt_out, unsigned* strip_count,
+                 DevState* ds, cudaStream_t st);
 void launch_exclusive_scan(const unsigned* in, unsigned long long* out, long long n, unsigned long long* tmp,
                            long long tmp_elems, cudaStream_t st);
 long long scan_tmp_elems(long long n);
 // Frees the iso-surface extractor's cached scratch of `device` (k_iso.cu).
 void release_iso_workspace(int device);
 // With `ds`, the pair lists are known to hold `cap_b` / `cap_s` entries: when the counts
-// of this SDF build exceed them the fill writes nothing and sets ds->overflow (the splat and
+// of this SDF build exceed them the fills write nothing and ds->overflow is set (the splat and
 // parity passes then skip the build).
-void launch_bin_fill(const SplatTri* stt, const ParTri* ptt, long long T, const Lattice& L,
-                     const unsigned long long* brick_off, unsigned* brick_cur, unsigned* brick_list,
-                     const unsigned long long* strip_off, unsigned* strip_cur, unsigned* strip_list,
-                     cudaStream_t st, DevState* ds = nullptr, unsigned long long cap_b = ~0ull,
-                     unsigned long long cap_s = ~0ull);
-// The bricks with binned triangles: those with at most `dense_cut` from the front of
-// `active` (DevState::active_bricks), the others from the back (DevState::dense_bricks).
+void launch_strip_fill(const ParTri* ptt, long long T, const Lattice& L, const unsigned long long* strip_off,
+                       unsigned* strip_cur, unsigned* strip_list, cudaStream_t st, DevState* ds = nullptr,
+                       unsigned long long cap_b = ~0ull, unsigned long long cap_s = ~0ull);
+struct Fwn;
+// The clusters whose band can touch each brick: counts (list null; DevState::brick_pairs in all),
+// or the lists, `count` being the cursor then.
+void launch_brick_bins(const Fwn& f, long long T, const Lattice& L, unsigned* count, const unsigned long long* off,
+                       unsigned* list, DevState* ds, cudaStream_t st, unsigned long long cap_b = ~0ull,
+                       unsigned long long cap_s = ~0ull);
+// Triangles per brick (a feature of the sign-risk model).
+void launch_brick_tris(const float* tris12, long long T, const Lattice& L, unsigned* count, cudaStream_t st);
+// The bricks with binned clusters: those of more than `dense_cut` triangles from the back of
+// `active` (DevState::dense_bricks; the splat takes them first), the others from the front
+// (DevState::active_bricks).
 constexpr unsigned kDenseCutDefault = 256;
 void launch_active_bricks(const unsigned* brick_count, long long nbricks, unsigned* active, DevState* ds,
                           cudaStream_t st, unsigned dense_cut);
-// The splat's tile cut of a lattice class (device, voxels, triangles; by octave): 0 when not
-// yet timed. The first fast-path build of a class times the candidates (engine.cu).
-unsigned tuned_dense_cut(int device, const Lattice& L, long long T);
-void set_tuned_dense_cut(int device, const Lattice& L, long long T, unsigned cut);
 void launch_fill(float* g, long long n, float value, cudaStream_t st);
-// n_active < 0: the active-brick count is read on the device (one CTA per brick of the
-// lattice is launched and the surplus exits), so the launch needs no host round trip.
 // The band splat's error against FP64: kBandErrSamples voxels, one per equal stratum of
 // the lattice at a fixed golden-ratio offset; those in the band (splat value <= 8h) get the FP64 distance to their
-// brick's binned triangles (the splat's own candidates) and the largest difference, in
+// brick's binned clusters' triangles (the splat's own candidates) and the largest difference, in
 // voxels, goes to DevState::band_err_bits / band_err_n.
 constexpr long long kBandErrSamples = 16384;
-void launch_band_error(const SplatTri* stt, const unsigned long long* brick_off, const unsigned* brick_count,
+void launch_band_error(const Fwn& f, long long T, const unsigned long long* brick_off, const unsigned* brick_count,
                        const unsigned* brick_list, const Lattice& L, const float* dist, DevState* ds, cudaStream_t st);
-// n_active / n_dense: the sparse / dense brick counts (< 0: read on the device, one CTA per
-// brick of the lattice launched and the surplus exits).
-void launch_splat(const SplatTri* stt, const unsigned long long* brick_off, const unsigned* brick_count,
-                  const unsigned* brick_list, const unsigned* active, long long n_active, long long n_dense,
-                  const Lattice& L, float* dist, DevState* ds, cudaStream_t st);
+// n_bricks < 0: the brick counts are read on the device, so the launch needs no host round trip.
+void launch_splat(const Fwn& f, long long T, const unsigned long long* brick_off, const unsigned* brick_count,
+                  const unsigned* brick_list, const unsigned* active, long long n_bricks, const Lattice& L, float* dist,
+                  DevState* ds, cudaStream_t st);
 void launch_parity(const ParTri* ptt, const unsigned long long* strip_off, const unsigned* strip_count,
                    const unsigned* strip_list, const Lattice& L, uint32_t* sbits, uint32_t* ubits, DevState* ds,
                    int signed_crossings, cudaStream_t st);

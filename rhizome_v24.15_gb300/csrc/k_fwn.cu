@@ -453,14 +453,6 @@ __device__ __forceinline__ void leaf_term(const float4* __restrict__ leaf, const
 }
 
 // ---- queries of listed voxels ---------------------------------------------------------
-struct FwnView {
-    const float4* cells[3];
-    const float4* box[3];
-    const float4* leaf;
-    int n[3];
-    long long T;
-};
-
 // One warp per listed voxel down the levels: the lanes take 32 clusters, the near ones' (by
 // ballot, in order) children next, two clusters' sixteen or four clusters' eight triangles at a
 // time. What a walk leaves undecided is walked again with a wider near range (smaller truncation
@@ -611,14 +603,6 @@ __global__ void __launch_bounds__(256) list_blocks_kernel(const uint32_t* __rest
     }
 }
 
-// Voxel of a brick by its place in Morton order (32 consecutive ones are a 4 x 4 x 2 box, so a
-// warp's voxels agree on what is near): x | y << 3 | z << 6.
-__device__ __forceinline__ int morton_voxel(int o) {
-    const int x = (o & 1) | ((o >> 2) & 2) | ((o >> 4) & 4), y = ((o >> 1) & 1) | ((o >> 3) & 2) | ((o >> 5) & 4),
-              z = ((o >> 2) & 1) | ((o >> 4) & 2) | ((o >> 6) & 4);
-    return x | (y << 3) | (z << 6);
-}
-
 // Polynomial of far clusters about a centre: value, gradient, half the Hessian (xx, yy, zz,
 // xy + yx, xz + zx, yz + zy), the bound of what it leaves out and the summed term magnitudes.
 struct Local {
@@ -742,10 +726,6 @@ __device__ __forceinline__ int cta_slots(bool flag, int base, int& slot, unsigne
     __syncthreads();
     slot = base + before + __popc(bal & ((1u << lane) - 1u));
     return all;
-}
-
-__device__ __forceinline__ float lattice_mid(int mn, int first, float half, float h) {
-    return ((float)(mn + first) + half) * h;
 }
 
 // Appends the flagged of `n` items to a list of capacity `cap` in item order; returns how many
@@ -1021,31 +1001,12 @@ __device__ __forceinline__ float cta_min(float x, float* red) {
     return x;
 }
 
-// Squared distance of a point to a box (2 float4: least and greatest corner); a NaN gives 0.
-__device__ __forceinline__ float box_dist_sq(const float4* __restrict__ box, const f3& p) {
-    const float4 lo = __ldg(box), hi = __ldg(box + 1);
-    const float dx = max3f(lo.x - p.x, p.x - hi.x, 0.0f), dy = max3f(lo.y - p.y, p.y - hi.y, 0.0f),
-                dz = max3f(lo.z - p.z, p.z - hi.z, 0.0f);
-    return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx));
-}
-
-__device__ __forceinline__ float leaf_dist_sq(const float4* __restrict__ leaf, const f3& p) {
-    const float4 a = __ldg(leaf + 2), b = __ldg(leaf + 3);
-    return ptd_sq(p, mk(a.x, a.y, a.z), mk(a.w, b.x, b.y), mk(b.z, b.w, __ldg(&leaf[4].x)));
-}
-
 // A warp's walk down to one cluster near p: of the n clusters item(i) the one of the least
 // box distance, then its nearest child, to the lowest level; returns the least distance to that
 // cluster's triangles (an upper bound of p's distance to the mesh; the same in all lanes).
 template <class F>
 __device__ __forceinline__ float walk_near(const FwnView& f, int level, int n, const f3& p, F item) {
     const int lane = threadIdx.x & 31;
-    auto pick = [](float d, int k) {  // the least d's k over the warp
-        unsigned long long key = ((unsigned long long)__float_as_uint(d) << 32) | (unsigned)k;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) key = min(key, __shfl_xor_sync(0xffffffffu, key, o));
-        return (int)(unsigned)key;
-    };
     float best = __int_as_float(0x7f800000);
     int bk = -1;
     for (int i = lane; i < n; i += 32) {
@@ -1056,11 +1017,11 @@ __device__ __forceinline__ float walk_near(const FwnView& f, int level, int n, c
             bk = k;
         }
     }
-    int k = pick(bk < 0 ? __int_as_float(0x7f800000) : best, bk < 0 ? 0x7fffffff : bk);
+    int k = warp_argmin(bk < 0 ? __int_as_float(0x7f800000) : best, bk < 0 ? 0x7fffffff : bk);
     for (int l = level - 1; l >= 0; --l) {
         const int c = k * kFwnFan + (lane & 15);
         const bool on = c < f.n[l];
-        k = pick(on ? box_dist_sq(f.box[l] + 2 * (size_t)c, p) : __int_as_float(0x7f800000), on ? c : 0x7fffffff);
+        k = warp_argmin(on ? box_dist_sq(f.box[l] + 2 * (size_t)c, p) : __int_as_float(0x7f800000), on ? c : 0x7fffffff);
     }
     const long long t = (long long)k * kFwnLeaf + (lane & 7);
     float d = t < f.T ? sqrtf(leaf_dist_sq(f.leaf + 5 * t, p)) : __int_as_float(0x7f800000);
@@ -1196,18 +1157,6 @@ __global__ void __launch_bounds__(kBqThreads) nearest_bricks_kernel(FwnView f, L
 }
 
 inline unsigned sort_tiles(long long T) { return (unsigned)((T + kSortTile - 1) / kSortTile); }
-
-FwnView view_of(const Fwn& f, long long T) {
-    FwnView v{};
-    for (int l = 0; l < 3; ++l) {
-        v.cells[l] = reinterpret_cast<const float4*>(f.cells[l]);
-        v.box[l] = f.box[l];
-        v.n[l] = (int)f.n[l];
-    }
-    v.leaf = f.leaf;
-    v.T = T;
-    return v;
-}
 
 // The listed voxels (or, list null, those the blocks left in f.fb2) by a walk each, then the rest
 // of them triangle by triangle.

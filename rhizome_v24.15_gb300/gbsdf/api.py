@@ -119,8 +119,8 @@ def compute_mesh_sdf(tris, voxel_size, min_coord, max_coord, out=None, mode=MODE
     ``host_output``: 0 lets a page-locked host output be written directly by the sign-apply
     kernel, 1 stages it in device memory and copies.
     ``winding_eval``: 0 clustered exact winding decisions, 1 triangle-by-triangle sums.
-    ``splat_dense_cut``: binned triangles per brick above which the splat uses its sub-brick
-    kernel (0 = autotuned per lattice class; identical results at every cut).
+    ``splat_dense_cut``: binned triangles per brick above which the splat takes the brick before
+    the others (0 = 256; identical results at every cut).
     ``wait_poll_limit``: the eikonal's staged-tile waits (0 default; < 0 gives up at once,
     which exercises the failure path). Returns ``(out, Result)``."""
     mn = np.asarray(min_coord, np.int64).reshape(3)

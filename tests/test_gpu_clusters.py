@@ -1,4 +1,4 @@
-"""The exact path's cluster kernels (winding numbers by blocks of bricks, by crossings and caps,
+"""The band splat by clusters against the oracle, and the exact path's cluster kernels (winding numbers by blocks of bricks, by crossings and caps,
 nearest distances) against its per-triangle ones (winding_eval = 1) on every voxel: watertight,
 holed, open, unwelded, degenerate and doubled meshes, ragged and tiny lattices, meshes partly
 or wholly outside the lattice, both block sizes."""
@@ -95,3 +95,20 @@ def test_triangle_counts(engine, n):
     # the edges of the clusters' runs (8, 128 and 2048 triangles) and of the sort's tiles
     tris = _mesh("closed")[:n]
     _compare(engine, tris, 1.1, (-14, -13, -12), (15, 14, 13))
+
+
+@pytest.mark.parametrize("kind,h,half", [(k, 0.9, (18, 17, 16)) for k in KINDS] +
+                         [("few", 0.16, (66, 69, 64)),      # a cluster's box over more than 2048 bricks
+                          ("closed", 4.0, (3, 4, 5)),       # hundreds of clusters in a brick
+                          ("closed", 0.05, (20, 20, 20))])  # triangles larger than a brick
+def test_band_splat(engine, oracle, kind, h, half):
+    tris = _mesh(kind)
+    mn, mx = -np.asarray(half), np.asarray(half) + (1, 0, 2)
+    if kind == "closed" and h < 0.1:
+        mn, mx = mn + (200, 0, 0), mx + (200, 0, 0)  # a window around the surface
+    out, res = engine.compute_mesh_sdf(tris, h, mn, mx, mode=engine.MODE_EXACT_SIGNS, path=engine.PATH_FAST,
+                                       raise_on_error=False)
+    st, ref, _, ost = oracle.fast_sdf(tris, h, mn, mx, fsm_mode=0, gwn_mode=1, signed_parity=True)
+    assert res.status == st and res.stats["band_voxels"] == ost["band_voxels"] > 0
+    if st == oracle.OK:
+        assert np.array_equal(out.view(np.uint32), ref.view(np.uint32))
