@@ -12,8 +12,11 @@
 //     that depend on counts read them on the device (splat over the lattice's bricks,
 //     persistent exact-winding passes), the fixup runs a fixed number of list passes, and
 //     a device-side check decides whether the mesh's output is written;
-//   * run: replay the graph, then read each mesh's state once. A run whose counts
-//     outgrow the planned lists (new triangle contents) re-plans and runs again.
+//   * run: replay the graph, then read each mesh's state once. A mesh whose first probe
+//     found mismatches is finished from the host (patch rounds, further probes, output): few
+//     do, and recording two more generations for all of them cost a fifth of the graph's
+//     launches. A run whose counts outgrow the planned lists (new triangle contents)
+//     re-plans and runs again.
 // Host triangles and host outputs go through pinned staging buffers owned by the batch
 // (a graph's copies need page-locked memory, and a failing mesh's output stays untouched).
 #include <algorithm>
@@ -27,6 +30,7 @@
 #include "../../include/gbsdf.h"
 #include "gbsdf_device.cuh"
 #include "gbsdf_internal.h"
+#include "signs.h"
 
 struct gbsdf_batch;
 
@@ -135,6 +139,7 @@ struct gbsdf_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     unsigned long long launches_per_run = 0;
+    gbsdf::CapScratch cap_scratch;  // patch rounds: crossings and caps of one member at a time
     // learned mode: the network's parameters (device memory, the caller's), the proposal
     // threshold as a logit and the budget (0: 1/16 of each lattice's bricks)
     const float* mlp_params = nullptr;
@@ -215,6 +220,38 @@ void enqueue_counts(gbsdf_batch& b, Job& j, cudaStream_t st) {
     launch_active_bricks(j.bcount, L.nbricks, j.active, j.ds, st, j.dense_cut);
 }
 
+// The sign state of a member on its buffers (the crossings' integer grid is B, which holds nothing
+// while winding numbers are decided).
+SignWork sign_work(const gbsdf_batch& b, Job& j, CapScratch* scratch) {
+    SignWork s;
+    s.t9 = j.t9;
+    s.T = j.T;
+    s.L = j.L;
+    s.dist = j.A;
+    s.stol = exact_signs_mode(b) ? kSurfaceTolExactSigns : kSurfaceTolVoxels;
+    s.grid = reinterpret_cast<int*>(j.B);
+    s.U = j.U;
+    s.S = j.S;
+    s.list = j.list;
+    s.recheck = j.recheck;
+    s.cap = j.list_cap;
+    s.ds = j.ds;
+    s.hs = j.hs;
+    s.fwn = &j.fwn;
+    s.num_sms = b.num_sms;
+    s.st = j.st;
+    s.scratch = scratch;
+    return s;
+}
+
+// [F], written only when the build passed its checks.
+void enqueue_output(gbsdf_batch& b, Job& j, cudaStream_t st) {
+    launch_apply(j.A, j.S, j.L, b.out_dev ? j.out : j.B, j.ds,
+                 exact_signs_mode(b) ? kSurfaceTolExactSigns * j.L.h : -1.0f, st);
+    if (!b.out_dev) cudaMemcpyAsync(j.hout, j.B, (size_t)j.L.N * 4, cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(j.hs, j.ds, sizeof(DevState), cudaMemcpyDeviceToHost, st);
+}
+
 // The rest of a build, with no host round trip.
 void enqueue_build(gbsdf_batch& b, Job& j, cudaStream_t st) {
     const Lattice& L = j.L;
@@ -267,20 +304,11 @@ void enqueue_build(gbsdf_batch& b, Job& j, cudaStream_t st) {
     if (pad) launch_unpad_rows(j.B, j.A, Lp, st, j.ds);  // with the audit's count
     else launch_audit(j.A, L, j.ds, st);
     launch_clamp(j.A, j.S, L, j.ds, st);
-    // [E]
-    for (int gen = 0; gen < kProbeGens; ++gen) {
-        launch_verify_prepare(L, gen, j.U, j.list, j.ds, st);
-        launch_winding(&j.fwn, j.t9, T, L, j.list, j.list_cap, kGwnVerify, 0, j.S, j.recheck, j.list_cap, j.A, 0,
-                       stol, j.ds, b.num_sms, st);
-        launch_gwn_recheck(j.t9, T, L, j.recheck, j.list_cap, kGwnVerify, j.S, j.ds, b.num_sms, st);
-        launch_verify_plan(gen, j.ds, st, learned ? 1 : 0);
-        if (gen == kProbeGens - 1) break;
-        launch_patch_mark(L, j.U, j.ds, st);
-        launch_list_blocks(j.U, L, j.list, j.list_cap, j.ds, 1, st);
-        launch_winding_blocks(j.fwn, j.t9, T, L, j.U, j.S, learned ? j.E : nullptr, j.list, j.list_cap, 1, j.recheck,
-                              j.list_cap, j.A, 0, stol, j.ds, b.num_sms, st);
-        launch_gwn_recheck(j.t9, T, L, j.recheck, j.list_cap, kGwnFixup, j.S, j.ds, b.num_sms, st);
-    }
+    // [E]: the first probe. Most builds come back clean; one that needs patch rounds writes no
+    // output here and is finished from the host after the graph (finish_job).
+    SignWork sw = sign_work(b, j, nullptr);
+    sw.st = st;
+    enqueue_probe(sw, 0, learned);
     // learned mode, as in the single-mesh path: the signed-crossing pass (its unknown
     // columns are not counted), escalation of a diverged verify, the brick features, the
     // network's scores and the budgeted proposals, re-decided by the exact winding number
@@ -302,11 +330,20 @@ void enqueue_build(gbsdf_batch& b, Job& j, cudaStream_t st) {
         launch_propose_dev(j.logits, L, b.logit_thr, budget, j.phist, j.ds, j.U, st);
         fixup_passes(nullptr);
     }
-    // [F], written only when the build passed its checks
     launch_batch_finalize(j.ds, learned ? 0 : 1, st);
-    launch_apply(j.A, j.S, L, b.out_dev ? j.out : j.B, j.ds, xs ? stol * L.h : -1.0f, st);
-    if (!b.out_dev) cudaMemcpyAsync(j.hout, j.B, (size_t)N * 4, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(j.hs, j.ds, sizeof(DevState), cudaMemcpyDeviceToHost, st);
+    enqueue_output(b, j, st);
+}
+
+// A member whose first probe found mismatches: its patch rounds and further probes, from the
+// host, on its own buffers, then its output.
+cudaError_t finish_job(gbsdf_batch& b, Job& j) {
+    const DevState& h = *j.hs;
+    if (learned_mode(b) || h.verify_state != 0 || !h.patching || h.overflow || h.abort_ || h.wait_timeouts)
+        return cudaSuccess;
+    SignWork sw = sign_work(b, j, &b.cap_scratch);
+    if (const cudaError_t err = finish_probes(sw, 0, nullptr)) return err;
+    enqueue_output(b, j, j.st);
+    return cudaStreamSynchronize(j.st);
 }
 
 void free_plan(gbsdf_batch& b) {
@@ -471,6 +508,9 @@ int run_once(gbsdf_batch& b, bool& any_overflow, float& ms, BErr& e) {
         if (j.pre_status == GBSDF_OK && !b.tris_dev) parallel_copy(j.hin, j.tris, (size_t)j.T * 48);
     GBB_CK(cudaEventRecord(b.t0, b.origin));
     GBB_CK(cudaGraphLaunch(b.exec, b.origin));
+    GBB_CK(cudaStreamSynchronize(b.origin));
+    for (Job& j : b.jobs)
+        if (j.pre_status == GBSDF_OK) GBB_CK(finish_job(b, j));
     GBB_CK(cudaEventRecord(b.t1, b.origin));
     GBB_CK(cudaStreamSynchronize(b.origin));
     GBB_CK(cudaEventElapsedTime(&ms, b.t0, b.t1));
@@ -488,6 +528,7 @@ void destroy(gbsdf_batch* b) {
     cudaSetDevice(b->device);
     if (b->origin) cudaStreamSynchronize(b->origin);
     free_plan(*b);
+    for (Buf* s : {&b->cap_scratch.etab, &b->cap_scratch.caps, &b->cap_scratch.cfw, &b->cap_scratch.cross}) release(*s);
     for (gbsdf::Job& j : b->jobs) {
         if (j.hin) cudaFreeHost(j.hin);
         if (j.hout) cudaFreeHost(j.hout);

@@ -25,6 +25,7 @@
 #include "../../include/gbsdf.h"
 #include "gbsdf_device.cuh"
 #include "gbsdf_internal.h"
+#include "signs.h"
 
 namespace gbsdf {
 
@@ -53,11 +54,6 @@ Lattice make_lattice(const int32_t mn[3], const int32_t mx[3], float h) {
 
 namespace {
 
-struct Buf {
-    void* p = nullptr;
-    size_t bytes = 0;
-};
-
 struct Workspace {
     int device = -1;
     int num_sms = 0;
@@ -65,8 +61,8 @@ struct Workspace {
     cudaEvent_t ev[14] = {};
     std::mutex mu;
     Buf A, B, S, U, t12, t9, ptt, btris, bcount, bcur, boff, active, blist, scount, scur, soff, slist, scan, list,
-        recheck, hb, verts, idx, flags, fpos, S2, U2, fbase, fX, logits, opencnt, ekeys, ecnt, mparts, mlossp, phist, E, fw, etab,
-        caps, cfw, cross;
+        recheck, hb, verts, idx, flags, fpos, S2, U2, fbase, fX, logits, opencnt, ekeys, ecnt, mparts, mlossp, phist, E, fw;
+    CapScratch cap_scratch;
     DevState* ds = nullptr;
     DevState* hs = nullptr;  // pinned host mirror
 };
@@ -96,21 +92,6 @@ struct Err {
                          #call, cudaGetErrorString(_e), __FILE__, __LINE__);                            \
         }                                                                                               \
     } while (0)
-
-cudaError_t ensure(Buf& b, size_t bytes) {
-    if (bytes <= b.bytes && b.p) return cudaSuccess;
-    if (b.p) cudaFree(b.p);
-    b.p = nullptr;
-    b.bytes = 0;
-    size_t want = bytes + bytes / 8 + 256;
-    cudaError_t err = cudaMalloc(&b.p, want);
-    if (err != cudaSuccess) {
-        cudaGetLastError();
-        return err;
-    }
-    b.bytes = want;
-    return cudaSuccess;
-}
 
 template <class T>
 T* P(Buf& b) {
@@ -164,11 +145,8 @@ void free_ws(Workspace& w) {
                    &w.active, &w.blist, &w.scount, &w.scur, &w.soff, &w.slist, &w.scan, &w.list, &w.recheck,
                    &w.hb, &w.verts, &w.idx, &w.flags, &w.fpos, &w.S2, &w.U2, &w.fbase, &w.fX, &w.logits,
                    &w.opencnt, &w.ekeys, &w.ecnt, &w.mparts, &w.mlossp, &w.phist, &w.E,
-                   &w.fw, &w.etab, &w.caps, &w.cfw, &w.cross};
-    for (Buf* b : bufs) {
-        if (b->p) cudaFree(b->p);
-        *b = Buf{};
-    }
+                   &w.fw, &w.cap_scratch.etab, &w.cap_scratch.caps, &w.cap_scratch.cfw, &w.cap_scratch.cross};
+    for (Buf* b : bufs) release(*b);
     if (w.ds) cudaFree(w.ds);
     if (w.hs) cudaFreeHost(w.hs);
     for (auto& ev : w.ev)
@@ -192,8 +170,6 @@ float ev_ms(cudaEvent_t a, cudaEvent_t b) {
 
 constexpr long long kListCap = 8ll * 1024 * 1024;  // >= 64 patch boxes of 49^3 voxels
 
-// Exact winding of every voxel flagged in U (initial unknown columns): compaction
-// into the dense list, FP32 pass, FP64 re-checks; repeats while the list overflowed.
 // Clusters of the hierarchical winding evaluation for the packed triangles (w.t9).
 int build_fwn(Workspace& w, const Lattice& L, long long T, Fwn& f, Err& e) {
     cudaStream_t st = w.st;
@@ -204,79 +180,29 @@ int build_fwn(Workspace& w, const Lattice& L, long long T, Fwn& f, Err& e) {
     return GBSDF_OK;
 }
 
-// The crossings and caps of one build, made when a pass first has enough marked voxels.
-struct Capped {
-    bool tried = false, on = false;
-    long long B = 0;
-    Fwn f{};
-    Crossings x{};
-};
-
-// The integer grid is w.B, which holds nothing while winding numbers are decided. Meshes whose
-// boundary is long (unwelded soups: more than one unmatched edge for every four triangles) keep
-// to the clusters of the mesh: their caps would be as many as its triangles. So does a build
-// that finds no memory for the table.
-int make_capped(Workspace& w, const Lattice& L, long long T, Capped& c, Err& e) {
-    cudaStream_t st = w.st;
-    c.tried = true;
-    if (T > (1ll << 26)) return GBSDF_OK;  // the table is 12 bytes a slot, over six slots a triangle
-    if (ensure(w.etab, edge_table_bytes(T)) != cudaSuccess) return GBSDF_OK;
-    launch_edge_table(P<float>(w.t9), T, w.etab.p, st);
-    unsigned long long counts[2] = {0, 0};
-    GB_CK(cudaMemcpyAsync(counts, w.etab.p, sizeof(counts), cudaMemcpyDeviceToHost, st));
-    GB_CK(cudaStreamSynchronize(st));
-    c.B = (long long)counts[0];
-    if (counts[1] || c.B > T / 4) return GBSDF_OK;
-    const float* caps9 = nullptr;
-    if (c.B > 0) {
-        if (ensure(w.caps, caps_bytes(c.B)) != cudaSuccess || ensure(w.cfw, fwn_bytes(c.B, 1)) != cudaSuccess)
-            return GBSDF_OK;
-        caps9 = launch_caps(P<float>(w.t9), T, w.etab.p, c.B, w.caps.p, st);
-        c.f = fwn_carve(w.cfw.p, c.B, 1);
-        launch_fwn_build(caps9, c.B, L, c.f, st);
-    }
-    if (ensure(w.cross, crossing_bytes(L)) != cudaSuccess) return GBSDF_OK;
-    c.x = launch_crossings(P<float>(w.t9), T, caps9, c.B, L, P<int>(w.B), w.cross.p, st);
-    GB_CK(cudaGetLastError());
-    c.on = true;
-    return GBSDF_OK;
-}
-
-int fixup_unknown(Workspace& w, const Lattice& L, long long T, float stol, Err& e, uint32_t* ebits, const Fwn* fwn,
-                  Capped& cap, int dist_sq = 0) {
-    const float* dist = P<float>(w.A);
-    cudaStream_t st = w.st;
-    for (int pass = 0; pass < 1 << 20; ++pass) {
-        GB_CK(cudaMemsetAsync(&w.ds->listed, 0, kPassCounters, st));
-        if (fwn) launch_list_blocks(P<uint32_t>(w.U), L, P<long long>(w.list), kListCap, w.ds, 0, st);
-        else launch_list_unknown(P<uint32_t>(w.U), P<uint32_t>(w.S), L, P<long long>(w.list), kListCap, w.ds, 0, st,
-                                 ebits);
-        GB_CK(cudaMemcpyAsync(w.hs, w.ds, sizeof(DevState), cudaMemcpyDeviceToHost, st));
-        GB_CK(cudaStreamSynchronize(st));
-        long long n = std::min<long long>((long long)w.hs->listed, kListCap);
-        if (n <= 0) return GBSDF_OK;
-        if (fwn && !cap.tried && w.hs->listed_voxels >= (unsigned long long)kCapsMinVoxels)
-            if (int rcc = make_capped(w, L, T, cap, e)) return rcc;
-        if (fwn && cap.on)
-            launch_capped_blocks(cap.f, cap.B, L, cap.x, P<uint32_t>(w.U), P<uint32_t>(w.S), ebits,
-                                 P<long long>(w.list), kListCap, dist, dist_sq, stol, w.ds, w.num_sms, st);
-        if (fwn)
-            launch_winding_blocks(*fwn, P<float>(w.t9), T, L, P<uint32_t>(w.U), P<uint32_t>(w.S), ebits,
-                                  P<long long>(w.list), kListCap, 0, P<long long>(w.recheck), kListCap, dist, dist_sq,
-                                  stol, w.ds, w.num_sms, st);
-        else if (n < 64 * 1024)
-            launch_gwn_small(P<float>(w.t9), T, L, P<long long>(w.list), kListCap, kGwnFixup, P<uint32_t>(w.S),
-                             P<long long>(w.recheck), kListCap, dist, dist_sq, stol, w.ds, n, st);
-        else
-            launch_gwn(P<float>(w.t9), T, L, P<long long>(w.list), kListCap, kGwnFixup, 0, P<uint32_t>(w.S),
-                       P<long long>(w.recheck), kListCap, dist, dist_sq, stol, w.ds, w.num_sms, st);
-        launch_gwn_recheck(P<float>(w.t9), T, L, P<long long>(w.recheck), kListCap, kGwnFixup, P<uint32_t>(w.S),
-                           w.ds, w.num_sms, st);
-        GB_CK(cudaGetLastError());
-        // blocks: the leftovers of a pass can outgrow their list too (their voxels stay marked)
-        if (w.hs->list_overflow == 0 && (!fwn || w.hs->listed_voxels <= (unsigned long long)kListCap)) return GBSDF_OK;
-    }
-    return e.set(GBSDF_ECUDA, "unknown-voxel fixup did not drain");
+// The sign state of a build on the workspace's buffers. The crossings' integer grid is w.B, which
+// holds nothing while winding numbers are decided.
+SignWork sign_work(Workspace& w, const Lattice& L, long long T, float stol, const Fwn* fwn, int dist_sq) {
+    SignWork s;
+    s.t9 = P<float>(w.t9);
+    s.T = T;
+    s.L = L;
+    s.dist = P<float>(w.A);
+    s.dist_sq = dist_sq;
+    s.stol = stol;
+    s.grid = P<int>(w.B);
+    s.U = P<uint32_t>(w.U);
+    s.S = P<uint32_t>(w.S);
+    s.list = P<long long>(w.list);
+    s.recheck = P<long long>(w.recheck);
+    s.cap = kListCap;
+    s.ds = w.ds;
+    s.hs = w.hs;
+    s.fwn = fwn;
+    s.num_sms = w.num_sms;
+    s.st = w.st;
+    s.scratch = &w.cap_scratch;
+    return s;
 }
 
 // The signed-crossing parity pass into w.S2 / w.U2 (learned mode: the escalation's signs
@@ -414,9 +340,8 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
     }
     GB_CK(cudaEventRecord(w.ev[4], st));
     // ---- [C]
-    Capped cap;
-    int rc = fixup_unknown(w, L, T, stol, e, ebits, fwn, cap);
-    if (rc != GBSDF_OK) return rc;
+    SignWork sw = sign_work(w, L, T, stol, fwn, 0);
+    GB_CK(decide_marked(sw, ebits, false));
     GB_CK(cudaEventRecord(w.ev[5], st));
     // ---- [D]
     const int rule = ref_eikonal ? 0 : 1;
@@ -510,30 +435,16 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
     GB_CK(cudaGetLastError());
     GB_CK(cudaEventRecord(w.ev[6], st));
     // ---- [E]
-    for (int gen = 0; gen < kProbeGens; ++gen) {
-        launch_verify_prepare(L, gen, P<uint32_t>(w.U), P<long long>(w.list), w.ds, st);
-        launch_winding(fwn, P<float>(w.t9), T, L, P<long long>(w.list), kListCap, kGwnVerify, 0, P<uint32_t>(w.S),
-                       P<long long>(w.recheck), kListCap, P<float>(w.A), 0, stol, w.ds, w.num_sms, st);
-        launch_gwn_recheck(P<float>(w.t9), T, L, P<long long>(w.recheck), kListCap, kGwnVerify, P<uint32_t>(w.S),
-                           w.ds, w.num_sms, st);
-        launch_verify_plan(gen, w.ds, st, learned ? 1 : 0);
-        if (gen == kProbeGens - 1) break;  // the last generation never patches
-        launch_patch_mark(L, P<uint32_t>(w.U), w.ds, st);
-        if (fwn) {
-            launch_list_blocks(P<uint32_t>(w.U), L, P<long long>(w.list), kListCap, w.ds, 1, st);
-            launch_winding_blocks(*fwn, P<float>(w.t9), T, L, P<uint32_t>(w.U), P<uint32_t>(w.S), ebits,
-                                  P<long long>(w.list), kListCap, 1, P<long long>(w.recheck), kListCap, P<float>(w.A),
-                                  0, stol, w.ds, w.num_sms, st);
-        } else {
-            launch_list_unknown(P<uint32_t>(w.U), P<uint32_t>(w.S), L, P<long long>(w.list), kListCap, w.ds, 1, st,
-                                ebits);
-            launch_gwn(P<float>(w.t9), T, L, P<long long>(w.list), kListCap, kGwnFixup, 1, P<uint32_t>(w.S),
-                       P<long long>(w.recheck), kListCap, P<float>(w.A), 0, stol, w.ds, w.num_sms, st);
-        }
-        launch_gwn_recheck(P<float>(w.t9), T, L, P<long long>(w.recheck), kListCap, kGwnFixup, P<uint32_t>(w.S),
-                           w.ds, w.num_sms, st);
-    }
+    // (the eikonal swaps the two grid copies)
+    sw.dist = P<float>(w.A);
+    sw.grid = P<int>(w.B);
+    enqueue_probe(sw, 0, learned);
     GB_CK(cudaGetLastError());
+    if (!learned) {  // learned mode has no patch rounds, and its state is read below
+        GB_CK(cudaMemcpyAsync(w.hs, w.ds, sizeof(DevState), cudaMemcpyDeviceToHost, st));
+        GB_CK(cudaStreamSynchronize(st));
+        GB_CK(finish_probes(sw, 0, ebits));
+    }
     // ---- learned mode, after [E] (the probes and patch boxes ran exactly as in the plain
     // path): the signed-crossing pass; a diverged verify escalates to its signs, its columns
     // through holes decided by the exact winding number, instead of declining; then the
@@ -546,8 +457,7 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
             launch_escalate(w.ds, P<uint32_t>(w.S), P<uint32_t>(w.U), P<uint32_t>(w.S2), P<uint32_t>(w.U2), L,
                             w.num_sms, st);
             GB_CK(cudaGetLastError());
-            int rce = fixup_unknown(w, L, T, stol, e, ebits, fwn, cap);
-            if (rce != GBSDF_OK) return rce;
+            GB_CK(decide_marked(sw, ebits, false));
         }
         int rcf = brick_features(w, T, L, e);
         if (rcf != GBSDF_OK) return rcf;
@@ -570,8 +480,7 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
         GB_CK(ensure(w.phist, (size_t)kPropBins * 4));
         launch_propose_dev(logits, L, lthr, budget, P<unsigned>(w.phist), w.ds, P<uint32_t>(w.U), st);
         GB_CK(cudaGetLastError());
-        int rcp = fixup_unknown(w, L, T, stol, e, nullptr, fwn, cap);
-        if (rcp != GBSDF_OK) return rcp;
+        GB_CK(decide_marked(sw, nullptr, false));
     }
     GB_CK(cudaEventRecord(w.ev[7], st));
     // ---- [F]
@@ -688,8 +597,8 @@ int run_legacy(Workspace& w, long long T, const Lattice& L, float* out, bool out
     if (fwn) {
         GB_CK(ensure(w.U, (size_t)L.nwords * 4));
         GB_CK(cudaMemsetAsync(w.U.p, 0xff, (size_t)L.nwords * 4, st));
-        Capped cap;
-        if (int rcx = fixup_unknown(w, L, T, kSurfaceTolVoxels, e, nullptr, fwn, cap, 1)) return rcx;
+        SignWork sw = sign_work(w, L, T, kSurfaceTolVoxels, fwn, 1);
+        GB_CK(decide_marked(sw, nullptr, false));
     } else {
         for (long long v0 = 0; v0 < N; v0 += kListCap) {
             long long n = std::min(kListCap, N - v0);

@@ -251,7 +251,7 @@ size_t crossing_bytes(const Lattice& L);
 Crossings launch_crossings(const float* tri9, long long T, const float* caps9, long long B, const Lattice& L,
                            int* grid, void* scratch, cudaStream_t st);
 void launch_capped_blocks(const Fwn& f, long long B, const Lattice& L, const Crossings& X, uint32_t* ubits,
-                          uint32_t* sbits, uint32_t* ebits, const long long* list, long long list_cap,
+                          uint32_t* sbits, uint32_t* ebits, const long long* list, long long list_cap, int only_if,
                           const float* dist, int dist_sq, float surf_tol_vox, DevState* ds, int num_sms,
                           cudaStream_t st);
 // Batches: decides on the device whether the build passed its checks (valid triangles,

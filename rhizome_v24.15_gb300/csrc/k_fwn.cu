@@ -1268,13 +1268,13 @@ void launch_nearest(const Fwn& f, long long T, const Lattice& L, float* d2, cuda
 }
 
 void launch_capped_blocks(const Fwn& f, long long B, const Lattice& L, const Crossings& X, uint32_t* ubits,
-                          uint32_t* sbits, uint32_t* ebits, const long long* list, long long list_cap,
+                          uint32_t* sbits, uint32_t* ebits, const long long* list, long long list_cap, int only_if,
                           const float* dist, int dist_sq, float surf_tol_vox, DevState* ds, int num_sms,
                           cudaStream_t st) {
     const int BB = block_bricks(L);
     const unsigned grid = (unsigned)std::min<long long>(block_count(L, BB), (long long)num_sms * 8);
     auto go = [&](auto kernel) {
-        kernel<<<grid, kBqThreads, 0, st>>>(view_of(f, B), L, X, ubits, sbits, ebits, list, list_cap, 0, dist, dist_sq,
+        kernel<<<grid, kBqThreads, 0, st>>>(view_of(f, B), L, X, ubits, sbits, ebits, list, list_cap, only_if, dist, dist_sq,
                                             surf_tol_vox, ds, nullptr, 0);
     };
     GBSDF_COUNT_LAUNCH();
