@@ -189,8 +189,9 @@ def run_learned_report(gbsdf, torch, dev, mlp):
 
 
 _X_SCHED = {1: "sweep_x_kernel", 2: "sweep_x_tma_kernel", 3: "sweep_x_pipe_kernel", 4: "sweep_x_pipe2_kernel",
-            5: "sweep_x_wide_kernel"}
-_W_SCHED = {1: "sweep_walk_kernel", 2: "sweep_walk_pipe_kernel", 3: "sweep_walk_vec_kernel", 4: "sweep_walk_vec2_kernel"}
+            5: "sweep_x_wide_kernel", 6: "sweep_x_pipe_kernel (narrow tiles)"}
+_W_SCHED = {1: "sweep_walk_kernel", 2: "sweep_walk_pipe_kernel", 3: "sweep_walk_vec_kernel", 4: "sweep_walk_vec2_kernel",
+            5: "sweep_walk_narrow_kernel"}
 
 
 def _sweep_kernels(sched):

@@ -115,14 +115,17 @@ typedef struct gbsdf_options {
                                tiles on a warp-specialised mbarrier pipeline, 4 the same with two
                                lines per thread updated in packed FP32 pairs (the reference's
                                update at voxel sizes 2^-20 to 2^20; otherwise 3 runs), 5 the
-                               pipeline with 16-voxel chunks staged as 20-column boxes; w = 1 y / z walks
+                               pipeline with 16-voxel chunks staged as 20-column boxes, 6 the
+                               pipeline on tiles of 32 x 4 lines; w = 1 y / z walks
                                staged by cp.async, 2 by TMA batches on a pipeline, 3 the same
                                with four adjacent lines per thread, 4 the same with the lines'
                                updates in packed FP32 pairs (the reference's update at voxel
-                               sizes 2^-20 to 2^20; otherwise 3 runs); a 0 digit (and
+                               sizes 2^-20 to 2^20; otherwise 3 runs), 5 one line per
+                               thread on tiles of 32 x 4 lines; a 0 digit (and
                                0 overall) = autotuned (the first build of a lattice class times
                                the candidates for the rounds after the first; the first round
-                               takes 3 + 10 x 4). Every lattice can take the TMA schedules: the
+                               takes 3 + 10 x 4, and 6 and 5 where the wide tiles are at
+                               most 1.5 per SM). Every lattice can take the TMA schedules: the
                                sweeps run in copies with rows padded to a multiple of 8 voxels. */
     int32_t host_output;    /* host outputs: 0 = a page-locked output is written by the sign-apply
                                kernel through its device mapping (no staging copy), others are
@@ -166,8 +169,8 @@ typedef struct gbsdf_stats {
     int64_t csr_entries;   /* entries of the reference's supercell CSR */
     int64_t kernel_launches; /* CUDA kernels this call launched */
     int64_t proposed;      /* learned mode: bricks the network proposed for the exact winding number */
-    int64_t sweep_schedule; /* schedules that ran in the rounds after the first: x schedule (1-5)
-                               + 10 x walk schedule (1-4), numbered as in
+    int64_t sweep_schedule; /* schedules that ran in the rounds after the first: x schedule (1-6)
+                               + 10 x walk schedule (1-5), numbered as in
                                gbsdf_options.sweep_schedule */
     int64_t winding_certified; /* exact winding decisions settled by the cluster bound */
     int64_t winding_summed;    /* ... and by the triangle-by-triangle sum */

@@ -375,16 +375,16 @@ int plan(gbsdf_batch& b, BErr& e) {
             const Lattice Lp = padded(j.L);
             encode_grid_map(j.map_a, j.A, Lp);
             encode_grid_map(j.map_b, j.B, Lp);
-            const SweepPlan plan = tuned_sweep_plan(b.device, Lp, j.A, j.B, &j.map_a, j.ds, b.origin, false, 0);
-            const SweepPlan plan1 = tuned_sweep_plan(b.device, Lp, j.A, j.B, &j.map_a, j.ds, b.origin, false, 1);
+            const SweepPlan plan = tuned_sweep_plan(b.device, Lp, j.A, j.B, &j.map_a, j.ds, b.origin, false, 0, 0);
+            const SweepPlan plan1 = tuned_sweep_plan(b.device, Lp, j.A, j.B, &j.map_a, j.ds, b.origin, false, 1, 0);
             j.xsched = plan.x;
             j.wsched = plan.w;
             if (b.dense_cut > 0) j.dense_cut = (unsigned)b.dense_cut;
             j.xsched1 = plan1.x;
             j.wsched1 = plan1.w;
             const int xs_opt = b.sweep_schedule % 10, ws_opt = b.sweep_schedule / 10;
-            if (xs_opt >= kXCpAsync && xs_opt <= kXTmaWide) j.xsched = j.xsched1 = xs_opt;
-            if (ws_opt >= kWCpAsync && ws_opt <= kWTmaVec2) j.wsched = j.wsched1 = ws_opt;
+            if (xs_opt >= kXCpAsync && xs_opt <= kXTmaNarrow) j.xsched = j.xsched1 = xs_opt;
+            if (ws_opt >= kWCpAsync && ws_opt <= kWTmaNarrow) j.wsched = j.wsched1 = ws_opt;
         }
     // counting pass
     for (Job& j : b.jobs) {

@@ -370,9 +370,9 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
     const bool tune = xs_opt == 0 || ws_opt == 0;
     SweepPlan plan;
     auto set_plan = [&](int phase, const GridMap* m, bool measure) -> int {
-        plan = tuned_sweep_plan(w.device, Lp, src, dst, m, w.ds, st, measure, phase);
-        if (xs_opt >= kXCpAsync && xs_opt <= kXTmaWide) plan.x = xs_opt;
-        if (ws_opt >= kWCpAsync && ws_opt <= kWTmaVec2) plan.w = ws_opt;
+        plan = tuned_sweep_plan(w.device, Lp, src, dst, m, w.ds, st, measure, phase, rule);
+        if (xs_opt >= kXCpAsync && xs_opt <= kXTmaNarrow) plan.x = xs_opt;
+        if (ws_opt >= kWCpAsync && ws_opt <= kWTmaNarrow) plan.w = ws_opt;
         GB_CK(cudaGetLastError());
         return (int)GBSDF_OK;
     };

@@ -274,6 +274,9 @@ struct GridMap {
     CUtensorMap ymap;  // y walk batch: 40 (x) x 4 (y slices) x 18 (z rows)
     CUtensorMap zmap;  // z walk batch: 40 (x) x 18 (y rows) x 4 (z slices)
     CUtensorMap wmap;  // wide x sweep tile: 20 (x) x 34 (y) x 10 (z), no swizzle
+    CUtensorMap nmap;  // narrow x sweep tile: 8 (x) x 34 (y) x 6 (z), 32-byte swizzle
+    CUtensorMap ynmap; // narrow y walk batch: 40 (x) x 4 (y slices) x 6 (z rows)
+    CUtensorMap znmap; // narrow z walk batch: 40 (x) x 6 (y rows) x 4 (z slices)
     bool valid;
     bool walk_valid;
     bool wide_valid;
@@ -288,29 +291,34 @@ void launch_unpad_rows(const float* pad, float* dense, const Lattice& P, cudaStr
 // copies, by TMA tiles on a CTA-barrier ring, by TMA tiles on a warp-specialised mbarrier
 // pipeline, the same pipeline with two lines per thread updated in packed FP32 pairs (the
 // reference's update on lattices with at least two voxels along y and z; elsewhere it runs
-// as the pipeline), or the pipeline with 16-voxel chunks staged as 20-column boxes (one
-// copy per chunk carries its downstream neighbour). 0 picks the pipeline when a TMA
-// descriptor is valid.
-enum XSchedule : int { kXAuto = 0, kXCpAsync = 1, kXTmaRing = 2, kXTmaPipe = 3, kXTmaPipe2 = 4, kXTmaWide = 5 };
+// as the pipeline), the pipeline with 16-voxel chunks staged as 20-column boxes (one copy
+// per chunk carries its downstream neighbour), or the pipeline on tiles of 32 x 4 lines.
+// 0 picks the pipeline when a TMA descriptor is valid.
+enum XSchedule : int {
+    kXAuto = 0, kXCpAsync = 1, kXTmaRing = 2, kXTmaPipe = 3, kXTmaPipe2 = 4, kXTmaWide = 5, kXTmaNarrow = 6
+};
 // Schedules of the y and z walks: cp.async slice ring, TMA batches on a warp-specialised
 // mbarrier pipeline (one line per thread in two rows, or four adjacent lines per thread,
 // or four adjacent lines per thread updated in packed FP32 pairs -- the reference's
 // update on lattices with at least two rows across the walk; elsewhere it runs as the
-// four-lines schedule). 0 picks the pipeline when its descriptors are valid.
-enum WSchedule : int { kWAuto = 0, kWCpAsync = 1, kWTmaPipe = 2, kWTmaVec = 3, kWTmaVec2 = 4 };
+// four-lines schedule, or one line per thread in tiles of 32 x 4 lines). 0 picks the
+// pipeline when its descriptors are valid.
+enum WSchedule : int {
+    kWAuto = 0, kWCpAsync = 1, kWTmaPipe = 2, kWTmaVec = 3, kWTmaVec2 = 4, kWTmaNarrow = 5
+};
 // `src_map`: the descriptor of `src` (or null); `x_schedule`: an XSchedule.
 void launch_sweep(int rule, int axis, int dir, int round, const float* src, float* dst, const Lattice& L,
                   DevState* ds, cudaStream_t st, const GridMap* src_map = nullptr, int x_schedule = kXAuto,
                   int w_schedule = kWAuto);
 // The sweep schedules for this lattice class and phase (0: the first round, 1: later
 // rounds): the remembered winners, else (measure) each candidate timed on src -> dst
-// (writes dst and changed[63]), else the pipelines.
+// (writes dst and changed[63]), else the default plan of the lattice and update rule.
 struct SweepPlan {
     int x;  // XSchedule
     int w;  // WSchedule
 };
 SweepPlan tuned_sweep_plan(int device, const Lattice& L, const float* src, float* dst, const GridMap* src_map,
-                           DevState* ds, cudaStream_t st, bool measure, int phase);
+                           DevState* ds, cudaStream_t st, bool measure, int phase, int rule);
 // Layout check of the x sweep's TMA tile (swizzled rows, out-of-lattice fill): writes the
 // number of mismatching elements to *mism.
 int selftest_tma_tile(unsigned long long* mism);

@@ -530,6 +530,17 @@ __global__ void __launch_bounds__(kXThreads) sweep_x_tma_kernel(const __grid_con
 constexpr int kPS = 4;                               // ring slots
 constexpr int kPThreads = kXThreads + 32;            // 8 consumer warps + 1 producer warp
 constexpr size_t kPSmem = (size_t)kPS * kTSlotBytes + 128 + 1024;
+// The pipeline on tiles of ZT lines along z: 8, or 4 with a deeper ring where tiles of 8 would
+// leave SMs without a CTA (224^3: 41.4 -> 38.8 us per sweep over all six directions).
+constexpr int kXZNarrow = 4;
+template <int ZT>
+struct XPipe {
+    static constexpr int kConsumers = kXY * ZT, kThreads = kConsumers + 32;
+    static constexpr int kBox = kXC * kXHY * (ZT + 2);
+    static constexpr int kSlotBytes = (kBox * 4 + 1023) / 1024 * 1024;
+    static constexpr int kSlots = ZT == kXZ ? kPS : 6;
+    static constexpr size_t kSmem = (size_t)kSlots * kSlotBytes + 128 + 1024;
+};
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
@@ -538,47 +549,48 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // NB: the reference's update without branches, RULE 0 at voxel sizes with pair_sqrt_ok
 // (1: godunov_ref_nb; 2: godunov_ref_nbp, its 2D and 3D arithmetic paired on packed FP32
 // lanes, 57-59 instructions per voxel against 66), identical results.
-template <int RULE, int DIR, int NB = 0>
-__global__ void __launch_bounds__(kPThreads) sweep_x_pipe_kernel(const __grid_constant__ CUtensorMap tm,
+template <int RULE, int DIR, int NB = 0, int ZT = kXZ>
+__global__ void __launch_bounds__(XPipe<ZT>::kThreads) sweep_x_pipe_kernel(const __grid_constant__ CUtensorMap tm,
                                                                   float* __restrict__ dst, Lattice L, int round,
                                                                   DevState* ds) {
     if (ds->stop) return;
+    constexpr int kSlots = XPipe<ZT>::kSlots, kSlotBytes = XPipe<ZT>::kSlotBytes, kConsumers = XPipe<ZT>::kConsumers;
     const int polls = wait_poll_limit(ds);
     extern __shared__ unsigned char tsm_raw[];
     unsigned char* tsm = align1k(tsm_raw);
-    uint64_t* full = reinterpret_cast<uint64_t*>(tsm + kPS * kTSlotBytes);
-    uint64_t* empty = full + kPS;
+    uint64_t* full = reinterpret_cast<uint64_t*>(tsm + kSlots * kSlotBytes);
+    uint64_t* empty = full + kSlots;
     const int dx = L.dims[0], dy = L.dims[1], dz = L.dims[2];
     const float h = L.h;
     const float m2h = -2.0f * h, na3 = -(3.0f * h * h);
     const GodunovOneConsts gc = godunov_one_consts(h);
     const size_t plane = (size_t)L.px * dy;
     const int tid = threadIdx.x;
-    const int y0 = blockIdx.x * kXY, z0 = blockIdx.y * kXZ;
+    const int y0 = blockIdx.x * kXY, z0 = blockIdx.y * ZT;
     const int nchunks = (dx + kXC - 1) / kXC;
     if (tid == 0) {
-        for (int s = 0; s < kPS; ++s) {
+        for (int s = 0; s < kSlots; ++s) {
             mbar_init(&full[s], 1);
-            mbar_init(&empty[s], kXThreads / 32);
+            mbar_init(&empty[s], kConsumers / 32);
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();  // the only CTA-wide barrier: the ring's barriers are initialised
-    if (tid >= kXThreads) {
+    if (tid >= kConsumers) {
         // producer warp: one lane issues every chunk's copy
-        if (tid != kXThreads) return;
+        if (tid != kConsumers) return;
         int ci = 0;
         for (; ci < nchunks; ++ci) {
-            const int s = ci % kPS;
-            if (ci >= kPS && !mbar_wait(&empty[s], ((ci / kPS) - 1) & 1, polls)) break;
+            const int s = ci % kSlots;
+            if (ci >= kSlots && !mbar_wait(&empty[s], ((ci / kSlots) - 1) & 1, polls)) break;
             const int c = (DIR > 0) ? ci : (nchunks - 1 - ci);
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-            mbar_expect_tx(&full[s], kTBox * 4);
-            tma_load_3d(tsm + s * kTSlotBytes, &tm, c * kXC, y0 - 1, z0 - 1, &full[s]);
+            mbar_expect_tx(&full[s], XPipe<ZT>::kBox * 4);
+            tma_load_3d(tsm + s * kSlotBytes, &tm, c * kXC, y0 - 1, z0 - 1, &full[s]);
         }
         // let every copy still in flight land before the producer leaves (consumers that gave
         // up have left already); a break means the consumers stopped releasing slots
-        for (int k = max(0, ci - kPS); k < ci; ++k) mbar_wait(&full[k % kPS], (k / kPS) & 1);
+        for (int k = max(0, ci - kSlots); k < ci; ++k) mbar_wait(&full[k % kSlots], (k / kSlots) & 1);
         if (ci < nchunks) atomicAdd(&ds->wait_timeouts, 1ull);
         return;
     }
@@ -591,8 +603,9 @@ __global__ void __launch_bounds__(kPThreads) sweep_x_pipe_kernel(const __grid_co
     bool ch = false;
 #pragma unroll 1
     for (int ci = 0; ci < nchunks; ++ci) {
-        bool ok = mbar_wait(&full[ci % kPS], (ci / kPS) & 1, polls);
-        if (ok && ci + 1 < nchunks) ok = mbar_wait(&full[(ci + 1) % kPS], ((ci + 1) / kPS) & 1, polls);
+        // (chunk ci's own barrier was waited for a chunk ago)
+        bool ok = ci > 0 || mbar_wait(&full[0], 0, polls);
+        if (ok && ci + 1 < nchunks) ok = mbar_wait(&full[(ci + 1) % kSlots], ((ci + 1) / kSlots) & 1, polls);
         if (!__all_sync(0xffffffffu, ok)) {
             if (ty == 0) atomicAdd(&ds->wait_timeouts, 1ull);
             return;
@@ -600,8 +613,8 @@ __global__ void __launch_bounds__(kPThreads) sweep_x_pipe_kernel(const __grid_co
         const int c = (DIR > 0) ? ci : (nchunks - 1 - ci);
         const int xc = c * kXC;
         if (active) {
-            const float* tile = reinterpret_cast<const float*>(tsm + (ci % kPS) * kTSlotBytes);
-            const float* ntile = reinterpret_cast<const float*>(tsm + ((ci + 1) % kPS) * kTSlotBytes);
+            const float* tile = reinterpret_cast<const float*>(tsm + (ci % kSlots) * kSlotBytes);
+            const float* ntile = reinterpret_cast<const float*>(tsm + ((ci + 1) % kSlots) * kSlotBytes);
             float res[kXC];
             if (xc + kXC <= dx && ci + 1 < nchunks) {
                 float cur[kXC], ay[kXC], az[kXC];
@@ -632,7 +645,7 @@ __global__ void __launch_bounds__(kPThreads) sweep_x_pipe_kernel(const __grid_co
                     if constexpr (NB == 2) u = godunov_ref_nbp(fminf(prev, down), ay[j], az[j], gc);
                     else if constexpr (NB == 1) u = godunov_ref_nb(fminf(prev, down), ay[j], az[j], h, m2h, na3);
                     else u = godunov<RULE>(fminf(prev, down), ay[j], az[j], h);
-                    const float out = (u < cur[j]) ? u : cur[j];
+                    const float out = fminf(u, cur[j]);
                     ch |= (u < cur[j]);
                     res[j] = out;
                     prev = out;
@@ -670,7 +683,7 @@ __global__ void __launch_bounds__(kPThreads) sweep_x_pipe_kernel(const __grid_co
         }
         // this warp's last read of chunk ci's slot is done (it was also chunk ci-1's "next")
         __syncwarp();
-        if (ty == 0) mbar_arrive(&empty[ci % kPS]);
+        if (ty == 0) mbar_arrive(&empty[ci % kSlots]);
     }
     mark_changed(ch, &ds->changed[round]);
 }
@@ -1316,75 +1329,212 @@ __global__ void __launch_bounds__(kWVThreads) sweep_walk_vec2_kernel(const __gri
     const bool act = (x < dx) && (r < n_rows);  // dim x is a multiple of 4: the quad is all in
     const GodunovPairConsts gc = godunov_pair_consts(L.h);
     const int m = (tr + 1) * kRowS + 4 * cx + 4;  // 16-byte aligned: kRowS, kSliceS are multiples of 4
-    auto slice_ptr = [&](int s) -> const float* {
-        const int b = s / kWPB, q = s - b * kWPB;
-        const int qb = (DIR > 0) ? q : (kWPB - 1 - q);
-        return reinterpret_cast<const float*>(tsm + (b % kWVS) * kWPSlotBytes) + qb * kSliceS;
-    };
+    // line m of the batch in slot s; slice q of the walk order is kSliceAt(q) floats on
+    auto batch_ptr = [&](int s) { return reinterpret_cast<const float*>(tsm + s * kWPSlotBytes) + m; };
+    constexpr auto kSliceAt = [](int q) { return ((DIR > 0) ? q : (kWPB - 1 - q)) * kSliceS; };
     float prev[4] = {kFarSentinel, kFarSentinel, kFarSentinel, kFarSentinel};
     float cur[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     bool ch = false;
     const long long sstep = (DIR > 0) ? (long long)step_stride : -(long long)step_stride;
     float* p = dst + (size_t)((DIR > 0) ? 0 : n_walk - 1) * step_stride + (size_t)r * row_stride + x;
+    // one slice of the four lines: cs its tile, n4 the next slice's values
+    auto step = [&](const float* cs, const float4& n4) {
+        const float nxt[4] = {n4.x, n4.y, n4.z, n4.w};
+        const float4 rm = *reinterpret_cast<const float4*>(cs - kRowS);
+        const float4 rp = *reinterpret_cast<const float4*>(cs + kRowS);
+        const float xl = cs[-1], xr = cs[4];
+        const float rmv[4] = {rm.x, rm.y, rm.z, rm.w}, rpv[4] = {rp.x, rp.y, rp.z, rp.w};
+        float ax[4], ar[4], al[4], u[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            // no far-sentinel clamps: an out-of-lattice NaN always meets an
+            // in-lattice partner here (dim x a multiple of 4, at least 2 rows)
+            ax[j] = fminf((j == 0) ? xl : cur[j - 1], (j == 3) ? xr : cur[j + 1]);
+            ar[j] = fminf(rmv[j], rpv[j]);
+            al[j] = fminf(prev[j], nxt[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j += 2) {
+            if (AXIS == 2) godunov_ref_pair(ax[j], ar[j], al[j], ax[j + 1], ar[j + 1], al[j + 1], gc, u[j], u[j + 1]);
+            else godunov_ref_pair(ax[j], al[j], ar[j], ax[j + 1], al[j + 1], ar[j + 1], gc, u[j], u[j + 1]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            ch |= u[j] < cur[j];
+            prev[j] = fminf(u[j], cur[j]);
+            cur[j] = nxt[j];
+        }
+        *reinterpret_cast<float4*>(p) = make_float4(prev[0], prev[1], prev[2], prev[3]);
+        p += sstep;
+    };
+    int slot = 0;
 #pragma unroll 1
     for (int b = 0; b < nbatches; ++b) {
-        bool ok = mbar_wait(&full[b % kWVS], (b / kWVS) & 1, polls);
-        if (ok && b + 1 < nbatches) ok = mbar_wait(&full[(b + 1) % kWVS], ((b + 1) / kWVS) & 1, polls);
+        const int next = (slot + 1 == kWVS) ? 0 : slot + 1;
+        // (batch b's own barrier was waited for a batch ago)
+        bool ok = b > 0 || mbar_wait(&full[0], 0, polls);
+        if (ok && b + 1 < nbatches) ok = mbar_wait(&full[next], ((b + 1) / kWVS) & 1, polls);
         if (!__all_sync(0xffffffffu, ok)) {
             if ((tid & 31) == 0) atomicAdd(&ds->wait_timeouts, 1ull);
             return;
         }
-        if (b == 0) {
-            const float4 c = *reinterpret_cast<const float4*>(slice_ptr(0) + m);
-            cur[0] = c.x; cur[1] = c.y; cur[2] = c.z; cur[3] = c.w;
-        }
-#pragma unroll
-        for (int q = 0; q < kWPB; ++q) {
-            const int s = b * kWPB + q;
-            if (s >= n_walk) break;
-            const float* cs = slice_ptr(s);
-            float nxt[4] = {kFarSentinel, kFarSentinel, kFarSentinel, kFarSentinel};
-            if (s + 1 < n_walk) {
-                const float4 n4 = *reinterpret_cast<const float4*>(slice_ptr(s + 1) + m);
-                nxt[0] = n4.x; nxt[1] = n4.y; nxt[2] = n4.z; nxt[3] = n4.w;
+        if (act) {
+            const float *cs = batch_ptr(slot), *ns = batch_ptr(next);
+            auto load = [](const float* q) { return *reinterpret_cast<const float4*>(q); };
+            if (b == 0) {
+                const float4 c = load(cs + kSliceAt(0));
+                cur[0] = c.x; cur[1] = c.y; cur[2] = c.z; cur[3] = c.w;
             }
-            if (act) {
-                const float4 rm = *reinterpret_cast<const float4*>(cs + m - kRowS);
-                const float4 rp = *reinterpret_cast<const float4*>(cs + m + kRowS);
-                const float xl = cs[m - 1], xr = cs[m + 4];
-                const float rmv[4] = {rm.x, rm.y, rm.z, rm.w}, rpv[4] = {rp.x, rp.y, rp.z, rp.w};
-                float ax[4], ar[4], al[4], u[4];
+            if (b + 1 < nbatches) {  // four slices, each with a next one
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    // no far-sentinel clamps: an out-of-lattice NaN always meets an
-                    // in-lattice partner here (dim x a multiple of 4, at least 2 rows)
-                    ax[j] = fminf((j == 0) ? xl : cur[j - 1], (j == 3) ? xr : cur[j + 1]);
-                    ar[j] = fminf(rmv[j], rpv[j]);
-                    al[j] = fminf(prev[j], nxt[j]);
-                }
+                for (int q = 0; q < kWPB; ++q)
+                    step(cs + kSliceAt(q), load(q + 1 < kWPB ? cs + kSliceAt(q + 1) : ns + kSliceAt(0)));
+            } else {
 #pragma unroll
-                for (int j = 0; j < 4; j += 2) {
-                    if (AXIS == 2) godunov_ref_pair(ax[j], ar[j], al[j], ax[j + 1], ar[j + 1], al[j + 1], gc, u[j], u[j + 1]);
-                    else godunov_ref_pair(ax[j], al[j], ar[j], ax[j + 1], al[j + 1], ar[j + 1], gc, u[j], u[j + 1]);
+                for (int q = 0; q < kWPB; ++q) {
+                    const int s = b * kWPB + q;
+                    if (s >= n_walk) break;
+                    const bool more = q + 1 < kWPB && s + 1 < n_walk;
+                    step(cs + kSliceAt(q), more ? load(cs + kSliceAt(q + 1 < kWPB ? q + 1 : q))
+                                                : make_float4(kFarSentinel, kFarSentinel, kFarSentinel, kFarSentinel));
                 }
-                float out[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    out[j] = cur[j];
-                    if (u[j] < cur[j]) {
-                        out[j] = u[j];
-                        ch = true;
-                    }
-                    prev[j] = out[j];
-                }
-                *reinterpret_cast<float4*>(p) = make_float4(out[0], out[1], out[2], out[3]);
             }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) cur[j] = nxt[j];
-            p += sstep;
         }
         __syncwarp();
-        if ((tid & 31) == 0) mbar_arrive(&empty[b % kWVS]);
+        if ((tid & 31) == 0) mbar_arrive(&empty[slot]);
+        slot = next;
+    }
+    mark_changed(ch, &ds->changed[round]);
+}
+
+// ---- y and z walks, TMA batches, one line per thread in narrow tiles --------------------
+// For lattices whose 32 x 16 tiles would leave SMs empty, and for the exact update: tiles of
+// 32 x 4 lines, one line per thread, so that a step costs a warp one update and the SM's four
+// schedulers a warp each, and a ring of eight batches, so that the walk does not wait for the
+// copies. Bound by one warp's chain, about 70 instructions a step at little more than one warp
+// per scheduler (128^3, profiled: stalls on dependent instructions, a third on the shared-memory
+// reads); so nothing but the update depends on the previous step -- the batch's cross
+// neighbours are read and reduced ahead, slot and slice offsets are constants, the result is
+// one minimum -- which took 128^3 from 22.6 to 19.9 us per sweep (four lines per thread: 36.2,
+// and 31.8 after the same change).
+constexpr int kWNR = 4;                                // rows of a tile
+constexpr int kWNThreads = 32 * kWNR + 32;             // 4 consumer warps + 1 producer warp
+constexpr int kWNBox = kWPX * (kWNR + 2) * kWPB;       // floats per batch (960)
+constexpr int kWNSlotBytes = (kWNBox * 4 + 1023) / 1024 * 1024;
+constexpr int kWNS = 8;                                // ring slots
+constexpr size_t kWNSmem = (size_t)kWNS * kWNSlotBytes + 128 + 1024;
+
+// PAIR: the reference's update in packed lanes (godunov_ref_nbp), voxel sizes with pair_sqrt_ok.
+template <int AXIS, int RULE, int DIR, bool PAIR>
+__global__ void __launch_bounds__(kWNThreads) sweep_walk_narrow_kernel(const __grid_constant__ CUtensorMap tm,
+                                                                       float* __restrict__ dst, Lattice L, int round,
+                                                                       DevState* ds) {
+    if (ds->stop) return;
+    const int polls = wait_poll_limit(ds);
+    extern __shared__ unsigned char tsm_raw[];
+    unsigned char* tsm = align1k(tsm_raw);
+    uint64_t* full = reinterpret_cast<uint64_t*>(tsm + kWNS * kWNSlotBytes);
+    uint64_t* empty = full + kWNS;
+    const int dx = L.dims[0], dy = L.dims[1], dz = L.dims[2];
+    const size_t plane = (size_t)L.px * dy;
+    const int n_walk = (AXIS == 2) ? dz : dy;
+    const int n_rows = (AXIS == 2) ? dy : dz;
+    const size_t step_stride = (AXIS == 2) ? plane : (size_t)L.px;
+    const size_t row_stride = (AXIS == 2) ? (size_t)L.px : plane;
+    constexpr int kSliceS = (AXIS == 2) ? (kWNR + 2) * kWPX : kWPX;   // next slice
+    constexpr int kRowS = (AXIS == 2) ? kWPX : kWPB * kWPX;           // next row
+    const int tid = threadIdx.x;
+    const int x0 = blockIdx.x * kWX, r0 = blockIdx.y * kWNR;
+    const int nbatches = (n_walk + kWPB - 1) / kWPB;
+    if (tid == 0) {
+        for (int s = 0; s < kWNS; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], kWNR);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncthreads();
+    if (tid >= 32 * kWNR) {
+        if (tid != 32 * kWNR) return;
+        int b = 0;
+        for (; b < nbatches; ++b) {
+            const int s = b % kWNS;
+            if (b >= kWNS && !mbar_wait(&empty[s], ((b / kWNS) - 1) & 1, polls)) break;
+            const int sl0 = (DIR > 0) ? b * kWPB : n_walk - kWPB - b * kWPB;
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            mbar_expect_tx(&full[s], kWNBox * 4);
+            if (AXIS == 2) tma_load_3d(tsm + s * kWNSlotBytes, &tm, x0 - 4, r0 - 1, sl0, &full[s]);
+            else tma_load_3d(tsm + s * kWNSlotBytes, &tm, x0 - 4, sl0, r0 - 1, &full[s]);
+        }
+        // let every copy still in flight land before the producer leaves (consumers that gave
+        // up have left already); a break means the consumers stopped releasing slots
+        for (int k = max(0, b - kWNS); k < b; ++k) mbar_wait(&full[k % kWNS], (k / kWNS) & 1);
+        if (b < nbatches) atomicAdd(&ds->wait_timeouts, 1ull);
+        return;
+    }
+    const int tx = tid & 31, tr = tid >> 5;
+    const int x = x0 + tx, r = r0 + tr;
+    const bool act = (x < dx) && (r < n_rows);
+    const float h = L.h;
+    const GodunovOneConsts gc = godunov_one_consts(h);
+    const int m = (tr + 1) * kRowS + (tx + 4);
+    // line m of the batch in slot s; slice q of the walk order is kSliceAt(q) floats on
+    auto batch_ptr = [&](int s) { return reinterpret_cast<const float*>(tsm + s * kWNSlotBytes) + m; };
+    constexpr auto kSliceAt = [](int q) { return ((DIR > 0) ? q : (kWPB - 1 - q)) * kSliceS; };
+    float prev = kFarSentinel, cur = 0.0f;
+    bool ch = false;
+    const long long sstep = (DIR > 0) ? (long long)step_stride : -(long long)step_stride;
+    float* p = dst + (size_t)((DIR > 0) ? 0 : n_walk - 1) * step_stride + (size_t)r * row_stride + x;
+    auto step = [&](float ax, float ar, float nxt) {
+        const float al = fminf(prev, nxt);
+        float u;
+        if constexpr (PAIR) u = (AXIS == 2) ? godunov_ref_nbp(ax, ar, al, gc) : godunov_ref_nbp(ax, al, ar, gc);
+        else u = (AXIS == 2) ? godunov<RULE>(ax, ar, al, h) : godunov<RULE>(ax, al, ar, h);
+        ch |= u < cur;
+        prev = fminf(u, cur);
+        cur = nxt;
+        *p = prev;
+        p += sstep;
+    };
+    int slot = 0;
+#pragma unroll 1
+    for (int b = 0; b < nbatches; ++b) {
+        const int next = (slot + 1) & (kWNS - 1);
+        // (batch b's own barrier was waited for a batch ago)
+        bool ok = b > 0 || mbar_wait(&full[0], 0, polls);
+        if (ok && b + 1 < nbatches) ok = mbar_wait(&full[next], ((b + 1) / kWNS) & 1, polls);
+        if (!__all_sync(0xffffffffu, ok)) {
+            if (tx == 0) atomicAdd(&ds->wait_timeouts, 1ull);
+            return;
+        }
+        if (act) {
+            const float *cs = batch_ptr(slot), *ns = batch_ptr(next);
+            if (b == 0) cur = cs[kSliceAt(0)];
+            // the batch's neighbours first: none of them depends on the chain
+            float ax[kWPB], ar[kWPB];
+#pragma unroll
+            for (int q = 0; q < kWPB; ++q) {
+                const float* c = cs + kSliceAt(q);
+                ax[q] = min3f(c[-1], c[1], kFarSentinel);
+                ar[q] = min3f(c[-kRowS], c[kRowS], kFarSentinel);
+            }
+            if (b + 1 < nbatches) {  // four slices, each with a next one
+#pragma unroll
+                for (int q = 0; q < kWPB; ++q)
+                    step(ax[q], ar[q], q + 1 < kWPB ? cs[kSliceAt(q + 1)] : ns[kSliceAt(0)]);
+            } else {
+#pragma unroll
+                for (int q = 0; q < kWPB; ++q) {
+                    const int s = b * kWPB + q;
+                    if (s >= n_walk) break;
+                    const bool more = q + 1 < kWPB && s + 1 < n_walk;
+                    step(ax[q], ar[q], more ? cs[kSliceAt(q + 1 < kWPB ? q + 1 : q)] : kFarSentinel);
+                }
+            }
+        }
+        __syncwarp();
+        if (tx == 0) mbar_arrive(&empty[slot]);
+        slot = next;
     }
     mark_changed(ch, &ds->changed[round]);
 }
@@ -1517,7 +1667,21 @@ void launch_sweep_t(int axis, int round, const float* src, float* dst, const Lat
     // size whose square-root operands stay where nsqrt2_rn is exact
     const bool pair_ok = (RULE == 0) && pair_sqrt_ok(L.h);
     if (wsched == kWTmaVec2 && (!pair_ok || (axis == 2 ? dy : dz) < 2)) wsched = kWTmaVec;
-    if (axis != 0 && wsched == kWTmaVec2) {
+    if (axis != 0 && wsched == kWTmaNarrow) {
+        const int n_rows = (axis == 2) ? dy : dz;
+        dim3 grid((dx + kWX - 1) / kWX, (n_rows + kWNR - 1) / kWNR);
+        auto go = [&](auto kernel, const CUtensorMap& map) {
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWNSmem);
+            kernel<<<grid, kWNThreads, kWNSmem, st>>>(map, dst, L, round, ds);
+        };
+        if (axis == 2) {
+            if (pair_ok) go(sweep_walk_narrow_kernel<2, 0, DIR, true>, src_map->znmap);
+            else go(sweep_walk_narrow_kernel<2, RULE, DIR, false>, src_map->znmap);
+        } else {
+            if (pair_ok) go(sweep_walk_narrow_kernel<1, 0, DIR, true>, src_map->ynmap);
+            else go(sweep_walk_narrow_kernel<1, RULE, DIR, false>, src_map->ynmap);
+        }
+    } else if (axis != 0 && wsched == kWTmaVec2) {
         const int n_rows = (axis == 2) ? dy : dz;
         dim3 grid((dx + kWX - 1) / kWX, (n_rows + kWR - 1) / kWR);
         if (axis == 2) {
@@ -1583,6 +1747,14 @@ void launch_sweep_t(int axis, int round, const float* src, float* dst, const Lat
             sweep_x_wide_kernel<RULE, DIR, false><<<grid, kPThreads, kXWSmem, st>>>(src_map->wmap, dst, L, round,
                                                                                    ds);
         }
+    } else if (xsched == kXTmaNarrow) {
+        dim3 grid((dy + kXY - 1) / kXY, (dz + kXZNarrow - 1) / kXZNarrow);
+        auto go = [&](auto kernel) {
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XPipe<kXZNarrow>::kSmem);
+            kernel<<<grid, XPipe<kXZNarrow>::kThreads, XPipe<kXZNarrow>::kSmem, st>>>(src_map->nmap, dst, L, round, ds);
+        };
+        if (pair_ok) go(sweep_x_pipe_kernel<0, DIR, 2, kXZNarrow>);
+        else go(sweep_x_pipe_kernel<RULE, DIR, 0, kXZNarrow>);
     } else if (xsched == kXTmaPipe || xsched == kXTmaPipe2 || xsched == kXTmaWide) {
         dim3 grid((dy + kXY - 1) / kXY, (dz + kXZ - 1) / kXZ);
         if (pair_ok) {
@@ -1652,6 +1824,11 @@ bool encode_grid_map(GridMap& m, const float* base, const Lattice& L) {
     m.walk_valid = m.valid &&
                    encode_box(&m.ymap, base, dx, dy, dz, L.px, kWPX, kWPB, kWHR, CU_TENSOR_MAP_SWIZZLE_NONE) &&
                    encode_box(&m.zmap, base, dx, dy, dz, L.px, kWPX, kWHR, kWPB, CU_TENSOR_MAP_SWIZZLE_NONE);
+    const bool narrow = encode_box(&m.nmap, base, dx, dy, dz, L.px, kXC, kXHY, kXZNarrow + 2) &&
+                        encode_box(&m.ynmap, base, dx, dy, dz, L.px, kWPX, kWPB, kWNR + 2, CU_TENSOR_MAP_SWIZZLE_NONE) &&
+                        encode_box(&m.znmap, base, dx, dy, dz, L.px, kWPX, kWNR + 2, kWPB, CU_TENSOR_MAP_SWIZZLE_NONE);
+    m.valid = m.valid && narrow;
+    m.walk_valid = m.walk_valid && narrow;
     m.wide_valid = m.valid && encode_box(&m.wmap, base, dx, dy, dz, L.px, kXWB, kXHY, kXHZ,
                                          CU_TENSOR_MAP_SWIZZLE_NONE);
     return m.valid;
