@@ -26,12 +26,14 @@
 //     ambiguous cubes the vertices may be connected differently from the reference's table.
 //
 // Passes:
-//   1. count: crossing mask (3 bits) per voxel, triangles per cube; per-row totals;
-//   2. exclusive scans of the row totals;
-//   3. vertices: row offsets plus within-row prefixes give each voxel's first vertex number
-//      (stored, 4 B per voxel); the vertices are written;
-//   4. triangles: the same for each cube's first triangle; a cube's edge vertex is its
-//      owner voxel's first vertex plus the edge's rank in the owner's mask.
+//   1. inside bits of the grid, words of 32 voxels along x;
+//   2. count: vertices and triangles per word and per block of 256 words; the words that hold
+//      any are listed;
+//   3. a scan of the blocks' totals;
+//   4. emission of the listed words' vertices and triangles; a cube's edge vertex is its owner
+//      word's first vertex plus the crossings before it in the word.
+#include <math_constants.h>
+
 #include <algorithm>
 #include <array>
 #include <cmath>
@@ -53,8 +55,9 @@ constexpr int kCorner[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0}, {0, 0
 constexpr int kEdge[12][2] = {{0, 1}, {1, 2}, {3, 2}, {0, 3}, {4, 5}, {5, 6}, {7, 6}, {4, 7}, {0, 4}, {1, 5}, {2, 6}, {3, 7}};
 constexpr int kFace[6][4] = {{0, 1, 2, 3}, {4, 5, 6, 7}, {0, 1, 5, 4}, {3, 2, 6, 7}, {0, 3, 7, 4}, {1, 2, 6, 5}};
 
-__device__ int8_t c_tri[256][16];  // read with divergent per-lane cases: global memory, L1-cached
-__device__ int8_t c_ntri[256];
+// The table on the device, a case a word: 4 bits an edge from the low end, the number of
+// triangles in the top 4. Read with divergent per-lane cases: global memory, L1-cached.
+__device__ unsigned long long c_tri[256];
 
 int8_t g_tri[256][16];
 std::once_flag g_tri_once;
@@ -195,250 +198,387 @@ void mc_table_init() {
     }
 }
 
-// Work layout: rows are the x lines (y, z), numbered y + z dy; the count pass totals each
-// row, scans over the rows give every row its first vertex and first triangle, and the emit
-// passes number within a row in x order -- so vertices and triangles come in linear voxel
-// order. A CTA takes kGR = 4 consecutive rows of one z plane and walks them in chunks of 128
-// x; a thread takes the 4 voxels at its x, loading their cubes' 20 corner values
-// ((y .. y+4) x (z, z+1) x (x, x+1)) at once. The within-row prefixes of the 4 rows come
-// from one CTA scan of a 64-bit word holding four 16-bit counts (a chunk holds at most
-// 128 x 5 triangles per row).
-constexpr int kIsoThreads = 128;
-constexpr int kGR = 4;
+// Work layout. The grid is read once, into one inside bit per voxel: words of 32 voxels along
+// x, rows padded to whole words, row y + z dy. The mesh hangs on the bits alone -- an edge is
+// crossed where neighbouring bits differ, a cube's case is eight bits -- so everything but the
+// vertex positions works on 1/32 of the grid, and, past the count, only on the words that hold
+// a vertex or a cut cube ("items"). 509 x 480 x 512: 0.32 ms a call (bits 88 us, count 40, scan 6,
+// emission 74); three walks over the grid with 5 B per voxel of masks and vertex numbers between
+// them took 2.40 ms.
+constexpr int kIsoThreads = 256;
+constexpr int kIsoWarps = kIsoThreads / 32;
+constexpr int kIsoChunk = 8;  // words a warp reads at once
 
 struct IsoGeom {
-    int dx, dy, dz, gpz;  // gpz: row groups per z plane
+    int dx, dy, dz, wpr;  // wpr: words per row
+    long long rows, nw;   // rows of the grid, words
     float iso, seal;
+    bool sealed;          // no border voxel is inside
 };
+
+__device__ __forceinline__ long long div_u(long long a, long long range, int b) {  // a / b, a < range
+    return (range >> 32) ? a / b : (long long)((unsigned)a / (unsigned)b);
+}
 
 // value relative to iso, with the reference's border seal
-__device__ __forceinline__ float iso_val(const float* __restrict__ g, int x, int y, int z, const IsoGeom& G) {
-    float v = __ldg(&g[((size_t)z * G.dy + y) * G.dx + x]);
-    if ((x == 0 || x == G.dx - 1 || y == 0 || y == G.dy - 1 || z == 0 || z == G.dz - 1) && v < G.seal) v = G.seal;
+__device__ __forceinline__ float iso_rel(float v, bool border, const IsoGeom& G) {
+    if (border && v < G.seal) v = G.seal;
     return v - G.iso;
 }
+__device__ __forceinline__ float iso_val(const float* __restrict__ g, int x, int y, int z, const IsoGeom& G) {
+    const bool border = x == 0 || x == G.dx - 1 || y == 0 || y == G.dy - 1 || z == 0 || z == G.dz - 1;
+    return iso_rel(__ldg(&g[((size_t)z * G.dy + y) * G.dx + x]), border, G);
+}
 
-struct Quad {
-    int x, y0, z, nr;   // voxels (x, y0 + r, z), r < nr
-    float v[kGR + 1][2][2];  // value at (x + i, y0 + r, z + k): v[r][k][i]
+// 1. inside bits: a warp takes rows, 8 words at a time, eight loads in flight per lane; blocks
+// by (rows, plane), so that no index is divided. A border voxel reads as iso + h at least, so it is
+// outside, unless the sum rounds to iso and nothing changes sides: the seal is a mask on the
+// words. Bound by the read of the grid.
+__global__ void __launch_bounds__(kIsoThreads, 8) iso_bits_kernel(const float* __restrict__ g, IsoGeom G,
+                                                                  unsigned* __restrict__ bits,
+                                                                  unsigned long long* __restrict__ n_items) {
+    if ((blockIdx.x | blockIdx.y | threadIdx.x) == 0) *n_items = 0;
+    const int lane = threadIdx.x & 31, step = gridDim.x * kIsoWarps;
+    for (int z = blockIdx.y; z < G.dz; z += gridDim.y)
+        for (int y = blockIdx.x * kIsoWarps + (threadIdx.x >> 5); y < G.dy; y += step) {
+            const long long row = (long long)z * G.dy + y;
+            const float* p = g + (size_t)row * G.dx + lane;
+            unsigned* out = bits + row * G.wpr + lane;
+            const bool sealed_row = G.sealed && (y == 0 || y == G.dy - 1 || z == 0 || z == G.dz - 1);
+            for (int w0 = 0; w0 < G.wpr; w0 += kIsoChunk, p += 32 * kIsoChunk, out += kIsoChunk) {
+                const int left = sealed_row ? 0 : G.dx - 32 * w0 - lane;  // voxels of the row from this lane's first
+                float v[kIsoChunk];
+                unsigned mine = 0;
+#pragma unroll
+                for (int j = 0; j < kIsoChunk; ++j) v[j] = 32 * j < left ? __ldg(p + 32 * j) : CUDART_NAN_F;
+#pragma unroll
+                for (int j = 0; j < kIsoChunk; ++j) {
+                    const unsigned b = __ballot_sync(0xffffffffu, v[j] - G.iso <= 0.0f);
+                    if (lane == j) mine = b;
+                }
+                if (lane < kIsoChunk && w0 + lane < G.wpr) {
+                    if (G.sealed && w0 + lane == 0) mine &= ~1u;
+                    if (G.sealed && w0 + lane == G.wpr - 1) mine &= ~(1u << ((G.dx - 1) & 31));
+                    *out = mine;
+                }
+            }
+        }
+}
+
+// bits of the voxels with a neighbour at x + 1, among the word's 32
+__device__ __forceinline__ unsigned has_next(const IsoGeom& G, int w) {
+    const int n = G.dx - 1 - 32 * w;
+    return n >= 32 ? ~0u : (1u << n) - 1u;
+}
+__device__ __forceinline__ unsigned shift_in(unsigned s, unsigned next) { return (s >> 1) | (next << 31); }
+
+// case (reference corner order) of the cube at bit l: lo[r][k] the bits of the row y + r,
+// plane z + k, hi the same one voxel on
+__device__ __forceinline__ int cube_case(const unsigned lo[2][2], const unsigned hi[2][2], int l) {
+    auto bit = [l](unsigned s) { return (int)((s >> l) & 1u); };
+    return bit(lo[0][0]) | bit(hi[0][0]) << 1 | bit(hi[1][0]) << 2 | bit(lo[1][0]) << 3 | bit(lo[0][1]) << 4 |
+           bit(hi[0][1]) << 5 | bit(hi[1][1]) << 6 | bit(lo[1][1]) << 7;
+}
+
+// 2. count: a thread a word. Vertices of a word and cut cubes by bit operations; the block's
+// items are packed in order and a thread counts each one's triangles, cube by cube (most words
+// hold a few cubes: with a warp an item, a lane a cube, 58 us at 509 x 480 x 512, this 40). Writes the
+// word's first vertex (within the block of 256 words), the items (word, first triangle within
+// the block; in the order the blocks come -- an item carries all that its emission needs) and
+// the block's totals. Bound by the loads of the bits, which come from L2.
+struct IsoItem {
+    unsigned block, rest;  // rest: word of the block | first triangle << 8 (at most 256 x 160)
 };
 
-__device__ __forceinline__ void group_of(const IsoGeom& G, int& y0, int& z, int& nr) {
-    z = blockIdx.x / G.gpz;
-    y0 = (blockIdx.x - z * G.gpz) * kGR;
-    nr = min(kGR, G.dy - y0);
-}
-
-__device__ __forceinline__ void load_quad(const float* __restrict__ g, const IsoGeom& G, Quad& q) {
-    const int xs = min(q.x, G.dx - 1), x1 = min(q.x + 1, G.dx - 1), z1 = min(q.z + 1, G.dz - 1);
+__global__ void __launch_bounds__(kIsoThreads) iso_count_kernel(IsoGeom G, const unsigned* __restrict__ bits,
+                                                                uint16_t* __restrict__ vpre,
+                                                                uint2* __restrict__ totals,
+                                                                IsoItem* __restrict__ items,
+                                                                unsigned long long* __restrict__ n_items) {
+    __shared__ unsigned s_lo[4][kIsoThreads], s_hi[4][kIsoThreads], s_cut[kIsoThreads];
+    __shared__ unsigned s_warp[2][kIsoWarps];
+    __shared__ uint8_t s_list[kIsoThreads];
+    __shared__ unsigned long long s_base;
+    const int t = threadIdx.x, lane = t & 31, wp = t >> 5;
+    const long long i = (long long)blockIdx.x * kIsoThreads + t;
+    unsigned nv = 0, cut = 0;
+    if (i < G.nw) {
+        const long long row = div_u(i, G.nw, G.wpr);
+        const int w = (int)(i - row * G.wpr);
+        const int z = (int)div_u(row, G.rows, G.dy), y = (int)(row - (long long)z * G.dy);
+        const unsigned nx = has_next(G, w);
+        const bool ny = y + 1 < G.dy, nz = z + 1 < G.dz, nw = w + 1 < G.wpr;
+        unsigned lo[2][2], hi[2][2];
 #pragma unroll
-    for (int r = 0; r <= kGR; ++r) {
-        const int y = min(q.y0 + r, G.dy - 1);
-        q.v[r][0][0] = iso_val(g, xs, y, q.z, G);
-        q.v[r][0][1] = iso_val(g, x1, y, q.z, G);
-        q.v[r][1][0] = iso_val(g, xs, y, z1, G);
-        q.v[r][1][1] = iso_val(g, x1, y, z1, G);
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const unsigned* p = bits + i + (r && ny ? G.wpr : 0) + (k && nz ? (long long)G.dy * G.wpr : 0);
+                lo[r][k] = __ldg(p);
+                hi[r][k] = shift_in(lo[r][k], nw ? __ldg(p + 1) : 0u);
+                s_lo[r + 2 * k][t] = lo[r][k];
+                s_hi[r + 2 * k][t] = hi[r][k];
+            }
+        // (past the last row or plane the neighbour is the row itself, past the last voxel both
+        // bits are 0: no crossing)
+        nv = __popc((lo[0][0] ^ hi[0][0]) & nx) + __popc(lo[0][0] ^ lo[1][0]) + __popc(lo[0][0] ^ lo[0][1]);
+        const unsigned any = lo[0][0] | lo[1][0] | lo[0][1] | lo[1][1] | hi[0][0] | hi[1][0] | hi[0][1] | hi[1][1];
+        const unsigned all = lo[0][0] & lo[1][0] & lo[0][1] & lo[1][1] & hi[0][0] & hi[1][0] & hi[0][1] & hi[1][1];
+        if (ny && nz) cut = any & ~all & nx;
     }
-}
-
-__device__ __forceinline__ bool quad_in(const IsoGeom& G, const Quad& q, int r) { return q.x < G.dx && r < q.nr; }
-
-__device__ __forceinline__ unsigned quad_mask(const IsoGeom& G, const Quad& q, int r) {
-    if (!quad_in(G, q, r)) return 0u;
-    const bool s0 = q.v[r][0][0] <= 0.0f;
-    unsigned m = 0;
-    if (q.x + 1 < G.dx && s0 != (q.v[r][0][1] <= 0.0f)) m |= 1;
-    if (q.y0 + r + 1 < G.dy && s0 != (q.v[r + 1][0][0] <= 0.0f)) m |= 2;
-    if (q.z + 1 < G.dz && s0 != (q.v[r][1][0] <= 0.0f)) m |= 4;
-    return m;
-}
-
-// cube case of the cube at voxel r (reference corner order), -1 when there is no cube
-__device__ __forceinline__ int quad_case(const IsoGeom& G, const Quad& q, int r) {
-    if (!quad_in(G, q, r) || q.x + 1 >= G.dx || q.y0 + r + 1 >= G.dy || q.z + 1 >= G.dz) return -1;
-    const float c[8] = {q.v[r][0][0], q.v[r][0][1], q.v[r + 1][0][1], q.v[r + 1][0][0],
-                        q.v[r][1][0], q.v[r][1][1], q.v[r + 1][1][1], q.v[r + 1][1][0]};
-    int cs = 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-        if (c[i] <= 0.0f) cs |= 1 << i;
-    return cs;
-}
-
-__device__ __forceinline__ int tri_count(int cs) { return cs < 0 ? 0 : __ldg(&c_ntri[cs]); }
-
-// exclusive prefix over the CTA in thread order of a word of four 16-bit counts; the
-// CTA total in *tot
-__device__ __forceinline__ unsigned long long cta_exclusive4(unsigned long long val, unsigned long long* tot) {
-    __shared__ unsigned long long warp_sum[kIsoThreads / 32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    unsigned long long inc = val;
+    s_cut[t] = cut;
+    // prefixes of the vertices and the items over the block, in word order
+    const unsigned act = __ballot_sync(0xffffffffu, nv || cut);
+    unsigned inc = nv;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
+        const unsigned u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
     }
-    if (lane == 31) warp_sum[w] = inc;
-    __syncthreads();
-    unsigned long long before = 0, all = 0;
-#pragma unroll
-    for (int i = 0; i < kIsoThreads / 32; ++i) {
-        if (i < w) before += warp_sum[i];
-        all += warp_sum[i];
-    }
-    __syncthreads();  // warp_sum is reused by the next chunk
-    *tot = all;
-    return before + inc - val;
-}
-
-__device__ __forceinline__ unsigned field(unsigned long long w, int r) { return (unsigned)(w >> (16 * r)) & 0xffffu; }
-
-// 1. masks and per-row totals
-__global__ void __launch_bounds__(kIsoThreads) iso_count_kernel(const float* __restrict__ g, IsoGeom G,
-                                                                uint8_t* __restrict__ mask,
-                                                                unsigned* __restrict__ row_v,
-                                                                unsigned* __restrict__ row_t) {
-    Quad q;
-    group_of(G, q.y0, q.z, q.nr);
-    unsigned tv[kGR] = {0, 0, 0, 0}, tt[kGR] = {0, 0, 0, 0};
-    for (int x0 = 0; x0 < G.dx; x0 += kIsoThreads) {
-        q.x = x0 + threadIdx.x;
-        load_quad(g, G, q);
-#pragma unroll
-        for (int r = 0; r < kGR; ++r) {
-            const unsigned m = quad_mask(G, q, r);
-            if (quad_in(G, q, r)) mask[((size_t)q.z * G.dy + q.y0 + r) * G.dx + q.x] = (uint8_t)m;
-            tv[r] += __popc(m);
-            tt[r] += tri_count(quad_case(G, q, r));
-        }
-    }
-    __shared__ unsigned red[2 * kGR][kIsoThreads / 32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int r = 0; r < kGR; ++r) {
-        unsigned a = tv[r], b = tt[r];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            a += __shfl_down_sync(0xffffffffu, a, o);
-            b += __shfl_down_sync(0xffffffffu, b, o);
-        }
-        if (lane == 0) {
-            red[r][w] = a;
-            red[kGR + r][w] = b;
-        }
+    if (lane == 31) {
+        s_warp[0][wp] = inc;
+        s_warp[1][wp] = __popc(act);
     }
     __syncthreads();
-    if (threadIdx.x < q.nr) {
-        unsigned a = 0, b = 0;
-        for (int i = 0; i < kIsoThreads / 32; ++i) {
-            a += red[threadIdx.x][i];
-            b += red[kGR + threadIdx.x][i];
+    unsigned vb = 0, ab = 0, vt = 0, na = 0;
+#pragma unroll
+    for (int k = 0; k < kIsoWarps; ++k) {
+        if (k < wp) {
+            vb += s_warp[0][k];
+            ab += s_warp[1][k];
         }
-        const size_t row = (size_t)q.z * G.dy + q.y0 + threadIdx.x;
-        row_v[row] = a;
-        row_t[row] = b;
+        vt += s_warp[0][k];
+        na += s_warp[1][k];
+    }
+    if (na == 0) {
+        if (t == 0) totals[blockIdx.x] = make_uint2(0u, 0u);
+        return;
+    }
+    if (i < G.nw) vpre[i] = (uint16_t)(vb + inc - nv);
+    if (nv || cut) s_list[ab + __popc(act & ((1u << lane) - 1u))] = (uint8_t)t;
+    __syncthreads();
+    unsigned nt = 0;
+    if ((unsigned)t < na) {  // a thread an item
+        const int l = s_list[t];
+        const unsigned lo[2][2] = {{s_lo[0][l], s_lo[2][l]}, {s_lo[1][l], s_lo[3][l]}};
+        const unsigned hi[2][2] = {{s_hi[0][l], s_hi[2][l]}, {s_hi[1][l], s_hi[3][l]}};
+        for (unsigned c = s_cut[l]; c; c &= c - 1)
+            nt += (unsigned)(__ldg(&c_tri[cube_case(lo, hi, __ffs(c) - 1)]) >> 60);
+    }
+    inc = nt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
+    }
+    if (lane == 31) s_warp[0][wp] = inc;  // (its readers are past the barriers above)
+    __syncthreads();
+    unsigned tb = 0, tt = 0;
+#pragma unroll
+    for (int k = 0; k < kIsoWarps; ++k) {
+        if (k < wp) tb += s_warp[0][k];
+        tt += s_warp[0][k];
+    }
+    if (t == 0) {
+        s_base = atomicAdd(n_items, (unsigned long long)na);
+        totals[blockIdx.x] = make_uint2(vt, tt);
+    }
+    __syncthreads();
+    if ((unsigned)t < na) items[s_base + t] = IsoItem{blockIdx.x, (unsigned)s_list[t] | (tb + inc - nt) << 8};
+}
+
+// 3. the blocks' first vertex and triangle, and the mesh's totals (sum[0], sum[1]). At most one
+// CTA per SM; each adds up the blocks before its own share itself, which at 15,360 blocks (509 x
+// 480 x 512) is 15 loads a thread against a second launch or a wait on its neighbours (one CTA
+// over all blocks: 16 us).
+constexpr int kScanThreads = 1024;
+__device__ __forceinline__ unsigned long long warp_inclusive(unsigned long long v) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long u = __shfl_up_sync(0xffffffffu, v, o);
+        if ((threadIdx.x & 31) >= o) v += u;
+    }
+    return v;
+}
+__global__ void __launch_bounds__(kScanThreads) iso_scan_kernel(const uint2* __restrict__ totals, long long n,
+                                                                long long share, ulonglong2* __restrict__ first,
+                                                                unsigned long long* __restrict__ sum) {
+    __shared__ unsigned long long s_w[2][32];
+    const int t = threadIdx.x, lane = t & 31, wp = t >> 5;
+    const long long begin = blockIdx.x * share, end = min(n, begin + share);
+    unsigned long long cv = 0, ct = 0;  // before the share
+    for (long long i = t; i < begin; i += kScanThreads) {
+        const uint2 q = __ldg(&totals[i]);
+        cv += q.x;
+        ct += q.y;
+    }
+    // inclusive over the CTA; the last one of s_w is the total
+    auto scan = [&](unsigned long long& v, unsigned long long& u) {
+        v = warp_inclusive(v);
+        u = warp_inclusive(u);
+        __syncthreads();  // s_w's last readers
+        if (lane == 31) {
+            s_w[0][wp] = v;
+            s_w[1][wp] = u;
+        }
+        __syncthreads();
+        if (wp < 2) s_w[wp][lane] = warp_inclusive(s_w[wp][lane]);
+        __syncthreads();
+        if (wp) {
+            v += s_w[0][wp - 1];
+            u += s_w[1][wp - 1];
+        }
+    };
+    scan(cv, ct);
+    cv = s_w[0][31];
+    ct = s_w[1][31];
+    for (long long b0 = begin; b0 < end; b0 += kScanThreads) {
+        const long long i = b0 + t;
+        const uint2 q = i < end ? __ldg(&totals[i]) : make_uint2(0u, 0u);
+        unsigned long long v = q.x, u = q.y;
+        scan(v, u);
+        if (i < end) first[i] = make_ulonglong2(cv + v - q.x, ct + u - q.y);
+        cv += s_w[0][31];
+        ct += s_w[1][31];
+    }
+    if (t == 0 && end == n) {
+        sum[0] = cv;
+        sum[1] = ct;
     }
 }
 
-// 3. vertex numbers and positions
-__global__ void __launch_bounds__(kIsoThreads) iso_vertex_kernel(const float* __restrict__ g, IsoGeom G, float h,
-                                                                 float ox, float oy, float oz,
-                                                                 const unsigned long long* __restrict__ row_vpos,
-                                                                 uint32_t* __restrict__ vbase,
-                                                                 float* __restrict__ out_v) {
-    Quad q;
-    group_of(G, q.y0, q.z, q.nr);
-    unsigned long long carry[kGR];
-#pragma unroll
-    for (int r = 0; r < kGR; ++r)
-        carry[r] = (r < q.nr) ? row_vpos[(size_t)q.z * G.dy + q.y0 + r] : 0ull;
-    const float pz = oz + (float)q.z * h;
-    for (int x0 = 0; x0 < G.dx; x0 += kIsoThreads) {
-        q.x = x0 + threadIdx.x;
-        load_quad(g, G, q);
-        unsigned m[kGR];
-        unsigned long long word = 0;
-#pragma unroll
-        for (int r = 0; r < kGR; ++r) {
-            m[r] = quad_mask(G, q, r);
-            word |= (unsigned long long)__popc(m[r]) << (16 * r);
-        }
-        unsigned long long tot;
-        const unsigned long long pre = cta_exclusive4(word, &tot);
-        const float px = ox + (float)q.x * h;
-#pragma unroll
-        for (int r = 0; r < kGR; ++r) {
-            if (quad_in(G, q, r)) {
-                const unsigned long long base = carry[r] + field(pre, r);
-                vbase[((size_t)q.z * G.dy + q.y0 + r) * G.dx + q.x] = (uint32_t)base;
-                const float v0 = q.v[r][0][0];
-                const float py = oy + (float)(q.y0 + r) * h;
-                unsigned long long n = base;
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    if (!((m[r] >> a) & 1)) continue;
-                    const float v1 = (a == 0) ? q.v[r][0][1] : (a == 1) ? q.v[r + 1][0][0] : q.v[r][1][0];
-                    const float den = v0 - v1;
-                    const float t = (fabsf(den) > 1e-7f) ? fminf(fmaxf(v0 / den, 0.001f), 0.999f) : 0.5f;
-                    float* o = out_v + 3ull * n;
-                    o[0] = (a == 0) ? px + t * h : px;
-                    o[1] = (a == 1) ? py + t * h : py;
-                    o[2] = (a == 2) ? pz + t * h : pz;
-                    ++n;
-                }
+// 4. emission: a thread an item, the vertices in blocks of their own (blockIdx.y). The bits around the word (rows y .. y + 2, planes z .. z + 2)
+// give the crossing masks of the words that own its cubes' edges, and these, with the words'
+// first vertices, every edge's vertex number. Most words hold a few cubes in a row of 32, which
+// is why a thread walks them: a warp an item, a lane a voxel, spent 800 instructions an item and
+// 346 us at 509 x 480 x 512, this 74 (88 with both kinds in one thread). Bound by latency: two rounds of loads, then the grid's values at the
+// crossings.
+constexpr int kEmitThreads = 128;
+__global__ void __launch_bounds__(kEmitThreads) iso_emit_kernel(const float* __restrict__ g, IsoGeom G, float h,
+                                                                float ox, float oy, float oz,
+                                                                const unsigned* __restrict__ bits,
+                                                                const uint16_t* __restrict__ vpre,
+                                                                const ulonglong2* __restrict__ first,
+                                                                const IsoItem* __restrict__ items, long long n_items,
+                                                                float* __restrict__ out_v,
+                                                                uint32_t* __restrict__ out_i) {
+    __shared__ unsigned s_id[12][kEmitThreads];  // a cube's vertex numbers, by edge
+    const int t = threadIdx.x;
+    const long long it = (long long)blockIdx.x * kEmitThreads + t;
+    if (it >= n_items) return;
+    const IsoItem item = items[it];
+    const long long i = (long long)item.block * kIsoThreads + (item.rest & 0xffu);
+    const long long row = div_u(i, G.nw, G.wpr);
+    const int w = (int)(i - row * G.wpr);
+    const int z = (int)div_u(row, G.rows, G.dy), y = (int)(row - (long long)z * G.dy);
+    const int ry = G.dy - 1 - y, rz = G.dz - 1 - z;  // rows and planes past this one
+    const unsigned nx = has_next(G, w);
+    // the word r rows and k planes on (past the last, the last one's own)
+    auto at = [&](int r, int k) { return i + min(r, ry) * (long long)G.wpr + min(k, rz) * ((long long)G.dy * G.wpr); };
+    auto word = [&](int r, int k, int n) { return w + n < G.wpr ? __ldg(&bits[at(r, k) + n]) : 0u; };
+    auto number = [&](int r, int k, int n) {  // fewer than 2^32 vertices; unused where the word has none
+        const long long j = at(r, k) + n;
+        return w + n < G.wpr ? (unsigned)first[j / kIsoThreads].x + vpre[j] : 0u;
+    };
+    if (blockIdx.y == 0) {  // vertices: this word's own edges, in voxel order
+        const unsigned s = word(0, 0, 0);
+        const unsigned mx = (s ^ shift_in(s, word(0, 0, 1))) & nx, my = s ^ word(1, 0, 0), mz = s ^ word(0, 1, 0);
+        const float py = oy + (float)y * h, pz = oz + (float)z * h;
+        float* o = out_v + 3ull * number(0, 0, 0);
+        for (unsigned m = mx | my | mz; m; m &= m - 1) {
+            const int l = __ffs(m) - 1, x = 32 * w + l;
+            const float px = ox + (float)x * h;
+            const float v0 = iso_val(g, x, y, z, G);
+            auto cross = [&](float v1) {
+                const float den = v0 - v1;
+                return (fabsf(den) > 1e-7f) ? fminf(fmaxf(v0 / den, 0.001f), 0.999f) : 0.5f;
+            };
+            if ((mx >> l) & 1u) {
+                o[0] = px + cross(iso_val(g, x + 1, y, z, G)) * h;
+                o[1] = py;
+                o[2] = pz;
+                o += 3;
             }
-            carry[r] += field(tot, r);
+            if ((my >> l) & 1u) {
+                o[0] = px;
+                o[1] = py + cross(iso_val(g, x, y + 1, z, G)) * h;
+                o[2] = pz;
+                o += 3;
+            }
+            if ((mz >> l) & 1u) {
+                o[0] = px;
+                o[1] = py;
+                o[2] = pz + cross(iso_val(g, x, y, z + 1, G)) * h;
+                o += 3;
+            }
         }
+        return;
     }
-}
-
-// 4. triangles: edge e of the cube at (x, y, z) belongs to voxel (x, y, z) + c_owner[e]
-// along axis c_axis[e]
-__constant__ int c_owner[12][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 0}, {0, 0, 1}, {1, 0, 1},
-                                   {0, 1, 1}, {0, 0, 1}, {0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0}};
-__constant__ int c_axis[12] = {0, 1, 0, 1, 0, 1, 0, 1, 2, 2, 2, 2};
-
-__global__ void __launch_bounds__(kIsoThreads) iso_triangle_kernel(const float* __restrict__ g, IsoGeom G,
-                                                                   const uint8_t* __restrict__ mask,
-                                                                   const uint32_t* __restrict__ vbase,
-                                                                   const unsigned long long* __restrict__ row_tpos,
-                                                                   uint32_t* __restrict__ out_i) {
-    Quad q;
-    group_of(G, q.y0, q.z, q.nr);
-    unsigned long long carry[kGR];
+    // triangles
+    if (ry == 0 || rz == 0) return;
+    unsigned lo[2][2], hi[2][2], mx[2][2], my[2][2], mz[2][2], f[2][2];
 #pragma unroll
-    for (int r = 0; r < kGR; ++r)
-        carry[r] = (r < q.nr) ? row_tpos[(size_t)q.z * G.dy + q.y0 + r] : 0ull;
-    const long long sy = G.dx, sz = (long long)G.dx * G.dy;
-    for (int x0 = 0; x0 < G.dx; x0 += kIsoThreads) {
-        q.x = x0 + threadIdx.x;
-        load_quad(g, G, q);
-        int cs[kGR];
-        unsigned long long word = 0;
+    for (int k = 0; k < 2; ++k)
 #pragma unroll
-        for (int r = 0; r < kGR; ++r) {
-            cs[r] = quad_case(G, q, r);
-            word |= (unsigned long long)tri_count(cs[r]) << (16 * r);
+        for (int r = 0; r < 2; ++r) {
+            lo[r][k] = word(r, k, 0);
+            hi[r][k] = shift_in(lo[r][k], word(r, k, 1));
+            f[r][k] = number(r, k, 0);
         }
-        unsigned long long tot;
-        const unsigned long long pre = cta_exclusive4(word, &tot);
 #pragma unroll
-        for (int r = 0; r < kGR; ++r) {
-            const int nt = (int)field(word, r);
-            if (nt) {
-                uint32_t* o = out_i + 3ull * (carry[r] + field(pre, r));
-                const long long v = ((long long)q.z * G.dy + q.y0 + r) * G.dx + q.x;
-                for (int j = 0; j < 3 * nt; ++j) {
-                    const int e = __ldg(&c_tri[cs[r]][j]);
-                    const long long w = v + c_owner[e][0] + c_owner[e][1] * sy + c_owner[e][2] * sz;
-                    const unsigned mw = mask[w];
-                    const int a = c_axis[e];
-                    const unsigned rank = (a == 0) ? 0u : (a == 1) ? (mw & 1u) : (unsigned)__popc(mw & 3u);
-                    o[j] = vbase[w] + rank;
-                }
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            mx[r][k] = (lo[r][k] ^ hi[r][k]) & nx;
+            my[r][k] = lo[r][k] ^ (r ? word(2, k, 0) : lo[1][k]);
+            mz[r][k] = lo[r][k] ^ (k ? word(r, 2, 0) : lo[r][1]);
+        }
+    const unsigned any = lo[0][0] | lo[1][0] | lo[0][1] | lo[1][1] | hi[0][0] | hi[1][0] | hi[0][1] | hi[1][1];
+    const unsigned all = lo[0][0] & lo[1][0] & lo[0][1] & lo[1][1] & hi[0][0] & hi[1][0] & hi[0][1] & hi[1][1];
+    uint32_t* o = out_i + 3ull * (first[item.block].y + (item.rest >> 8));
+    for (unsigned m = any & ~all & nx; m; m &= m - 1) {
+        const int l = __ffs(m) - 1;
+        const unsigned below = (1u << l) - 1u;
+        unsigned c[2][2], bx[2][2], by[2][2], c1[2][2], bx1[2][2], by1[2][2];  // first vertices of voxels l, l + 1
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                c[r][k] = f[r][k] + __popc(mx[r][k] & below) + __popc(my[r][k] & below) + __popc(mz[r][k] & below);
+                bx[r][k] = (mx[r][k] >> l) & 1u;
+                by[r][k] = (my[r][k] >> l) & 1u;
+                if (r == 1 && k == 1) continue;
+                c1[r][k] = c[r][k] + bx[r][k] + by[r][k] + ((mz[r][k] >> l) & 1u);
+                bx1[r][k] = (mx[r][k] >> l >> 1) & 1u;  // (l = 31: below)
+                by1[r][k] = (my[r][k] >> l >> 1) & 1u;
             }
-            carry[r] += field(tot, r);
+        if (l == 31) {  // voxel l + 1 is the next word's first
+            const bool next_x = 32 * w + 33 < G.dx;
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    if (r == 1 && k == 1) continue;
+                    const unsigned n = word(r, k, 1);
+                    c1[r][k] = number(r, k, 1);
+                    bx1[r][k] = next_x ? (n ^ (n >> 1)) & 1u : 0u;
+                    by1[r][k] = (n ^ word(r + 1, k, 1)) & 1u;
+                }
         }
+        s_id[0][t] = c[0][0];
+        s_id[1][t] = c1[0][0] + bx1[0][0];
+        s_id[2][t] = c[1][0];
+        s_id[3][t] = c[0][0] + bx[0][0];
+        s_id[4][t] = c[0][1];
+        s_id[5][t] = c1[0][1] + bx1[0][1];
+        s_id[6][t] = c[1][1];
+        s_id[7][t] = c[0][1] + bx[0][1];
+        s_id[8][t] = c[0][0] + bx[0][0] + by[0][0];
+        s_id[9][t] = c1[0][0] + bx1[0][0] + by1[0][0];
+        s_id[10][t] = c1[1][0] + bx1[1][0] + by1[1][0];
+        s_id[11][t] = c[1][0] + bx[1][0] + by[1][0];
+        unsigned long long tri = __ldg(&c_tri[cube_case(lo, hi, l)]);
+        for (unsigned j = 3 * (unsigned)(tri >> 60); j; --j, tri >>= 4) *o++ = s_id[tri & 15u][t];
     }
 }
 
@@ -516,6 +656,7 @@ struct IsoErr {
 // one lattice, allocate nothing. Calls on one device hold its lock for their duration.
 struct IsoCache {
     std::mutex mu;
+    bool table = false;    // the device holds the triangle table
     void* base = nullptr;  // scratch
     size_t bytes = 0;
     void* out = nullptr;   // library-owned mesh (gbsdf_extract_iso_surface_device)
@@ -557,13 +698,17 @@ struct IsoScratch {
 
 bool table_to_device() {
     std::call_once(g_tri_once, mc_table_init);
-    int8_t n[256];
+    unsigned long long t[256];
     for (int cs = 0; cs < 256; ++cs) {
-        n[cs] = 0;
-        while (n[cs] < 5 && g_tri[cs][3 * n[cs]] >= 0) ++n[cs];
+        unsigned long long n = 0;
+        t[cs] = 0;
+        while (n < 5 && g_tri[cs][3 * n] >= 0) {
+            for (int k = 0; k < 3; ++k) t[cs] |= (unsigned long long)g_tri[cs][3 * n + k] << (4 * (3 * n + k));
+            ++n;
+        }
+        t[cs] |= n << 60;
     }
-    return cudaMemcpyToSymbol(c_tri, g_tri, sizeof(g_tri)) == cudaSuccess &&
-           cudaMemcpyToSymbol(c_ntri, n, sizeof(n)) == cudaSuccess;
+    return cudaMemcpyToSymbol(c_tri, t, sizeof(t)) == cudaSuccess;
 }
 
 }  // namespace
@@ -574,6 +719,7 @@ void release_iso_workspace(int device) {
     if (g_iso[device].base) cudaFree(g_iso[device].base);
     if (g_iso[device].out) cudaFree(g_iso[device].out);
     g_iso[device].base = g_iso[device].out = nullptr;
+    g_iso[device].table = false;
     g_iso[device].bytes = g_iso[device].out_bytes = 0;
 }
 
@@ -607,35 +753,40 @@ static int extract_iso(const float* grid, int32_t grid_on_device, const int32_t 
         cudaGetLastError();
         return e.set(GBSDF_ECUDA, "cudaSetDevice failed");
     }
-    if (!table_to_device()) {
-        cudaGetLastError();
-        return e.set(GBSDF_ECUDA, "triangle table upload failed");
-    }
     const long long N = (long long)dx * dy * dz;
-    const int gpz = (dy + kGR - 1) / kGR;  // row groups per z plane
-    const long long groups = (long long)gpz * dz;
-    const long long tiles = (long long)dy * dz;  // rows: the units of the scans
+    const long long groups = (long long)((dy + 3) / 4) * dz;
     if (groups > 0x7fffffffLL) return e.set(GBSDF_EINVAL, "lattice too large (%lld row groups)", groups);
-    const IsoGeom G{dx, dy, dz, gpz, iso_value, iso_value + voxel_size};
+    const int wpr = (dx + 31) / 32;
+    const IsoGeom G{dx, dy, dz, wpr, (long long)dy * dz, (long long)dy * dz * wpr, iso_value, iso_value + voxel_size,
+                    !(iso_value + voxel_size - iso_value <= 0.0f)};
+    const long long blocks = (G.nw + kIsoThreads - 1) / kIsoThreads;
     cudaError_t ce = cudaSuccess;
     std::lock_guard<std::mutex> lock(g_iso[device].mu);
+    if (!g_iso[device].table) {
+        if (!table_to_device()) {
+            cudaGetLastError();
+            return e.set(GBSDF_ECUDA, "triangle table upload failed");
+        }
+        g_iso[device].table = true;
+    }
     IsoScratch s{g_iso[device]};
     // two passes over the same carving: sizing, then placing
     const float* g = grid;
     float* d_up = nullptr;
-    uint8_t* d_mask = nullptr;
-    unsigned *d_tv = nullptr, *d_tt = nullptr;
-    unsigned long long *d_pv = nullptr, *d_pt = nullptr, *d_scan = nullptr;
-    uint32_t* d_vbase = nullptr;
+    unsigned* d_bits = nullptr;
+    uint16_t* d_vpre = nullptr;
+    uint2* d_tot = nullptr;
+    ulonglong2* d_first = nullptr;
+    IsoItem* d_items = nullptr;
+    unsigned long long* d_sum = nullptr;  // vertices, triangles, items
     for (int pass = 0; pass < 2; ++pass) {
         if (!grid_on_device) d_up = s.get<float>((size_t)N, ce);
-        d_mask = s.get<uint8_t>((size_t)N, ce);
-        d_tv = s.get<unsigned>((size_t)tiles, ce);
-        d_tt = s.get<unsigned>((size_t)tiles, ce);
-        d_pv = s.get<unsigned long long>((size_t)tiles + 1, ce);
-        d_pt = s.get<unsigned long long>((size_t)tiles + 1, ce);
-        d_scan = s.get<unsigned long long>((size_t)scan_tmp_elems(tiles), ce);
-        d_vbase = s.get<uint32_t>((size_t)N, ce);
+        d_bits = s.get<unsigned>((size_t)G.nw, ce);
+        d_vpre = s.get<uint16_t>((size_t)G.nw, ce);
+        d_tot = s.get<uint2>((size_t)blocks, ce);
+        d_first = s.get<ulonglong2>((size_t)blocks, ce);
+        d_items = s.get<IsoItem>((size_t)G.nw, ce);
+        d_sum = s.get<unsigned long long>(3, ce);
         if (pass == 0) ce = s.commit();
     }
     if (ce != cudaSuccess) {
@@ -648,21 +799,24 @@ static int extract_iso(const float* grid, int32_t grid_on_device, const int32_t 
         if (ce != cudaSuccess) return e.set(GBSDF_ECUDA, "grid upload: %s", cudaGetErrorString(ce));
         g = d_up;
     }
+    // about 64 CTAs per SM (16 read the grid 10% slower), one a plane at least
+    const int by = std::min(dz, 65535), rows8 = (dy + kIsoWarps - 1) / kIsoWarps;
+    const int bx = std::max(1, std::min(rows8, (152 * 64 + by - 1) / by));
     GBSDF_COUNT_LAUNCH();
-    iso_count_kernel<<<(unsigned)groups, kIsoThreads, 0, st>>>(g, G, d_mask, d_tv, d_tt);
-    launch_exclusive_scan(d_tv, d_pv, tiles, d_scan, 0, st);
-    launch_exclusive_scan(d_tt, d_pt, tiles, d_scan, 0, st);
+    iso_bits_kernel<<<dim3(bx, by), kIsoThreads, 0, st>>>(g, G, d_bits, d_sum + 2);
+    GBSDF_COUNT_LAUNCH();
+    iso_count_kernel<<<(unsigned)blocks, kIsoThreads, 0, st>>>(G, d_bits, d_vpre, d_tot, d_items, d_sum + 2);
+    GBSDF_COUNT_LAUNCH();
+    const long long share = std::max<long long>((blocks + 151) / 152, kScanThreads);
+    iso_scan_kernel<<<(unsigned)((blocks + share - 1) / share), kScanThreads, 0, st>>>(d_tot, blocks, share, d_first,
+                                                                                      d_sum);
     ce = cudaGetLastError();  // launch errors are not reported by the synchronisation
     if (ce != cudaSuccess) return e.set(GBSDF_ECUDA, "iso-surface count launch: %s", cudaGetErrorString(ce));
-    unsigned long long pv = 0, pt = 0;
-    unsigned lv = 0, lt = 0;
-    cudaMemcpyAsync(&pv, d_pv + (tiles - 1), 8, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(&pt, d_pt + (tiles - 1), 8, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(&lv, d_tv + (tiles - 1), 4, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(&lt, d_tt + (tiles - 1), 4, cudaMemcpyDeviceToHost, st);
+    unsigned long long sum[3] = {0, 0, 0};
+    cudaMemcpyAsync(sum, d_sum, sizeof(sum), cudaMemcpyDeviceToHost, st);
     ce = cudaStreamSynchronize(st);
     if (ce != cudaSuccess) return e.set(GBSDF_ECUDA, "iso-surface count: %s", cudaGetErrorString(ce));
-    const long long V = (long long)(pv + lv), T = (long long)(pt + lt);
+    const long long V = (long long)sum[0], T = (long long)sum[1], n_items = (long long)sum[2];
     *n_vertices = V;
     *n_indices = 3 * T;
     if (V > 0xffffffffLL) return e.set(GBSDF_EINVAL, "%lld vertices exceed 32-bit indices", V);
@@ -714,10 +868,8 @@ static int extract_iso(const float* grid, int32_t grid_on_device, const int32_t 
         }
     } free_stage{stage};
     GBSDF_COUNT_LAUNCH();
-    iso_vertex_kernel<<<(unsigned)groups, kIsoThreads, 0, st>>>(g, G, voxel_size, origin[0], origin[1], origin[2],
-                                                               d_pv, d_vbase, d_v);
-    GBSDF_COUNT_LAUNCH();
-    iso_triangle_kernel<<<(unsigned)groups, kIsoThreads, 0, st>>>(g, G, d_mask, d_vbase, d_pt, d_i);
+    iso_emit_kernel<<<dim3((unsigned)((n_items + kEmitThreads - 1) / kEmitThreads), 2), kEmitThreads, 0, st>>>(
+        g, G, voxel_size, origin[0], origin[1], origin[2], d_bits, d_vpre, d_first, d_items, n_items, d_v, d_i);
     ce = cudaGetLastError();
     if (ce == cudaSuccess && !outputs_on_device) {
         ce = cudaMemcpyAsync(out_vertices, d_v, (size_t)V * 12, cudaMemcpyDeviceToHost, st);
