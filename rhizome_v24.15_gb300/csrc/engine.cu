@@ -992,6 +992,7 @@ void gbsdf_release_workspace(int32_t device) {
     std::lock_guard<std::mutex> lk(g_ws[device].mu);
     free_ws(g_ws[device]);
     release_iso_workspace(device);
+    release_io_workspace(device);
 }
 
 int gbsdf_selftest(int32_t which, int32_t device, uint64_t* result, char* err, size_t errlen) {

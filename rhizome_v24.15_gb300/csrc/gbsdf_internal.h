@@ -120,6 +120,7 @@ void launch_exclusive_scan(const unsigned* in, unsigned long long* out, long lon
 long long scan_tmp_elems(long long n);
 // Frees the iso-surface extractor's cached scratch of `device` (k_iso.cu).
 void release_iso_workspace(int device);
+void release_io_workspace(int device);
 // With `ds`, the pair lists are known to hold `cap_b` / `cap_s` entries: when the counts
 // of this SDF build exceed them the fills write nothing and ds->overflow is set (the splat and
 // parity passes then skip the build).

@@ -32,10 +32,11 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
-#include <vector>
+#include <mutex>
 
 #include "../../include/gbsdf.h"
 #include "gbsdf_internal.h"
+#include "io_scratch.h"
 
 namespace gbsdf {
 namespace {
@@ -350,21 +351,6 @@ struct IErr {
     }
 };
 
-// Device allocations of one call, freed on every exit.
-struct Scratch {
-    std::vector<void*> ptrs;
-    ~Scratch() {
-        for (void* p : ptrs) cudaFree(p);
-    }
-    template <class T>
-    T* get(size_t count, cudaError_t& err) {
-        void* p = nullptr;
-        if (err == cudaSuccess) err = cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T));
-        if (err == cudaSuccess) ptrs.push_back(p);
-        return static_cast<T*>(p);
-    }
-};
-
 // ---- ASCII STL ----------------------------------------------------------------------
 // "vertex" token flags (gpu_find_ascii_stl_vertices_kernel, cuda_mesh_io.cu:1094-1118): at
 // the text start or after a space, tab, CR or LF, followed by a space or tab, and starting
@@ -418,7 +404,54 @@ int set_device(int32_t device, IErr& e) {
     return GBSDF_OK;
 }
 
+struct IoBlock {
+    std::mutex mu;
+    bool taken = false;
+    void* base = nullptr;
+    size_t bytes = 0;
+};
+IoBlock g_io[64];
+
 }  // namespace
+
+bool io_block_take(int device, void** base, size_t* bytes) {
+    if (device < 0 || device >= 64) return false;
+    IoBlock& b = g_io[device];
+    std::lock_guard<std::mutex> lock(b.mu);
+    if (b.taken) return false;
+    b.taken = true;
+    *base = b.base;
+    *bytes = b.bytes;
+    return true;
+}
+
+void io_block_give(int device, size_t want) {
+    IoBlock& b = g_io[device];
+    std::lock_guard<std::mutex> lock(b.mu);
+    if (want > b.bytes) {
+        if (b.base) cudaFree(b.base);
+        b.base = nullptr;
+        b.bytes = 0;
+        if (cudaMalloc(&b.base, want) == cudaSuccess) {
+            b.bytes = want;
+        } else {
+            cudaGetLastError();
+            b.base = nullptr;
+        }
+    }
+    b.taken = false;
+}
+
+void release_io_workspace(int device) {
+    if (device < 0 || device >= 64) return;
+    IoBlock& b = g_io[device];
+    std::lock_guard<std::mutex> lock(b.mu);
+    if (b.taken) return;  // a call in flight keeps its block
+    if (b.base) cudaFree(b.base);
+    b.base = nullptr;
+    b.bytes = 0;
+}
+
 }  // namespace gbsdf
 
 using namespace gbsdf;
@@ -449,7 +482,7 @@ int gbsdf_parse_binary_stl(const uint8_t* bytes, size_t n_bytes, float* out_vert
     uint32_t cap = 1024;
     while ((long long)cap < 2 * n) cap <<= 1;
     cudaError_t ce = cudaSuccess;
-    Scratch s;
+    IoScratch s(device);
     uint8_t* d_payload = s.get<uint8_t>((size_t)T * 50, ce);
     float* d_raw = s.get<float>((size_t)n * 3, ce);
     float* d_norm = s.get<float>((size_t)T * 3, ce);
@@ -519,7 +552,7 @@ int gbsdf_parse_obj(const char* text, size_t n_bytes, float* out_vertices, int64
     const long long n = (long long)n_bytes;
     const long long cap = n / 10 + 1024;  // the reference's line cap (cuda_mesh_io.cu:980)
     cudaError_t ce = cudaSuccess;
-    Scratch s;
+    IoScratch s(device);
     char* d_text = s.get<char>((size_t)n + 1, ce);
     unsigned* d_fv = s.get<unsigned>((size_t)n, ce);
     unsigned* d_ff = s.get<unsigned>((size_t)n, ce);
@@ -620,7 +653,7 @@ int gbsdf_parse_ascii_stl(const char* text, size_t n_bytes, float* out_vertices,
     if (rc != GBSDF_OK) return rc;
     const long long n = (long long)n_bytes;
     cudaError_t ce = cudaSuccess;
-    Scratch s;
+    IoScratch s(device);
     char* d_text = s.get<char>((size_t)n + 1, ce);
     unsigned* d_fl = s.get<unsigned>((size_t)n, ce);
     unsigned long long* d_pos = s.get<unsigned long long>((size_t)n + 1, ce);
