@@ -378,7 +378,7 @@ int gbsdf_find_default_seed(const float* grid, int32_t grid_on_device, const int
  * Needs no GPU. */
 int gbsdf_iso_surface_table(int8_t* out_table);
 
-/* Releases the cached device workspaces of `device` -- the SDF builder's and the
+/* Releases the cached device workspaces of `device` -- the SDF builder's, the mesh-file calls' and the
  * iso-surface extractor's (buffers are otherwise reused across calls on the same device). */
 void gbsdf_release_workspace(int32_t device);
 

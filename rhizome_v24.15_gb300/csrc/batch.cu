@@ -184,10 +184,10 @@ void place_phase1(Job& j, Carver& c) {
     j.bcur = c.take<unsigned>((size_t)L.nbricks * 4);
     j.active = c.take<unsigned>((size_t)L.nbricks * 4);
     j.boff = c.take<unsigned long long>((size_t)L.nbricks * 8);
-    j.scount = c.take<unsigned>((size_t)L.nstrips * 4);
-    j.scur = c.take<unsigned>((size_t)L.nstrips * 4);
-    j.soff = c.take<unsigned long long>((size_t)L.nstrips * 8);
-    j.scan = c.take<unsigned long long>((size_t)std::max(scan_tmp_elems(L.nbricks), scan_tmp_elems(L.nstrips)) * 8);
+    j.scount = c.take<unsigned>((size_t)L.nslists * 4);
+    j.scur = c.take<unsigned>((size_t)L.nslists * 4);
+    j.soff = c.take<unsigned long long>((size_t)L.nslists * 8);
+    j.scan = c.take<unsigned long long>((size_t)std::max(scan_tmp_elems(L.nbricks), scan_tmp_elems(L.nslists)) * 8);
     j.list_cap = std::max<long long>(kVerifySamples, std::min<long long>(kBatchListCap, N));
     j.list = c.take<long long>((size_t)j.list_cap * 8);
     j.recheck = c.take<long long>((size_t)j.list_cap * 8);
@@ -210,13 +210,13 @@ void enqueue_counts(gbsdf_batch& b, Job& j, cudaStream_t st) {
         cudaMemcpyAsync(j.t12, j.hin, (size_t)T * 48, cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(j.ds, 0, sizeof(DevState), st);
     cudaMemsetAsync(j.bcount, 0, (size_t)L.nbricks * 4, st);
-    cudaMemsetAsync(j.scount, 0, (size_t)L.nstrips * 4, st);
+    cudaMemsetAsync(j.scount, 0, (size_t)L.nslists * 4, st);
     launch_prep(j.t12, T, L, j.ptt, j.scount, j.ds, st);
     launch_pack_tri9(j.t12, T, j.t9, st);
     launch_fwn_build(j.t9, T, L, j.fwn, st);
     launch_brick_bins(j.fwn, T, L, j.bcount, nullptr, nullptr, j.ds, st);
     launch_exclusive_scan(j.bcount, j.boff, L.nbricks, j.scan, 0, st);
-    launch_exclusive_scan(j.scount, j.soff, L.nstrips, j.scan, 0, st);
+    launch_exclusive_scan(j.scount, j.soff, L.nslists, j.scan, 0, st);
     launch_active_bricks(j.bcount, L.nbricks, j.active, j.ds, st, j.dense_cut);
 }
 
@@ -259,7 +259,7 @@ void enqueue_build(gbsdf_batch& b, Job& j, cudaStream_t st) {
     const bool xs = exact_signs_mode(b);
     const float stol = xs ? kSurfaceTolExactSigns : kSurfaceTolVoxels;
     cudaMemsetAsync(j.bcur, 0, (size_t)L.nbricks * 4, st);
-    cudaMemsetAsync(j.scur, 0, (size_t)L.nstrips * 4, st);
+    cudaMemsetAsync(j.scur, 0, (size_t)L.nslists * 4, st);
     launch_strip_fill(j.ptt, T, L, j.soff, j.scur, j.slist, st, j.ds, j.cap_b, j.cap_s);
     launch_brick_bins(j.fwn, T, L, j.bcur, j.boff, j.blist, j.ds, st, j.cap_b, j.cap_s);
     // [init] + [A]

@@ -48,6 +48,7 @@ Lattice make_lattice(const int32_t mn[3], const int32_t mx[3], float h) {
     L.nbricks = (long long)L.nb[0] * L.nb[1] * L.nb[2];
     L.nsx = (L.dims[0] + kStrip - 1) / kStrip;
     L.nstrips = (long long)L.nsx * L.dims[1];
+    L.nslists = (long long)L.nsx * ((L.dims[1] + kSup - 1) / kSup) * kListSub;
     L.px = L.dims[0];
     return L;
 }
@@ -267,10 +268,10 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
     GB_CK(ensure(w.bcur, (size_t)L.nbricks * 4));
     GB_CK(ensure(w.boff, (size_t)L.nbricks * 8));
     GB_CK(ensure(w.active, (size_t)L.nbricks * 4));
-    GB_CK(ensure(w.scount, (size_t)L.nstrips * 4));
-    GB_CK(ensure(w.scur, (size_t)L.nstrips * 4));
-    GB_CK(ensure(w.soff, (size_t)L.nstrips * 8));
-    GB_CK(ensure(w.scan, (size_t)std::max(scan_tmp_elems(L.nbricks), scan_tmp_elems(L.nstrips)) * 8));
+    GB_CK(ensure(w.scount, (size_t)L.nslists * 4));
+    GB_CK(ensure(w.scur, (size_t)L.nslists * 4));
+    GB_CK(ensure(w.soff, (size_t)L.nslists * 8));
+    GB_CK(ensure(w.scan, (size_t)std::max(scan_tmp_elems(L.nbricks), scan_tmp_elems(L.nslists)) * 8));
     GB_CK(ensure(w.list, (size_t)kListCap * 8));
     GB_CK(ensure(w.recheck, (size_t)kListCap * 8));
 
@@ -282,7 +283,7 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
         GB_CK(cudaStreamSynchronize(st));
     }
     GB_CK(cudaMemsetAsync(w.bcount.p, 0, (size_t)L.nbricks * 4, st));
-    GB_CK(cudaMemsetAsync(w.scount.p, 0, (size_t)L.nstrips * 4, st));
+    GB_CK(cudaMemsetAsync(w.scount.p, 0, (size_t)L.nslists * 4, st));
     launch_prep(P<float>(w.t12), T, L, P<ParTri>(w.ptt), P<unsigned>(w.scount), w.ds, st);
     launch_pack_tri9(P<float>(w.t12), T, P<float>(w.t9), st);
     Fwn clusters{};
@@ -291,7 +292,7 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
     launch_brick_bins(clusters, T, L, P<unsigned>(w.bcount), nullptr, nullptr, w.ds, st);
     launch_exclusive_scan(P<unsigned>(w.bcount), P<unsigned long long>(w.boff), L.nbricks,
                           P<unsigned long long>(w.scan), 0, st);
-    launch_exclusive_scan(P<unsigned>(w.scount), P<unsigned long long>(w.soff), L.nstrips,
+    launch_exclusive_scan(P<unsigned>(w.scount), P<unsigned long long>(w.soff), L.nslists,
                           P<unsigned long long>(w.scan), 0, st);
     const unsigned dense_cut = o.splat_dense_cut > 0 ? (unsigned)o.splat_dense_cut : kDenseCutDefault;
     launch_active_bricks(P<unsigned>(w.bcount), L.nbricks, P<unsigned>(w.active), w.ds, st, dense_cut);
@@ -311,7 +312,7 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
     GB_CK(ensure(w.blist, (size_t)std::max<long long>(brick_pairs, 1) * 4));
     GB_CK(ensure(w.slist, (size_t)std::max<long long>(strip_pairs, 1) * 4));
     GB_CK(cudaMemsetAsync(w.bcur.p, 0, (size_t)L.nbricks * 4, st));
-    GB_CK(cudaMemsetAsync(w.scur.p, 0, (size_t)L.nstrips * 4, st));
+    GB_CK(cudaMemsetAsync(w.scur.p, 0, (size_t)L.nslists * 4, st));
     launch_brick_bins(clusters, T, L, P<unsigned>(w.bcur), P<unsigned long long>(w.boff), P<unsigned>(w.blist), w.ds,
                       st);
     launch_strip_fill(P<ParTri>(w.ptt), T, L, P<unsigned long long>(w.soff), P<unsigned>(w.scur), P<unsigned>(w.slist),

@@ -47,6 +47,13 @@ constexpr unsigned long long kFastMinVoxels = 32ull * 1024ull * 1024ull;
 // Brick edge of the band splat and lattice strip width of the parity pass.
 constexpr int kBrick = 8;
 constexpr int kStrip = 32;
+// Candidate lists of the parity pass: one per strip and supercell row (the rows of a supercell
+// share their candidates), kept in kListSub adjacent parts filled by lane, so that the many
+// triangles stacked over one strip do not queue at one counter.
+constexpr int kListSub = 8;
+__host__ __device__ __forceinline__ long long strip_list(int supy, int nsx, int sx) {
+    return ((long long)supy * nsx + sx) * kListSub;
+}
 
 struct f3 {
     float x, y, z;

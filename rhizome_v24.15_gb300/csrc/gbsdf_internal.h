@@ -21,6 +21,7 @@ struct Lattice {
     long long nbricks;
     int nsx;            // parity strips per row: ceil(dims[0] / kStrip)
     long long nstrips;  // nsx * dims[1]
+    long long nslists;  // strip candidate lists: nsx * ceil(dims[1] / kSup) * kListSub
     int px;             // row pitch (floats) of the distance grid the eikonal sweeps address:
                         // dims[0], or dims[0] rounded up to 8 in the sweeps' padded copies
 };
@@ -52,7 +53,7 @@ static_assert(sizeof(ParTri) == 80, "ParTri layout");
 // counters from `listed` to `recheck_n` are one pass's, and are cleared together.
 struct DevState {
     unsigned long long brick_pairs;    // (cluster, brick) pairs of the splat
-    unsigned long long strip_pairs;    // (triangle, strip) pairs of the parity pass
+    unsigned long long strip_pairs;    // entries of the parity pass's candidate lists
     unsigned long long csr_entries;    // entries of the reference's supercell CSR (guard)
     unsigned long long invalid_tris;   // non-finite or out-of-range coordinates
     unsigned long long active_bricks;
