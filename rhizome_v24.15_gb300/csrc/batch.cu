@@ -296,6 +296,7 @@ void enqueue_build(gbsdf_batch& b, Job& j, cudaStream_t st) {
         for (int axis = 0; axis < 3; ++axis)
             for (int dir = 1; dir >= -1; dir -= 2) {
                 launch_sweep(0, axis, dir, r, src, dst, Lp, j.ds, st, src == j.A ? &j.map_a : &j.map_b,
+                             dst == j.A ? &j.map_a : &j.map_b,
                              r == 0 ? j.xsched : j.xsched1, r == 0 ? j.wsched : j.wsched1);
                 std::swap(src, dst);
             }
@@ -375,8 +376,8 @@ int plan(gbsdf_batch& b, BErr& e) {
             const Lattice Lp = padded(j.L);
             encode_grid_map(j.map_a, j.A, Lp);
             encode_grid_map(j.map_b, j.B, Lp);
-            const SweepPlan plan = tuned_sweep_plan(b.device, Lp, j.A, j.B, &j.map_a, j.ds, b.origin, false, 0, 0);
-            const SweepPlan plan1 = tuned_sweep_plan(b.device, Lp, j.A, j.B, &j.map_a, j.ds, b.origin, false, 1, 0);
+            const SweepPlan plan = tuned_sweep_plan(b.device, Lp, j.A, j.B, &j.map_a, &j.map_b, j.ds, b.origin, false, 0, 0);
+            const SweepPlan plan1 = tuned_sweep_plan(b.device, Lp, j.A, j.B, &j.map_a, &j.map_b, j.ds, b.origin, false, 1, 0);
             j.xsched = plan.x;
             j.wsched = plan.w;
             if (b.dense_cut > 0) j.dense_cut = (unsigned)b.dense_cut;

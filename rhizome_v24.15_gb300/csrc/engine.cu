@@ -371,7 +371,7 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
     const bool tune = xs_opt == 0 || ws_opt == 0;
     SweepPlan plan;
     auto set_plan = [&](int phase, const GridMap* m, bool measure) -> int {
-        plan = tuned_sweep_plan(w.device, Lp, src, dst, m, w.ds, st, measure, phase, rule);
+        plan = tuned_sweep_plan(w.device, Lp, src, dst, m, map_of(dst), w.ds, st, measure, phase, rule);
         if (xs_opt >= kXCpAsync && xs_opt <= kXTmaNarrow) plan.x = xs_opt;
         if (ws_opt >= kWCpAsync && ws_opt <= kWTmaNarrow) plan.w = ws_opt;
         GB_CK(cudaGetLastError());
@@ -392,8 +392,8 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
                 if (int rcp = set_plan(1, map_of(src), tune)) return rcp;
             for (int axis = 0; axis < 3; ++axis)
                 for (int dir = 1; dir >= -1; dir -= 2) {
-                    launch_sweep(rule, axis, dir, r, src, dst, Lp, w.ds, st, lead ? lead : map_of(src), plan.x,
-                                 plan.w);
+                    launch_sweep(rule, axis, dir, r, src, dst, Lp, w.ds, st, lead ? lead : map_of(src), map_of(dst),
+                                 plan.x, plan.w);
                     lead = nullptr;
                     std::swap(src, dst);
                 }
@@ -410,7 +410,7 @@ int run_fast(Workspace& w, long long T, const Lattice& L, const gbsdf_options& o
                 for (int axis = 0; axis < 3; ++axis)
                     for (int dir = 1; dir >= -1; dir -= 2) {
                         launch_sweep(rule, axis, dir, r % 64, src, dst, Lp, w.ds, st, lead ? lead : map_of(src),
-                                     plan.x, plan.w);
+                                     map_of(dst), plan.x, plan.w);
                         lead = nullptr;
                         std::swap(src, dst);
                     }

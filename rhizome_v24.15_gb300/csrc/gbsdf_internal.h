@@ -276,6 +276,7 @@ struct GridMap {
     CUtensorMap ymap;  // y walk batch: 40 (x) x 4 (y slices) x 18 (z rows)
     CUtensorMap zmap;  // z walk batch: 40 (x) x 18 (y rows) x 4 (z slices)
     CUtensorMap wmap;  // wide x sweep tile: 20 (x) x 34 (y) x 10 (z), no swizzle
+    CUtensorMap smap;  // results of an x sweep's chunk: 8 (x) x 32 (y) x 1 (z), 32-byte swizzle
     CUtensorMap nmap;  // narrow x sweep tile: 8 (x) x 34 (y) x 6 (z), 32-byte swizzle
     CUtensorMap ynmap; // narrow y walk batch: 40 (x) x 4 (y slices) x 6 (z rows)
     CUtensorMap znmap; // narrow z walk batch: 40 (x) x 6 (y rows) x 4 (z slices)
@@ -308,9 +309,10 @@ enum XSchedule : int {
 enum WSchedule : int {
     kWAuto = 0, kWCpAsync = 1, kWTmaPipe = 2, kWTmaVec = 3, kWTmaVec2 = 4, kWTmaNarrow = 5
 };
-// `src_map`: the descriptor of `src` (or null); `x_schedule`: an XSchedule.
+// `src_map`, `dst_map`: the descriptors of `src` and `dst` (or null); `x_schedule`: an XSchedule.
 void launch_sweep(int rule, int axis, int dir, int round, const float* src, float* dst, const Lattice& L,
-                  DevState* ds, cudaStream_t st, const GridMap* src_map = nullptr, int x_schedule = kXAuto,
+                  DevState* ds, cudaStream_t st, const GridMap* src_map = nullptr,
+                  const GridMap* dst_map = nullptr, int x_schedule = kXAuto,
                   int w_schedule = kWAuto);
 // The sweep schedules for this lattice class and phase (0: the first round, 1: later
 // rounds): the remembered winners, else (measure) each candidate timed on src -> dst
@@ -320,6 +322,7 @@ struct SweepPlan {
     int w;  // WSchedule
 };
 SweepPlan tuned_sweep_plan(int device, const Lattice& L, const float* src, float* dst, const GridMap* src_map,
+                           const GridMap* dst_map,
                            DevState* ds, cudaStream_t st, bool measure, int phase, int rule);
 // Layout check of the x sweep's TMA tile (swizzled rows, out-of-lattice fill): writes the
 // number of mismatching elements to *mism.

@@ -381,6 +381,16 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
         : "memory");
 }
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int x, int y, int z, const void* src) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];\n"
+                 "cp.async.bulk.commit_group;\n" ::"l"(reinterpret_cast<uint64_t>(map)),
+                 "r"(x), "r"(y), "r"(z), "r"(smem_u32(src))
+                 : "memory");
+}
+// at most one of this thread's stores still reads its shared memory / none is in flight
+__device__ __forceinline__ void tma_store_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory"); }
+__device__ __forceinline__ void tma_store_wait_read2() { asm volatile("cp.async.bulk.wait_group.read 2;\n" ::: "memory"); }
+__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
 // float offset of element j (0..7) of staged line r in a 32-byte-swizzled tile
 __device__ __forceinline__ int tsw(int r, int j) { return r * 8 + ((((j >> 2) ^ (r >> 2)) & 1) << 2) + (j & 3); }
 // 16-byte half c (0, 1) of staged line r
@@ -529,9 +539,11 @@ __global__ void __launch_bounds__(kXThreads) sweep_x_tma_kernel(const __grid_con
 // lets its copies in flight land before it leaves.
 constexpr int kPS = 4;                               // ring slots
 constexpr int kPThreads = kXThreads + 32;            // 8 consumer warps + 1 producer warp
-constexpr size_t kPSmem = (size_t)kPS * kTSlotBytes + 128 + 1024;
 // The pipeline on tiles of ZT lines along z: 8, or 4 with a deeper ring where tiles of 8 would
-// leave SMs without a CTA (224^3: 41.4 -> 38.8 us per sweep over all six directions).
+// leave SMs without a CTA (224^3: 41.4 -> 38.8 us per sweep over all six directions). A warp's
+// results of a chunk, 32 bytes of 32 rows, go out as one TMA store from shared memory: as two
+// 16-byte stores a lane they took half of the L1's time (860 x 860 x 880: 1,194 -> 1,167 us per
+// sweep over all six directions; 512^3: 287 -> 283).
 constexpr int kXZNarrow = 4;
 template <int ZT>
 struct XPipe {
@@ -539,7 +551,8 @@ struct XPipe {
     static constexpr int kBox = kXC * kXHY * (ZT + 2);
     static constexpr int kSlotBytes = (kBox * 4 + 1023) / 1024 * 1024;
     static constexpr int kSlots = ZT == kXZ ? kPS : 6;
-    static constexpr size_t kSmem = (size_t)kSlots * kSlotBytes + 128 + 1024;
+    static constexpr int kStageBytes = 2 * ZT * kXY * kXC * 4;  // two chunks of results a warp
+    static constexpr size_t kSmem = (size_t)kSlots * kSlotBytes + kStageBytes + 128 + 1024;
 };
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -550,21 +563,20 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // (1: godunov_ref_nb; 2: godunov_ref_nbp, its 2D and 3D arithmetic paired on packed FP32
 // lanes, 57-59 instructions per voxel against 66), identical results.
 template <int RULE, int DIR, int NB = 0, int ZT = kXZ>
-__global__ void __launch_bounds__(XPipe<ZT>::kThreads) sweep_x_pipe_kernel(const __grid_constant__ CUtensorMap tm,
-                                                                  float* __restrict__ dst, Lattice L, int round,
-                                                                  DevState* ds) {
+__global__ void __launch_bounds__(XPipe<ZT>::kThreads, ZT == kXZ ? 3 : 1) sweep_x_pipe_kernel(const __grid_constant__ CUtensorMap tm,
+                                                                                const __grid_constant__ CUtensorMap tmo,
+                                                                                Lattice L, int round, DevState* ds) {
     if (ds->stop) return;
     constexpr int kSlots = XPipe<ZT>::kSlots, kSlotBytes = XPipe<ZT>::kSlotBytes, kConsumers = XPipe<ZT>::kConsumers;
     const int polls = wait_poll_limit(ds);
     extern __shared__ unsigned char tsm_raw[];
     unsigned char* tsm = align1k(tsm_raw);
-    uint64_t* full = reinterpret_cast<uint64_t*>(tsm + kSlots * kSlotBytes);
+    uint64_t* full = reinterpret_cast<uint64_t*>(tsm + kSlots * kSlotBytes + XPipe<ZT>::kStageBytes);
     uint64_t* empty = full + kSlots;
     const int dx = L.dims[0], dy = L.dims[1], dz = L.dims[2];
     const float h = L.h;
     const float m2h = -2.0f * h, na3 = -(3.0f * h * h);
     const GodunovOneConsts gc = godunov_one_consts(h);
-    const size_t plane = (size_t)L.px * dy;
     const int tid = threadIdx.x;
     const int y0 = blockIdx.x * kXY, z0 = blockIdx.y * ZT;
     const int nchunks = (dx + kXC - 1) / kXC;
@@ -599,6 +611,7 @@ __global__ void __launch_bounds__(XPipe<ZT>::kThreads) sweep_x_pipe_kernel(const
     const bool active = (y < dy) && (z < dz);
     const int rme = (tz + 1) * kXHY + (ty + 1);
     const int rym = rme - 1, ryp = rme + 1, rzm = rme - kXHY, rzp = rme + kXHY;
+    float* stage = reinterpret_cast<float*>(tsm + kSlots * kSlotBytes) + 2 * tz * (kXY * kXC);
     float prev = kFarSentinel;
     bool ch = false;
 #pragma unroll 1
@@ -607,7 +620,10 @@ __global__ void __launch_bounds__(XPipe<ZT>::kThreads) sweep_x_pipe_kernel(const
         bool ok = ci > 0 || mbar_wait(&full[0], 0, polls);
         if (ok && ci + 1 < nchunks) ok = mbar_wait(&full[(ci + 1) % kSlots], ((ci + 1) / kSlots) & 1, polls);
         if (!__all_sync(0xffffffffu, ok)) {
-            if (ty == 0) atomicAdd(&ds->wait_timeouts, 1ull);
+            if (ty == 0) {
+                tma_store_wait_all();
+                atomicAdd(&ds->wait_timeouts, 1ull);
+            }
             return;
         }
         const int c = (DIR > 0) ? ci : (nchunks - 1 - ci);
@@ -671,20 +687,24 @@ __global__ void __launch_bounds__(XPipe<ZT>::kThreads) sweep_x_pipe_kernel(const
                     prev = out;
                 }
             }
-            float* drow = dst + (size_t)z * plane + (size_t)y * L.px + xc;
-            if (xc + kXC <= dx) {
-                reinterpret_cast<float4*>(drow)[0] = make_float4(res[0], res[1], res[2], res[3]);
-                reinterpret_cast<float4*>(drow)[1] = make_float4(res[4], res[5], res[6], res[7]);
-            } else {
-#pragma unroll
-                for (int j = 0; j < kXC; ++j)
-                    if (xc + j < dx) drow[j] = res[j];
-            }
+            // (the pair of buffers' second-last store has been read)
+            float4* out = reinterpret_cast<float4*>(stage + (ci & 1) * (kXY * kXC));
+            out[2 * ty + ((ty >> 2) & 1)] = make_float4(res[0], res[1], res[2], res[3]);
+            out[2 * ty + (((ty >> 2) & 1) ^ 1)] = make_float4(res[4], res[5], res[6], res[7]);
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         }
         // this warp's last read of chunk ci's slot is done (it was also chunk ci-1's "next")
         __syncwarp();
-        if (ty == 0) mbar_arrive(&empty[ci % kSlots]);
+        if (ty == 0) {
+            mbar_arrive(&empty[ci % kSlots]);
+            if (z < dz) {  // rows past dy and voxels past dx are clipped
+                tma_store_3d(&tmo, xc, y0, z, stage + (ci & 1) * (kXY * kXC));
+                tma_store_wait_read1();
+            }
+        }
+        __syncwarp();  // the next chunk's buffer is free
     }
+    if (ty == 0) tma_store_wait_all();
     mark_changed(ch, &ds->changed[round]);
 }
 
@@ -698,24 +718,26 @@ __global__ void __launch_bounds__(XPipe<ZT>::kThreads) sweep_x_pipe_kernel(const
 // partner); the launcher falls back to sweep_x_pipe_kernel elsewhere.
 constexpr int kP2Consumers = kXThreads / 2;              // 4 consumer warps
 constexpr int kP2Threads = kP2Consumers + 32;
+constexpr int kP2S = 3;                                  // ring slots: three CTAs and their results fit an SM
+constexpr int kP2StageBytes = 2 * kXZ * kXY * kXC * 4;   // two chunks of results a line group
+constexpr size_t kP2Smem = (size_t)kP2S * kTSlotBytes + kP2StageBytes + 128 + 1024;
 
 template <int DIR>
 __global__ void __launch_bounds__(kP2Threads, 4) sweep_x_pipe2_kernel(const __grid_constant__ CUtensorMap tm,
-                                                                   float* __restrict__ dst, Lattice L, int round,
-                                                                   DevState* ds) {
+                                                                      const __grid_constant__ CUtensorMap tmo,
+                                                                      Lattice L, int round, DevState* ds) {
     if (ds->stop) return;
     const int polls = wait_poll_limit(ds);
     extern __shared__ unsigned char tsm_raw[];
     unsigned char* tsm = align1k(tsm_raw);
-    uint64_t* full = reinterpret_cast<uint64_t*>(tsm + kPS * kTSlotBytes);
-    uint64_t* empty = full + kPS;
+    uint64_t* full = reinterpret_cast<uint64_t*>(tsm + kP2S * kTSlotBytes + kP2StageBytes);
+    uint64_t* empty = full + kP2S;
     const int dx = L.dims[0], dy = L.dims[1], dz = L.dims[2];
-    const size_t plane = (size_t)L.px * dy;
     const int tid = threadIdx.x;
     const int y0 = blockIdx.x * kXY, z0 = blockIdx.y * kXZ;
     const int nchunks = (dx + kXC - 1) / kXC;
     if (tid == 0) {
-        for (int s = 0; s < kPS; ++s) {
+        for (int s = 0; s < kP2S; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], kP2Consumers / 32);
         }
@@ -726,8 +748,8 @@ __global__ void __launch_bounds__(kP2Threads, 4) sweep_x_pipe2_kernel(const __gr
         if (tid != kP2Consumers) return;
         int ci = 0;
         for (; ci < nchunks; ++ci) {
-            const int s = ci % kPS;
-            if (ci >= kPS && !mbar_wait(&empty[s], ((ci / kPS) - 1) & 1, polls)) break;
+            const int s = ci % kP2S;
+            if (ci >= kP2S && !mbar_wait(&empty[s], ((ci / kP2S) - 1) & 1, polls)) break;
             const int c = (DIR > 0) ? ci : (nchunks - 1 - ci);
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
             mbar_expect_tx(&full[s], kTBox * 4);
@@ -735,7 +757,7 @@ __global__ void __launch_bounds__(kP2Threads, 4) sweep_x_pipe2_kernel(const __gr
         }
         // let every copy still in flight land before the producer leaves (consumers that gave
         // up have left already); a break means the consumers stopped releasing slots
-        for (int k = max(0, ci - kPS); k < ci; ++k) mbar_wait(&full[k % kPS], (k / kPS) & 1);
+        for (int k = max(0, ci - kP2S); k < ci; ++k) mbar_wait(&full[k % kP2S], (k / kP2S) & 1);
         if (ci < nchunks) atomicAdd(&ds->wait_timeouts, 1ull);
         return;
     }
@@ -747,25 +769,29 @@ __global__ void __launch_bounds__(kP2Threads, 4) sweep_x_pipe2_kernel(const __gr
     const GodunovPairConsts gc = godunov_pair_consts(L.h);
     const float h = L.h;
     float preva = kFarSentinel, prevb = kFarSentinel;
-    bool ch = false;
+    float* stage = reinterpret_cast<float*>(tsm + kP2S * kTSlotBytes) + tz * (4 * kXY * kXC);
+    bool ch = false, chb = false;  // (line b's updates outside the lattice do not count)
 #pragma unroll 1
     for (int ci = 0; ci < nchunks; ++ci) {
-        bool ok = mbar_wait(&full[ci % kPS], (ci / kPS) & 1, polls);
-        if (ok && ci + 1 < nchunks) ok = mbar_wait(&full[(ci + 1) % kPS], ((ci + 1) / kPS) & 1, polls);
+        // (chunk ci's own barrier was waited for a chunk ago)
+        bool ok = ci > 0 || mbar_wait(&full[0], 0, polls);
+        if (ok && ci + 1 < nchunks) ok = mbar_wait(&full[(ci + 1) % kP2S], ((ci + 1) / kP2S) & 1, polls);
         if (!__all_sync(0xffffffffu, ok)) {
-            if (ty == 0) atomicAdd(&ds->wait_timeouts, 1ull);
+            if (ty == 0) {
+                tma_store_wait_all();
+                atomicAdd(&ds->wait_timeouts, 1ull);
+            }
             return;
         }
         const int c = (DIR > 0) ? ci : (nchunks - 1 - ci);
         const int xc = c * kXC;
-        const float* tile = reinterpret_cast<const float*>(tsm + (ci % kPS) * kTSlotBytes);
-        const float* ntile = reinterpret_cast<const float*>(tsm + ((ci + 1) % kPS) * kTSlotBytes);
+        const float* tile = reinterpret_cast<const float*>(tsm + (ci % kP2S) * kTSlotBytes);
+        const float* ntile = reinterpret_cast<const float*>(tsm + ((ci + 1) % kP2S) * kTSlotBytes);
+        float4* out = reinterpret_cast<float4*>(stage + (ci & 1) * (2 * kXY * kXC));
         if (act_a && xc + kXC <= dx && ci + 1 < nchunks) {
             // both lines' chunks are whole (line b may be outside the lattice: it then
             // reads the NaN fill and its results are not stored). The chunk is walked in
             // two 4-voxel halves, so only one half's operands are live at a time.
-            float* da = dst + (size_t)za * plane + (size_t)y * L.px + xc;
-            float* db = dst + (size_t)zb * plane + (size_t)y * L.px + xc;
             const float nxta = (DIR > 0) ? ntile[tsw(rma, 0)] : ntile[tsw(rma, kXC - 1)];
             const float nxtb = (DIR > 0) ? ntile[tsw(rmb, 0)] : ntile[tsw(rmb, kXC - 1)];
             float4 ma = tvec(tile, rma, (DIR > 0) ? 0 : 1), mb = tvec(tile, rmb, (DIR > 0) ? 0 : 1);
@@ -801,15 +827,16 @@ __global__ void __launch_bounds__(kP2Threads, 4) sweep_x_pipe2_kernel(const __gr
                     float ua, ub;
                     godunov_ref_pair(fminf(preva, downa), aya[j], aza[j], fminf(prevb, downb), ayb[j], azb[j], gc, ua,
                                      ub);
-                    const bool la = ua < cura[j], lb = act_b && (ub < curb[j]);
-                    resa[j] = la ? ua : cura[j];
-                    resb[j] = lb ? ub : curb[j];
-                    ch |= la | lb;
+                    ch |= ua < cura[j];
+                    chb |= ub < curb[j];
+                    resa[j] = fminf(ua, cura[j]);
+                    resb[j] = fminf(ub, curb[j]);
                     preva = resa[j];
                     prevb = resb[j];
                 }
-                reinterpret_cast<float4*>(da)[hv] = make_float4(resa[0], resa[1], resa[2], resa[3]);
-                if (act_b) reinterpret_cast<float4*>(db)[hv] = make_float4(resb[0], resb[1], resb[2], resb[3]);
+                const int at = 2 * ty + (((ty >> 2) ^ hv) & 1);
+                out[at] = make_float4(resa[0], resa[1], resa[2], resa[3]);
+                out[at + 2 * kXY] = make_float4(resb[0], resb[1], resb[2], resb[3]);
             }
         } else {
             // a partial or the last chunk: each line on its own with the scalar update
@@ -818,7 +845,6 @@ __global__ void __launch_bounds__(kP2Threads, 4) sweep_x_pipe2_kernel(const __gr
                 const bool act = side ? act_b : act_a;
                 if (!act) continue;
                 const int rme = side ? rmb : rma;
-                const int z = side ? zb : za;
                 float prev = side ? prevb : preva;
                 float res[kXC];
 #pragma unroll
@@ -840,24 +866,25 @@ __global__ void __launch_bounds__(kP2Threads, 4) sweep_x_pipe2_kernel(const __gr
                     res[j] = out;
                     prev = out;
                 }
-                float* drow = dst + (size_t)z * plane + (size_t)y * L.px + xc;
-                if (xc + kXC <= dx) {
-                    reinterpret_cast<float4*>(drow)[0] = make_float4(res[0], res[1], res[2], res[3]);
-                    reinterpret_cast<float4*>(drow)[1] = make_float4(res[4], res[5], res[6], res[7]);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < kXC; ++j)
-                        if (xc + j < dx) drow[j] = res[j];
-                }
+                out[2 * ty + ((ty >> 2) & 1) + 2 * kXY * side] = make_float4(res[0], res[1], res[2], res[3]);
+                out[2 * ty + (((ty >> 2) & 1) ^ 1) + 2 * kXY * side] = make_float4(res[4], res[5], res[6], res[7]);
                 if (side) prevb = prev;
                 else preva = prev;
             }
         }
         // this warp's last read of chunk ci's slot is done (it was also chunk ci-1's "next")
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         __syncwarp();
-        if (ty == 0) mbar_arrive(&empty[ci % kPS]);
+        if (ty == 0) {
+            mbar_arrive(&empty[ci % kP2S]);
+            if (za < dz) tma_store_3d(&tmo, xc, y0, za, out);
+            if (zb < dz) tma_store_3d(&tmo, xc, y0, zb, out + 2 * kXY);
+            tma_store_wait_read2();
+        }
+        __syncwarp();  // the next chunk's buffers are free
     }
-    mark_changed(ch, &ds->changed[round]);
+    if (ty == 0) tma_store_wait_all();
+    mark_changed(ch || (chb && act_b), &ds->changed[round]);
 }
 
 // ---- x sweeps, wide TMA tiles ----------------------------------------------------------
@@ -1652,9 +1679,11 @@ __global__ void __launch_bounds__(256) apply_kernel(const float* __restrict__ g,
 
 template <int RULE, int DIR>
 void launch_sweep_t(int axis, int round, const float* src, float* dst, const Lattice& L, DevState* ds,
-                    cudaStream_t st, const GridMap* src_map, int xsched, int wsched) {
+                    cudaStream_t st, const GridMap* src_map, const GridMap* dst_map, int xsched, int wsched) {
     const bool tma = src_map && src_map->valid;
     if (xsched == 0) xsched = tma ? kXTmaPipe : kXCpAsync;
+    // the pipelines write through the destination's descriptor
+    if ((xsched == kXTmaPipe || xsched == kXTmaNarrow) && !(dst_map && dst_map->valid)) xsched = kXTmaRing;
     if (!tma) xsched = kXCpAsync;
     const bool wtma = src_map && src_map->walk_valid;
     if (wsched == 0) wsched = wtma ? kWTmaPipe : kWCpAsync;
@@ -1731,10 +1760,10 @@ void launch_sweep_t(int axis, int round, const float* src, float* dst, const Lat
         cudaFuncSetAttribute(sweep_walk_kernel<1, RULE, DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kWSmem);
         sweep_walk_kernel<1, RULE, DIR><<<grid, kWThreads, kWSmem, st>>>(src, dst, L, round, ds);
-    } else if (xsched == kXTmaPipe2 && pair_ok && dy >= 2 && dz >= 2) {
+    } else if (xsched == kXTmaPipe2 && pair_ok && dy >= 2 && dz >= 2 && dst_map && dst_map->valid) {
         dim3 grid((dy + kXY - 1) / kXY, (dz + kXZ - 1) / kXZ);
-        cudaFuncSetAttribute(sweep_x_pipe2_kernel<DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPSmem);
-        sweep_x_pipe2_kernel<DIR><<<grid, kP2Threads, kPSmem, st>>>(src_map->map, dst, L, round, ds);
+        cudaFuncSetAttribute(sweep_x_pipe2_kernel<DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kP2Smem);
+        sweep_x_pipe2_kernel<DIR><<<grid, kP2Threads, kP2Smem, st>>>(src_map->map, dst_map->smap, L, round, ds);
     } else if (xsched == kXTmaWide && src_map->wide_valid) {
         dim3 grid((dy + kXY - 1) / kXY, (dz + kXZ - 1) / kXZ);
         if (pair_ok) {
@@ -1751,22 +1780,19 @@ void launch_sweep_t(int axis, int round, const float* src, float* dst, const Lat
         dim3 grid((dy + kXY - 1) / kXY, (dz + kXZNarrow - 1) / kXZNarrow);
         auto go = [&](auto kernel) {
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XPipe<kXZNarrow>::kSmem);
-            kernel<<<grid, XPipe<kXZNarrow>::kThreads, XPipe<kXZNarrow>::kSmem, st>>>(src_map->nmap, dst, L, round, ds);
+            kernel<<<grid, XPipe<kXZNarrow>::kThreads, XPipe<kXZNarrow>::kSmem, st>>>(src_map->nmap, dst_map->smap, L, round, ds);
         };
         if (pair_ok) go(sweep_x_pipe_kernel<0, DIR, 2, kXZNarrow>);
         else go(sweep_x_pipe_kernel<RULE, DIR, 0, kXZNarrow>);
-    } else if (xsched == kXTmaPipe || xsched == kXTmaPipe2 || xsched == kXTmaWide) {
+    } else if (dst_map && dst_map->valid && (xsched == kXTmaPipe || xsched == kXTmaPipe2 || xsched == kXTmaWide)) {
         dim3 grid((dy + kXY - 1) / kXY, (dz + kXZ - 1) / kXZ);
-        if (pair_ok) {
-            cudaFuncSetAttribute(sweep_x_pipe_kernel<0, DIR, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kPSmem);
-            sweep_x_pipe_kernel<0, DIR, 2><<<grid, kPThreads, kPSmem, st>>>(src_map->map, dst, L, round, ds);
-        } else {
-            cudaFuncSetAttribute(sweep_x_pipe_kernel<RULE, DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kPSmem);
-            sweep_x_pipe_kernel<RULE, DIR><<<grid, kPThreads, kPSmem, st>>>(src_map->map, dst, L, round, ds);
-        }
-    } else if (xsched == kXTmaRing) {
+        auto go = [&](auto kernel) {
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XPipe<kXZ>::kSmem);
+            kernel<<<grid, XPipe<kXZ>::kThreads, XPipe<kXZ>::kSmem, st>>>(src_map->map, dst_map->smap, L, round, ds);
+        };
+        if (pair_ok) go(sweep_x_pipe_kernel<0, DIR, 2>);
+        else go(sweep_x_pipe_kernel<RULE, DIR>);
+    } else if (xsched == kXTmaRing || xsched == kXTmaPipe || xsched == kXTmaPipe2 || xsched == kXTmaWide) {
         dim3 grid((dy + kXY - 1) / kXY, (dz + kXZ - 1) / kXZ);
         cudaFuncSetAttribute(sweep_x_tma_kernel<RULE, DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kTSmem);
@@ -1799,7 +1825,8 @@ EncodeTiledFn tiled_encoder() {
 
 // A 3D tiled descriptor of a grid of dx x dy x dz voxels whose rows are px floats apart.
 bool encode_box(CUtensorMap* m, const float* base, int dx, int dy, int dz, int px, int bx = kXC, int by = kXHY,
-                int bz = kXHZ, CUtensorMapSwizzle sw = CU_TENSOR_MAP_SWIZZLE_32B) {
+                int bz = kXHZ, CUtensorMapSwizzle sw = CU_TENSOR_MAP_SWIZZLE_32B,
+                CUtensorMapFloatOOBfill fill = CU_TENSOR_MAP_FLOAT_OOB_FILL_NAN_REQUEST_ZERO_FMA) {
     EncodeTiledFn fn = tiled_encoder();
     if (!fn) return false;
     const cuuint64_t gdim[3] = {(cuuint64_t)dx, (cuuint64_t)dy, (cuuint64_t)dz};
@@ -1807,8 +1834,7 @@ bool encode_box(CUtensorMap* m, const float* base, int dx, int dy, int dz, int p
     const cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz};
     const cuuint32_t estr[3] = {1, 1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), gdim, gstride, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NAN_REQUEST_ZERO_FMA) == CUDA_SUCCESS;
+              CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, fill) == CUDA_SUCCESS;
 }
 
 }  // namespace
@@ -1827,7 +1853,9 @@ bool encode_grid_map(GridMap& m, const float* base, const Lattice& L) {
     const bool narrow = encode_box(&m.nmap, base, dx, dy, dz, L.px, kXC, kXHY, kXZNarrow + 2) &&
                         encode_box(&m.ynmap, base, dx, dy, dz, L.px, kWPX, kWPB, kWNR + 2, CU_TENSOR_MAP_SWIZZLE_NONE) &&
                         encode_box(&m.znmap, base, dx, dy, dz, L.px, kWPX, kWNR + 2, kWPB, CU_TENSOR_MAP_SWIZZLE_NONE);
-    m.valid = m.valid && narrow;
+    m.valid = m.valid && narrow &&
+              encode_box(&m.smap, base, dx, dy, dz, L.px, kXC, kXY, 1, CU_TENSOR_MAP_SWIZZLE_32B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     m.walk_valid = m.walk_valid && narrow;
     m.wide_valid = m.valid && encode_box(&m.wmap, base, dx, dy, dz, L.px, kXWB, kXHY, kXHZ,
                                          CU_TENSOR_MAP_SWIZZLE_NONE);
@@ -1835,13 +1863,13 @@ bool encode_grid_map(GridMap& m, const float* base, const Lattice& L) {
 }
 
 void launch_sweep(int rule, int axis, int dir, int round, const float* src, float* dst, const Lattice& L,
-                  DevState* ds, cudaStream_t st, const GridMap* src_map, int x_schedule, int w_schedule) {
+                  DevState* ds, cudaStream_t st, const GridMap* src_map, const GridMap* dst_map, int x_schedule, int w_schedule) {
     if (rule == 0) {
-        if (dir > 0) launch_sweep_t<0, 1>(axis, round, src, dst, L, ds, st, src_map, x_schedule, w_schedule);
-        else launch_sweep_t<0, -1>(axis, round, src, dst, L, ds, st, src_map, x_schedule, w_schedule);
+        if (dir > 0) launch_sweep_t<0, 1>(axis, round, src, dst, L, ds, st, src_map, dst_map, x_schedule, w_schedule);
+        else launch_sweep_t<0, -1>(axis, round, src, dst, L, ds, st, src_map, dst_map, x_schedule, w_schedule);
     } else {
-        if (dir > 0) launch_sweep_t<1, 1>(axis, round, src, dst, L, ds, st, src_map, x_schedule, w_schedule);
-        else launch_sweep_t<1, -1>(axis, round, src, dst, L, ds, st, src_map, x_schedule, w_schedule);
+        if (dir > 0) launch_sweep_t<1, 1>(axis, round, src, dst, L, ds, st, src_map, dst_map, x_schedule, w_schedule);
+        else launch_sweep_t<1, -1>(axis, round, src, dst, L, ds, st, src_map, dst_map, x_schedule, w_schedule);
     }
 }
 

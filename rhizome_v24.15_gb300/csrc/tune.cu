@@ -58,6 +58,7 @@ SweepPlan default_plan(const Lattice& L, int rule, bool tma, bool wtma) {
 }  // namespace
 
 SweepPlan tuned_sweep_plan(int device, const Lattice& L, const float* src, float* dst, const GridMap* src_map,
+                           const GridMap* dst_map,
                            DevState* ds, cudaStream_t st, bool measure, int phase, int rule) {
     const bool tma = src_map && src_map->valid, wtma = src_map && src_map->walk_valid;
     SweepPlan plan = default_plan(L, rule, tma, wtma);
@@ -82,9 +83,9 @@ SweepPlan tuned_sweep_plan(int device, const Lattice& L, const float* src, float
     const int slot = 63;  // a change-flag slot the reference round loop never uses
     // one warm-up and two timed launches of one directional sweep; < 0 on failure
     auto time_it = [&](int axis, int xs, int ws) -> float {
-        launch_sweep(0, axis, 1, slot, src, dst, L, ds, st, src_map, xs, ws);
+        launch_sweep(0, axis, 1, slot, src, dst, L, ds, st, src_map, dst_map, xs, ws);
         cudaEventRecord(a, st);
-        for (int r = 0; r < 2; ++r) launch_sweep(0, axis, 1, slot, src, dst, L, ds, st, src_map, xs, ws);
+        for (int r = 0; r < 2; ++r) launch_sweep(0, axis, 1, slot, src, dst, L, ds, st, src_map, dst_map, xs, ws);
         cudaEventRecord(b, st);
         float ms = -1.0f;
         if (cudaEventSynchronize(b) != cudaSuccess || cudaEventElapsedTime(&ms, a, b) != cudaSuccess) {
