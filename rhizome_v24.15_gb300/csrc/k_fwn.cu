@@ -1003,9 +1003,10 @@ __device__ __forceinline__ float cta_min(float x, float* red) {
 
 // A warp's walk down to one cluster near p: of the n clusters item(i) the one of the least
 // box distance, then its nearest child, to the lowest level; returns the least distance to that
-// cluster's triangles (an upper bound of p's distance to the mesh; the same in all lanes).
+// cluster's triangles (an upper bound of p's distance to the mesh; the same in all lanes) and the
+// cluster.
 template <class F>
-__device__ __forceinline__ float walk_near(const FwnView& f, int level, int n, const f3& p, F item) {
+__device__ __forceinline__ float walk_near(const FwnView& f, int level, int n, const f3& p, F item, int& k) {
     const int lane = threadIdx.x & 31;
     float best = __int_as_float(0x7f800000);
     int bk = -1;
@@ -1017,7 +1018,7 @@ __device__ __forceinline__ float walk_near(const FwnView& f, int level, int n, c
             bk = k;
         }
     }
-    int k = warp_argmin(bk < 0 ? __int_as_float(0x7f800000) : best, bk < 0 ? 0x7fffffff : bk);
+    k = warp_argmin(bk < 0 ? __int_as_float(0x7f800000) : best, bk < 0 ? 0x7fffffff : bk);
     for (int l = level - 1; l >= 0; --l) {
         const int c = k * kFwnFan + (lane & 15);
         const bool on = c < f.n[l];
@@ -1035,16 +1036,20 @@ __device__ __forceinline__ float walk_near(const FwnView& f, int level, int n, c
 // triangle, no voxel within rho of the centre is farther than u + rho from the mesh, and a
 // cluster whose box is farther than u + 2 rho from the centre holds no voxel's nearest triangle.
 // The brick keeps the clusters of each level that pass, each of its octants those that pass for
-// it, and a voxel skips a cluster whose box, or a triangle whose bounding sphere or plane,
-// lies beyond its best so far. The tests are widened by the rounding of both sides, so the
+// it, nearest ones first, and a voxel skips a cluster whose box, or a triangle whose bounding
+// sphere or plane, lies beyond its best so far. The lanes first test (cluster, 2^3 cube) and
+// (triangle, 2^3 cube) pairs, 32 at a time, against the cubes' worst bests: of what an octant
+// keeps, most is near none of its voxels. The tests are widened by the rounding of both sides, so the
 // minimum is that over all triangles. (Boxes, not spheres: a run of a mug wall's long
 // triangles is flat, and a voxel within its sphere's radius of the wall would keep it.)
-// Bound by the FP32 work of the exact distances (57% of the issue slots, 24 lanes of 32).
+// Bound by the FP32 work of the tests and exact distances (57% of the issue slots, 24 lanes of
+// 32; 80 registers, three CTAs an SM: with the 97 the compiler takes, two, 3.5 ms below).
 // Replaces a walk of 128-triangle tiles in input order for each voxel: 181 x 135 x 156 mug,
-// 24,000 triangles, 56.5 -> 3.4 ms; 48 x 48 x 52, 2,712 triangles, 0.72 -> 0.47 ms.
+// 24,000 triangles, 56.5 -> 3.0 ms (3.4 without the pairs and the order); 48 x 48 x 52, 2,712
+// triangles, 0.72 -> 0.32 (0.46).
 // One CTA a brick and no persistent loop: the bricks' work differs by more than ten times (on
 // a mug's axis the whole wall is equally near), and the hardware's own order balances it.
-__global__ void __launch_bounds__(kBqThreads) nearest_bricks_kernel(FwnView f, Lattice L, float* __restrict__ d2out) {
+__global__ void __launch_bounds__(kBqThreads, 3) nearest_bricks_kernel(FwnView f, Lattice L, float* __restrict__ d2out) {
     __shared__ unsigned s_2[kNdCap2], s_1[kNdCap1], s_0[kNdCap0], s_w[kBqWarps][kNdCapW];
     __shared__ unsigned s_cnt[kBqWarps];
     __shared__ float s_u;
@@ -1061,7 +1066,8 @@ __global__ void __launch_bounds__(kBqThreads) nearest_bricks_kernel(FwnView f, L
             return r * r;
         };
         if (tid < 32) {
-            const float u = walk_near(f, 2, f.n[2], kc, [](int i) { return i; });
+            int kn;
+            const float u = walk_near(f, 2, f.n[2], kc, [](int i) { return i; }, kn);
             if (tid == 0) s_u = u;
         }
         __syncthreads();
@@ -1085,27 +1091,31 @@ __global__ void __launch_bounds__(kBqThreads) nearest_bricks_kernel(FwnView f, L
             const f3 oc = mk(lattice_mid(L.mn[0], bx * 8 + ox, 1.5f, L.h), lattice_mid(L.mn[1], by * 8 + oy, 1.5f, L.h),
                              lattice_mid(L.mn[2], bz * 8 + oz, 1.5f, L.h));
             const float rho_o = 2.5981f * L.h * 1.0002f + slop;
-            int nc = all ? f.n[0] : n0;
+            int nc = all ? f.n[0] : n0, kn = -1, far0 = 0;
             const unsigned* near = nullptr;  // null: every cluster
             float start = 1e6f;              // distances start at 1e6 (squared 1e12)
             if (!all) {
                 near = s_0;
-                const float u = walk_near(f, 0, n0, oc, [&](int i) { return (int)s_0[i]; });
+                const float u = walk_near(f, 0, n0, oc, [&](int i) { return (int)s_0[i]; }, kn);
                 start = fminf(start, u + rho_o);
-                const float lim = reach_sq(u, rho_o);
-                int n = 0;
+                const float lim = reach_sq(u, rho_o), soon = u * u;  // (u + rho / 4 to u + rho: within 1%)
+                int n = 0, m = 0;  // kept from the front (near ones) and from the back of the list
                 for (int base = 0; base < n0; base += 32) {
                     const int i = base + lane;
-                    const bool keep = i < n0 && !(box_dist_sq(f.box[0] + 2 * (size_t)s_0[i], oc) > lim);
-                    const unsigned bal = __ballot_sync(0xffffffffu, keep);
-                    const int slot = n + __popc(bal & ((1u << lane) - 1u));
-                    if (keep && slot < kNdCapW) s_w[warp][slot] = s_0[i];
-                    n += __popc(bal);
+                    const float d = i < n0 && (int)s_0[i] != kn ? box_dist_sq(f.box[0] + 2 * (size_t)s_0[i], oc) : 2.0f * lim;
+                    const bool keep = !(d > lim), first = keep && !(d > soon);
+                    const unsigned bal = __ballot_sync(0xffffffffu, keep), balf = __ballot_sync(0xffffffffu, first);
+                    const unsigned below = (1u << lane) - 1u;
+                    const int slot = first ? n + __popc(balf & below) : kNdCapW - 1 - (m + __popc(bal & ~balf & below));
+                    n += __popc(balf);
+                    m += __popc(bal & ~balf);
+                    if (keep && n + m <= kNdCapW) s_w[warp][slot] = s_0[i];
                 }
                 __syncwarp();
-                if (n <= kNdCapW) {
+                if (n + m <= kNdCapW) {
                     near = s_w[warp];
-                    nc = n;
+                    nc = n + m;
+                    far0 = n;
                 }
             }
             f3 p[2];
@@ -1119,14 +1129,53 @@ __global__ void __launch_bounds__(kBqThreads) nearest_bricks_kernel(FwnView f, L
                 lim[k] = start * 1.00002f + slop;
                 lim_sq[k] = lim[k] * lim[k];
             }
-            for (int i = 0; i < nc; ++i) {
-                const long long k0 = near ? (long long)near[i] : i;
+            // the octant's eight 2^3 cubes: lane group g = lane / 8 holds voxels of cubes g and 4 + g
+            f3 cc[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int cv = morton_voxel(warp * 64 + k * 32 + (lane & 24));
+                cc[k] = mk(lattice_mid(L.mn[0], bx * 8 + (cv & 7), 0.5f, L.h),
+                           lattice_mid(L.mn[1], by * 8 + ((cv >> 3) & 7), 0.5f, L.h),
+                           lattice_mid(L.mn[2], bz * 8 + (cv >> 6), 0.5f, L.h));
+            }
+            const float rho_c = 0.8661f * L.h * 1.0002f + slop;
+            auto cube_reach = [&](int k) {  // a cube's points are within this of whatever changes a voxel of it
+                float l = lim[k];
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) l = fmaxf(l, __shfl_xor_sync(0xffffffffu, l, o));
+                return l * 1.00002f + rho_c;
+            };
+            // the triangles of cluster k0: each against the cubes, a lane a pair, then those that
+            // come near voxel by voxel
+            auto take = [&](long long k0, unsigned cubes) {
                 bool need[2];
 #pragma unroll
-                for (int k = 0; k < 2; ++k) need[k] = !(box_dist_sq(f.box[0] + 2 * k0, p[k]) > lim_sq[k]);
-                if (!__any_sync(0xffffffffu, need[0] || need[1])) continue;
-                const int m = (int)min((long long)kFwnLeaf, f.T - k0 * kFwnLeaf);
-                for (int t = 0; t < m; ++t) {
+                for (int k = 0; k < 2; ++k)
+                    need[k] = ((cubes >> (4 * k + (lane >> 3))) & 1u) &&
+                              !(box_dist_sq(f.box[0] + 2 * k0, p[k]) > lim_sq[k]);
+                if (!__any_sync(0xffffffffu, need[0] || need[1])) return;
+                const float r0 = cube_reach(0), r1 = cube_reach(1);
+                const long long tl = k0 * kFwnLeaf + (lane & 7);
+                unsigned pass[2];
+                {
+                    const bool on = tl < f.T;
+                    const float4* o = f.leaf + 5 * (on ? tl : 0);
+                    const float4 g = __ldg(o), n = __ldg(o + 1);
+                    const float nn = __ldg(&o[4].y) * 1.0001f;
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const float dx = g.x - cc[k].x, dy = g.y - cc[k].y, dz = g.z - cc[k].z;
+                        const float rr = k ? r1 : r0, r = rr + g.w;
+                        const float h = __fmaf_rn(n.z, dz, __fmaf_rn(n.y, dy, n.x * dx));
+                        pass[k] = __ballot_sync(0xffffffffu, on && !(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)) > r * r ||
+                                                                     h * h > nn * (rr * rr)));
+                    }
+                }
+                unsigned some = pass[0] | pass[1];
+                some |= some >> 16;
+                some = (some | some >> 8) & 0xffu;
+                for (; some; some &= some - 1) {
+                    const int t = __ffs(some) - 1;
                     const float4* o = f.leaf + 5 * (k0 * kFwnLeaf + t);
                     const float4 g = __ldg(o), n = __ldg(o + 1);
                     const float nn = __ldg(&o[4].y) * 1.0001f;
@@ -1134,7 +1183,8 @@ __global__ void __launch_bounds__(kBqThreads) nearest_bricks_kernel(FwnView f, L
                     for (int k = 0; k < 2; ++k) {
                         const float dx = g.x - p[k].x, dy = g.y - p[k].y, dz = g.z - p[k].z, r = lim[k] + g.w;
                         const float h = __fmaf_rn(n.z, dz, __fmaf_rn(n.y, dy, n.x * dx));
-                        if (!need[k] || __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)) > r * r || h * h > nn * lim_sq[k])
+                        if (!need[k] || !((pass[k] >> ((lane & 24) + t)) & 1u) ||
+                            __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)) > r * r || h * h > nn * lim_sq[k])
                             continue;
                         const float d2 = leaf_dist_sq(o, p[k]);
                         if (d2 < best[k]) {
@@ -1143,6 +1193,30 @@ __global__ void __launch_bounds__(kBqThreads) nearest_bricks_kernel(FwnView f, L
                             lim_sq[k] = lim[k] * lim[k];
                         }
                     }
+                }
+            };
+            // the cluster found nearest to the centre first, then the near ones, then the others:
+            // four clusters at a time against the cubes, a lane a pair
+            if (kn >= 0) take(kn, 0xffu);
+            const int cv = morton_voxel(warp * 64 + 8 * (lane & 7));
+            const f3 cl = mk(lattice_mid(L.mn[0], bx * 8 + (cv & 7), 0.5f, L.h),
+                             lattice_mid(L.mn[1], by * 8 + ((cv >> 3) & 7), 0.5f, L.h),
+                             lattice_mid(L.mn[2], bz * 8 + (cv >> 6), 0.5f, L.h));
+            for (int base = 0; base < nc; base += 4) {
+                const float r0 = __shfl_sync(0xffffffffu, cube_reach(0), 8 * (lane & 3)),
+                            r1 = __shfl_sync(0xffffffffu, cube_reach(1), 8 * (lane & 3));
+                const float r = (lane & 4) ? r1 : r0;
+                const int i = base + (lane >> 3);
+                unsigned k = i;
+                if (near == s_w[warp]) k = near[min(i, nc - 1) < far0 ? i : kNdCapW - 1 - (min(i, nc - 1) - far0)];
+                else if (near) k = near[min(i, nc - 1)];
+                unsigned pass = __ballot_sync(0xffffffffu, i < nc && (int)k != kn &&
+                                                               !(box_dist_sq(f.box[0] + 2 * (size_t)k, cl) > r * r));
+                while (pass) {
+                    const int q = (__ffs(pass) - 1) & ~7;
+                    const unsigned cubes = (pass >> q) & 0xffu;
+                    pass &= ~(0xffu << q);
+                    take((long long)__shfl_sync(0xffffffffu, k, q), cubes);
                 }
             }
 #pragma unroll
