@@ -648,19 +648,28 @@ __global__ void __launch_bounds__(kBwdThreads) mlp_backward_kernel(const float* 
     }
 }
 
+// Sums the partial gradients and losses in CTA order, a thread a parameter and one more for the
+// loss. Bound by the latency of the chain: 16 partials are read at a time, added in order, and
+// the loss does not wait behind a parameter (4,096 rows
+// 4.8 -> 3.8 us).
 __global__ void mlp_reduce_kernel(const float* __restrict__ partial, const float* __restrict__ loss_partial,
                                   int nparts, float* __restrict__ grad, float* __restrict__ loss) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < kMlpParams) {
-        float s = 0.0f;
-        for (int p = 0; p < nparts; ++p) s += partial[(long long)p * kMlpParams + i];
-        grad[i] = s;
+    if (i > kMlpParams) return;
+    const float* from = i < kMlpParams ? partial + i : loss_partial;
+    const long long stride = i < kMlpParams ? kMlpParams : 1;
+    float s = 0.0f;
+    int p = 0;
+    for (; p + 16 <= nparts; p += 16) {
+        float v[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = __ldg(from + (p + k) * stride);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) s += v[k];
     }
-    if (i == 0) {
-        float s = 0.0f;
-        for (int p = 0; p < nparts; ++p) s += loss_partial[p];
-        *loss = s;
-    }
+    for (; p < nparts; ++p) s += __ldg(from + p * stride);
+    if (i < kMlpParams) grad[i] = s;
+    else *loss = s;
 }
 
 __global__ void adam_kernel(float* __restrict__ P, const float* __restrict__ g, float* __restrict__ m,
@@ -813,7 +822,7 @@ void launch_mlp_backward(const float* P, const float* X, const float* y, const f
     cudaFuncSetAttribute(mlp_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmemBytes);
     mlp_backward_kernel<<<parts, kBwdThreads, kBwdSmemBytes, st>>>(P, X, y, wt, B, partial, loss_partial);
     GBSDF_COUNT_LAUNCH();
-    mlp_reduce_kernel<<<(kMlpParams + 255) / 256, 256, 0, st>>>(partial, loss_partial, parts, grad, loss);
+    mlp_reduce_kernel<<<(kMlpParams + 1 + 63) / 64, 64, 0, st>>>(partial, loss_partial, parts, grad, loss);
 }
 
 void launch_adam(float* P, const float* g, float* m, float* v, int n, float lr, float b1, float b2, float eps,
