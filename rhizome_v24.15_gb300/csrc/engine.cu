@@ -6,13 +6,13 @@
 //
 //   H2D triangles -> [prep] per-triangle records, brick / strip counts
 //   -> [bin] counting-sort lists  -> [init] sentinel fill -> [A] brick splat
-//   -> [B] parity ballots -> [C] exact winding of unknown columns
+//   -> [B] parity strips -> [C] exact winding of unknown columns
 //   -> [D] eikonal sweeps (+ audit / clamp) -> [E] stratified verify + patch boxes
 //   -> [F] sign apply -> D2H (host output) .
 //
 // Host synchronisation points: one after binning (list sizes, guards), one after
-// the parity pass (unknown-voxel count), one at the end (status); the eikonal round
-// loop and the verify / patch loop are driven by device-side state.
+// the parity pass (unknown-voxel count), one at the end (status) and one per patch round; the
+// eikonal round loop is driven by device-side state.
 #include <algorithm>
 #include <chrono>
 #include <cmath>

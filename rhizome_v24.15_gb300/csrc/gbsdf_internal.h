@@ -57,7 +57,7 @@ struct DevState {
     unsigned long long csr_entries;    // entries of the reference's supercell CSR (guard)
     unsigned long long invalid_tris;   // non-finite or out-of-range coordinates
     unsigned long long active_bricks;
-    unsigned long long dense_bricks;   // bricks with more binned triangles than the dense-splat threshold
+    unsigned long long dense_bricks;   // bricks of many binned clusters, splatted first
     unsigned long long band_voxels;
     unsigned long long splat_evals;    // exact point-triangle evaluations
     unsigned long long unknown_columns;
