@@ -461,7 +461,8 @@ __device__ __forceinline__ void leaf_term(const float4* __restrict__ leaf, const
 // ballot, in order) children next, two clusters' sixteen or four clusters' eight triangles at a
 // time. What a walk leaves undecided is walked again with a wider near range (smaller truncation
 // bounds, more exact terms): beta0, 8, 32; then the voxel is handed to the sum over every
-// triangle. Latency-bound: a walk is a chain of some tens of
+// triangle. The blocks' leftovers start at 32: most come from 8 undecided (512^3 vessel tree, its
+// two queries 3.6 + 3.1 ms from 8, 3.1 + 3.0 from 16, 2.9 + 2.7 so; 640^3 blob 5.1, 6.1, 4.2). Latency-bound: a walk is a chain of some tens of
 // loads and ballots; the lists are short (4,096 probes, the block kernel's leftovers).
 __global__ void __launch_bounds__(kQueryThreads) fwn_query_kernel(
     FwnView f, Lattice L, const long long* __restrict__ list, const unsigned long long* __restrict__ list_n,
@@ -1245,7 +1246,7 @@ void winding_query(const Fwn& f, const float* tri9, long long T, const Lattice& 
     GBSDF_COUNT_LAUNCH();
     fwn_query_kernel<<<(unsigned)(num_sms * 4), kQueryThreads, 0, st>>>(
         view_of(f, T), L, list ? list : f.fb2, list ? &ds->listed : &ds->fwn_left, list ? list_cap : f.fb_cap, consumer,
-        only_if, sbits, dist, dist_sq, surf_tol_vox, ds, f.fb, f.fb_cap, list ? kFwnBeta : kFwnBetaFine);
+        only_if, sbits, dist, dist_sq, surf_tol_vox, ds, f.fb, f.fb_cap, list ? kFwnBeta : kFwnBetaRefine);
     launch_gwn_team(tri9, T, L, f.fb, f.fb_cap, consumer, sbits, recheck, recheck_cap, dist, dist_sq, surf_tol_vox, ds,
                     num_sms, st, only_if);
 }
