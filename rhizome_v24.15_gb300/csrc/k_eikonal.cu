@@ -382,14 +382,16 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         : "memory");
 }
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int x, int y, int z, const void* src) {
-    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];\n"
-                 "cp.async.bulk.commit_group;\n" ::"l"(reinterpret_cast<uint64_t>(map)),
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];\n" ::"l"(
+                     reinterpret_cast<uint64_t>(map)),
                  "r"(x), "r"(y), "r"(z), "r"(smem_u32(src))
                  : "memory");
 }
-// at most one of this thread's stores still reads its shared memory / none is in flight
+// One group a chunk, whatever it stores: a wait counts groups, so that a chunk of one store
+// where the others have two would let a buffer be written while its store still reads it.
+__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;\n" ::: "memory"); }
+// at most one of this thread's groups still reads its shared memory / none is in flight
 __device__ __forceinline__ void tma_store_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory"); }
-__device__ __forceinline__ void tma_store_wait_read2() { asm volatile("cp.async.bulk.wait_group.read 2;\n" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
 // float offset of element j (0..7) of staged line r in a 32-byte-swizzled tile
 __device__ __forceinline__ int tsw(int r, int j) { return r * 8 + ((((j >> 2) ^ (r >> 2)) & 1) << 2) + (j & 3); }
@@ -699,6 +701,7 @@ __global__ void __launch_bounds__(XPipe<ZT>::kThreads, ZT == kXZ ? 3 : 1) sweep_
             mbar_arrive(&empty[ci % kSlots]);
             if (z < dz) {  // rows past dy and voxels past dx are clipped
                 tma_store_3d(&tmo, xc, y0, z, stage + (ci & 1) * (kXY * kXC));
+                tma_store_commit();
                 tma_store_wait_read1();
             }
         }
@@ -879,7 +882,8 @@ __global__ void __launch_bounds__(kP2Threads, 4) sweep_x_pipe2_kernel(const __gr
             mbar_arrive(&empty[ci % kP2S]);
             if (za < dz) tma_store_3d(&tmo, xc, y0, za, out);
             if (zb < dz) tma_store_3d(&tmo, xc, y0, zb, out + 2 * kXY);
-            tma_store_wait_read2();
+            tma_store_commit();
+            tma_store_wait_read1();
         }
         __syncwarp();  // the next chunk's buffers are free
     }
