@@ -1088,7 +1088,9 @@ __global__ void __launch_bounds__(kBqThreads, 3) nearest_bricks_kernel(FwnView f
         if (n2 <= kNdCap2) n1 = cta_list(n2 * kFwnFan, s_1, kNdCap1, s_cnt, [&](int i) { return children(s_2, 1, i); });
         if (n2 <= kNdCap2 && n1 <= kNdCap1)
             n0 = cta_list(n1 * kFwnFan, s_0, kNdCap0, s_cnt, [&](int i) { return children(s_1, 0, i); });
-        const bool all = n2 > kNdCap2 || n1 > kNdCap1 || n0 > kNdCap0;  // too many to list: every cluster
+        // too many to list, or none (an FP32 distance to a sliver can fall short of its own box):
+        // every cluster
+        const bool all = n2 > kNdCap2 || n1 > kNdCap1 || n0 > kNdCap0 || n0 == 0;
         {
             // a warp takes the 4 x 4 x 4 voxels of one octant (Morton order), two a lane, and
             // keeps the clusters that pass for the octant
@@ -1107,8 +1109,10 @@ __global__ void __launch_bounds__(kBqThreads, 3) nearest_bricks_kernel(FwnView f
                 int n = 0, m = 0;  // kept from the front (near ones) and from the back of the list
                 for (int base = 0; base < n0; base += 32) {
                     const int i = base + lane;
-                    const float d = i < n0 && (int)s_0[i] != kn ? box_dist_sq(f.box[0] + 2 * (size_t)s_0[i], oc) : 2.0f * lim;
-                    const bool keep = !(d > lim), first = keep && !(d > soon);
+                    // (u, and with it lim, is NaN when the nearest cluster has no area: all pass)
+                    const bool on = i < n0 && (int)s_0[i] != kn;
+                    const float d = on ? box_dist_sq(f.box[0] + 2 * (size_t)s_0[i], oc) : 0.0f;
+                    const bool keep = on && !(d > lim), first = keep && !(d > soon);
                     const unsigned bal = __ballot_sync(0xffffffffu, keep), balf = __ballot_sync(0xffffffffu, first);
                     const unsigned below = (1u << lane) - 1u;
                     const int slot = first ? n + __popc(balf & below) : kNdCapW - 1 - (m + __popc(bal & ~balf & below));
