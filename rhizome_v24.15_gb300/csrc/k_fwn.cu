@@ -1098,135 +1098,148 @@ __global__ void __launch_bounds__(kBqThreads, 3) nearest_bricks_kernel(FwnView f
             const f3 oc = mk(lattice_mid(L.mn[0], bx * 8 + ox, 1.5f, L.h), lattice_mid(L.mn[1], by * 8 + oy, 1.5f, L.h),
                              lattice_mid(L.mn[2], bz * 8 + oz, 1.5f, L.h));
             const float rho_o = 2.5981f * L.h * 1.0002f + slop;
-            int nc = all ? f.n[0] : n0, kn = -1, far0 = 0;
-            const unsigned* near = nullptr;  // null: every cluster
-            float start = 1e6f;              // distances start at 1e6 (squared 1e12)
-            if (!all) {
-                near = s_0;
-                const float u = walk_near(f, 0, n0, oc, [&](int i) { return (int)s_0[i]; }, kn);
-                start = fminf(start, u + rho_o);
-                const float lim = reach_sq(u, rho_o), soon = u * u;  // (u + rho / 4 to u + rho: within 1%)
-                int n = 0, m = 0;  // kept from the front (near ones) and from the back of the list
-                for (int base = 0; base < n0; base += 32) {
-                    const int i = base + lane;
-                    // (u, and with it lim, is NaN when the nearest cluster has no area: all pass)
-                    const bool on = i < n0 && (int)s_0[i] != kn;
-                    const float d = on ? box_dist_sq(f.box[0] + 2 * (size_t)s_0[i], oc) : 0.0f;
-                    const bool keep = on && !(d > lim), first = keep && !(d > soon);
-                    const unsigned bal = __ballot_sync(0xffffffffu, keep), balf = __ballot_sync(0xffffffffu, first);
-                    const unsigned below = (1u << lane) - 1u;
-                    const int slot = first ? n + __popc(balf & below) : kNdCapW - 1 - (m + __popc(bal & ~balf & below));
-                    n += __popc(balf);
-                    m += __popc(bal & ~balf);
-                    if (keep && n + m <= kNdCapW) s_w[warp][slot] = s_0[i];
-                }
-                __syncwarp();
-                if (n + m <= kNdCapW) {
-                    near = s_w[warp];
-                    nc = n + m;
-                    far0 = n;
-                }
-            }
-            f3 p[2];
-            float best[2] = {1e12f, 1e12f}, lim[2], lim_sq[2];
             int vx[2];
+            float best[2];
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                vx[k] = morton_voxel(warp * 64 + k * 32 + lane);
-                p[k] = lattice_point(L.mn[0], L.mn[1], L.mn[2], bx * 8 + (vx[k] & 7), by * 8 + ((vx[k] >> 3) & 7),
-                                     bz * 8 + (vx[k] >> 6), L.h);
-                lim[k] = start * 1.00002f + slop;
-                lim_sq[k] = lim[k] * lim[k];
-            }
-            // the octant's eight 2^3 cubes: lane group g = lane / 8 holds voxels of cubes g and 4 + g
-            f3 cc[2];
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const int cv = morton_voxel(warp * 64 + k * 32 + (lane & 24));
-                cc[k] = mk(lattice_mid(L.mn[0], bx * 8 + (cv & 7), 0.5f, L.h),
-                           lattice_mid(L.mn[1], by * 8 + ((cv >> 3) & 7), 0.5f, L.h),
-                           lattice_mid(L.mn[2], bz * 8 + (cv >> 6), 0.5f, L.h));
-            }
-            const float rho_c = 0.8661f * L.h * 1.0002f + slop;
-            auto cube_reach = [&](int k) {  // a cube's points are within this of whatever changes a voxel of it
-                float l = lim[k];
-#pragma unroll
-                for (int o = 1; o < 8; o <<= 1) l = fmaxf(l, __shfl_xor_sync(0xffffffffu, l, o));
-                return l * 1.00002f + rho_c;
-            };
-            // the triangles of cluster k0: each against the cubes, a lane a pair, then those that
-            // come near voxel by voxel
-            auto take = [&](long long k0, unsigned cubes) {
-                bool need[2];
-#pragma unroll
-                for (int k = 0; k < 2; ++k)
-                    need[k] = ((cubes >> (4 * k + (lane >> 3))) & 1u) &&
-                              !(box_dist_sq(f.box[0] + 2 * k0, p[k]) > lim_sq[k]);
-                if (!__any_sync(0xffffffffu, need[0] || need[1])) return;
-                const float r0 = cube_reach(0), r1 = cube_reach(1);
-                const long long tl = k0 * kFwnLeaf + (lane & 7);
-                unsigned pass[2];
-                {
-                    const bool on = tl < f.T;
-                    const float4* o = f.leaf + 5 * (on ? tl : 0);
-                    const float4 g = __ldg(o), n = __ldg(o + 1);
-                    const float nn = __ldg(&o[4].y) * 1.0001f;
-#pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        const float dx = g.x - cc[k].x, dy = g.y - cc[k].y, dz = g.z - cc[k].z;
-                        const float rr = k ? r1 : r0, r = rr + g.w;
-                        const float h = __fmaf_rn(n.z, dz, __fmaf_rn(n.y, dy, n.x * dx));
-                        pass[k] = __ballot_sync(0xffffffffu, on && !(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)) > r * r ||
-                                                                     h * h > nn * (rr * rr)));
+            for (int k = 0; k < 2; ++k) vx[k] = morton_voxel(warp * 64 + k * 32 + lane);
+            // A limit comes from the FP32 distance of a centre to some triangle. A triangle without
+            // area has none for some points, and a sliver's can be far off, so a limit may not
+            // hold for a voxel: a voxel left above its limit shows it, and the octant then takes every
+            // cluster without one.
+            for (bool again = false;; again = true) {
+                const bool every = all || again;
+                int nc = every ? f.n[0] : n0, kn = -1, far0 = 0;
+                const unsigned* near = nullptr;  // null: every cluster
+                // distances start at 1e6 (squared 1e12)
+                float start = again ? 1e6f : fminf(1e6f, s_u + rho);
+                if (!every) {
+                    near = s_0;
+                    const float u = walk_near(f, 0, n0, oc, [&](int i) { return (int)s_0[i]; }, kn);
+                    start = fminf(start, u + rho_o);
+                    const float lim = reach_sq(u, rho_o), soon = u * u;  // (u + rho / 4 to u + rho: within 1%)
+                    int n = 0, m = 0;  // kept from the front (near ones) and from the back of the list
+                    for (int base = 0; base < n0; base += 32) {
+                        const int i = base + lane;
+                        // (u, and with it lim, is NaN when the nearest cluster has no area: all pass)
+                        const bool on = i < n0 && (int)s_0[i] != kn;
+                        const float d = on ? box_dist_sq(f.box[0] + 2 * (size_t)s_0[i], oc) : 0.0f;
+                        const bool keep = on && !(d > lim), first = keep && !(d > soon);
+                        const unsigned bal = __ballot_sync(0xffffffffu, keep), balf = __ballot_sync(0xffffffffu, first);
+                        const unsigned below = (1u << lane) - 1u;
+                        const int slot = first ? n + __popc(balf & below) : kNdCapW - 1 - (m + __popc(bal & ~balf & below));
+                        n += __popc(balf);
+                        m += __popc(bal & ~balf);
+                        if (keep && n + m <= kNdCapW) s_w[warp][slot] = s_0[i];
+                    }
+                    __syncwarp();
+                    if (n + m <= kNdCapW) {
+                        near = s_w[warp];
+                        nc = n + m;
+                        far0 = n;
                     }
                 }
-                unsigned some = pass[0] | pass[1];
-                some |= some >> 16;
-                some = (some | some >> 8) & 0xffu;
-                for (; some; some &= some - 1) {
-                    const int t = __ffs(some) - 1;
-                    const float4* o = f.leaf + 5 * (k0 * kFwnLeaf + t);
-                    const float4 g = __ldg(o), n = __ldg(o + 1);
-                    const float nn = __ldg(&o[4].y) * 1.0001f;
+                f3 p[2];
+                float lim[2], lim_sq[2];
 #pragma unroll
-                    for (int k = 0; k < 2; ++k) {
-                        const float dx = g.x - p[k].x, dy = g.y - p[k].y, dz = g.z - p[k].z, r = lim[k] + g.w;
-                        const float h = __fmaf_rn(n.z, dz, __fmaf_rn(n.y, dy, n.x * dx));
-                        if (!need[k] || !((pass[k] >> ((lane & 24) + t)) & 1u) ||
-                            __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)) > r * r || h * h > nn * lim_sq[k])
-                            continue;
-                        const float d2 = leaf_dist_sq(o, p[k]);
-                        if (d2 < best[k]) {
-                            best[k] = d2;
-                            lim[k] = fminf(lim[k], sqrtf(d2) * 1.00002f + slop);
-                            lim_sq[k] = lim[k] * lim[k];
+                for (int k = 0; k < 2; ++k) {
+                    best[k] = 1e12f;
+                    p[k] = lattice_point(L.mn[0], L.mn[1], L.mn[2], bx * 8 + (vx[k] & 7), by * 8 + ((vx[k] >> 3) & 7),
+                                         bz * 8 + (vx[k] >> 6), L.h);
+                    lim[k] = start * 1.00002f + slop;
+                    lim_sq[k] = lim[k] * lim[k];
+                }
+                // the octant's eight 2^3 cubes: lane group g = lane / 8 holds voxels of cubes g and 4 + g
+                f3 cc[2];
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const int cv = morton_voxel(warp * 64 + k * 32 + (lane & 24));
+                    cc[k] = mk(lattice_mid(L.mn[0], bx * 8 + (cv & 7), 0.5f, L.h),
+                               lattice_mid(L.mn[1], by * 8 + ((cv >> 3) & 7), 0.5f, L.h),
+                               lattice_mid(L.mn[2], bz * 8 + (cv >> 6), 0.5f, L.h));
+                }
+                const float rho_c = 0.8661f * L.h * 1.0002f + slop;
+                auto cube_reach = [&](int k) {  // a cube's points are within this of whatever changes a voxel of it
+                    float l = lim[k];
+#pragma unroll
+                    for (int o = 1; o < 8; o <<= 1) l = fmaxf(l, __shfl_xor_sync(0xffffffffu, l, o));
+                    return l * 1.00002f + rho_c;
+                };
+                // the triangles of cluster k0: each against the cubes, a lane a pair, then those that
+                // come near voxel by voxel
+                auto take = [&](long long k0, unsigned cubes) {
+                    bool need[2];
+#pragma unroll
+                    for (int k = 0; k < 2; ++k)
+                        need[k] = ((cubes >> (4 * k + (lane >> 3))) & 1u) &&
+                                  !(box_dist_sq(f.box[0] + 2 * k0, p[k]) > lim_sq[k]);
+                    if (!__any_sync(0xffffffffu, need[0] || need[1])) return;
+                    const float r0 = cube_reach(0), r1 = cube_reach(1);
+                    const long long tl = k0 * kFwnLeaf + (lane & 7);
+                    unsigned pass[2];
+                    {
+                        const bool on = tl < f.T;
+                        const float4* o = f.leaf + 5 * (on ? tl : 0);
+                        const float4 g = __ldg(o), n = __ldg(o + 1);
+                        const float nn = __ldg(&o[4].y) * 1.0001f;
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            const float dx = g.x - cc[k].x, dy = g.y - cc[k].y, dz = g.z - cc[k].z;
+                            const float rr = k ? r1 : r0, r = rr + g.w;
+                            const float h = __fmaf_rn(n.z, dz, __fmaf_rn(n.y, dy, n.x * dx));
+                            pass[k] = __ballot_sync(0xffffffffu, on && !(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)) > r * r ||
+                                                                         h * h > nn * (rr * rr)));
                         }
                     }
+                    unsigned some = pass[0] | pass[1];
+                    some |= some >> 16;
+                    some = (some | some >> 8) & 0xffu;
+                    for (; some; some &= some - 1) {
+                        const int t = __ffs(some) - 1;
+                        const float4* o = f.leaf + 5 * (k0 * kFwnLeaf + t);
+                        const float4 g = __ldg(o), n = __ldg(o + 1);
+                        const float nn = __ldg(&o[4].y) * 1.0001f;
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            const float dx = g.x - p[k].x, dy = g.y - p[k].y, dz = g.z - p[k].z, r = lim[k] + g.w;
+                            const float h = __fmaf_rn(n.z, dz, __fmaf_rn(n.y, dy, n.x * dx));
+                            if (!need[k] || !((pass[k] >> ((lane & 24) + t)) & 1u) ||
+                                __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)) > r * r || h * h > nn * lim_sq[k])
+                                continue;
+                            const float d2 = leaf_dist_sq(o, p[k]);
+                            if (d2 < best[k]) {
+                                best[k] = d2;
+                                lim[k] = fminf(lim[k], sqrtf(d2) * 1.00002f + slop);
+                                lim_sq[k] = lim[k] * lim[k];
+                            }
+                        }
+                    }
+                };
+                // the cluster found nearest to the centre first, then the near ones, then the others:
+                // four clusters at a time against the cubes, a lane a pair
+                if (kn >= 0) take(kn, 0xffu);
+                const int cv = morton_voxel(warp * 64 + 8 * (lane & 7));
+                const f3 cl = mk(lattice_mid(L.mn[0], bx * 8 + (cv & 7), 0.5f, L.h),
+                                 lattice_mid(L.mn[1], by * 8 + ((cv >> 3) & 7), 0.5f, L.h),
+                                 lattice_mid(L.mn[2], bz * 8 + (cv >> 6), 0.5f, L.h));
+                for (int base = 0; base < nc; base += 4) {
+                    const float r0 = __shfl_sync(0xffffffffu, cube_reach(0), 8 * (lane & 3)),
+                                r1 = __shfl_sync(0xffffffffu, cube_reach(1), 8 * (lane & 3));
+                    const float r = (lane & 4) ? r1 : r0;
+                    const int i = base + (lane >> 3);
+                    unsigned k = i;
+                    if (near == s_w[warp]) k = near[min(i, nc - 1) < far0 ? i : kNdCapW - 1 - (min(i, nc - 1) - far0)];
+                    else if (near) k = near[min(i, nc - 1)];
+                    unsigned pass = __ballot_sync(0xffffffffu, i < nc && (int)k != kn &&
+                                                                   !(box_dist_sq(f.box[0] + 2 * (size_t)k, cl) > r * r));
+                    while (pass) {
+                        const int q = (__ffs(pass) - 1) & ~7;
+                        const unsigned cubes = (pass >> q) & 0xffu;
+                        pass &= ~(0xffu << q);
+                        take((long long)__shfl_sync(0xffffffffu, k, q), cubes);
+                    }
                 }
-            };
-            // the cluster found nearest to the centre first, then the near ones, then the others:
-            // four clusters at a time against the cubes, a lane a pair
-            if (kn >= 0) take(kn, 0xffu);
-            const int cv = morton_voxel(warp * 64 + 8 * (lane & 7));
-            const f3 cl = mk(lattice_mid(L.mn[0], bx * 8 + (cv & 7), 0.5f, L.h),
-                             lattice_mid(L.mn[1], by * 8 + ((cv >> 3) & 7), 0.5f, L.h),
-                             lattice_mid(L.mn[2], bz * 8 + (cv >> 6), 0.5f, L.h));
-            for (int base = 0; base < nc; base += 4) {
-                const float r0 = __shfl_sync(0xffffffffu, cube_reach(0), 8 * (lane & 3)),
-                            r1 = __shfl_sync(0xffffffffu, cube_reach(1), 8 * (lane & 3));
-                const float r = (lane & 4) ? r1 : r0;
-                const int i = base + (lane >> 3);
-                unsigned k = i;
-                if (near == s_w[warp]) k = near[min(i, nc - 1) < far0 ? i : kNdCapW - 1 - (min(i, nc - 1) - far0)];
-                else if (near) k = near[min(i, nc - 1)];
-                unsigned pass = __ballot_sync(0xffffffffu, i < nc && (int)k != kn &&
-                                                               !(box_dist_sq(f.box[0] + 2 * (size_t)k, cl) > r * r));
-                while (pass) {
-                    const int q = (__ffs(pass) - 1) & ~7;
-                    const unsigned cubes = (pass >> q) & 0xffu;
-                    pass &= ~(0xffu << q);
-                    take((long long)__shfl_sync(0xffffffffu, k, q), cubes);
-                }
+                const float held = start * 1.00002f + slop;
+                if (again || !__any_sync(0xffffffffu, fmaxf(best[0], best[1]) > held * held)) break;
             }
 #pragma unroll
             for (int k = 0; k < 2; ++k) {

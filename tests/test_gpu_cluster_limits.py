@@ -28,3 +28,27 @@ def test_nearest_cluster_without_area(engine, flat, whole):
     assert np.array_equal(np.signbit(a), np.signbit(b))
     # the two minima may differ by the rounding of one squared distance
     assert np.abs(a - b).max() <= 2.0 ** -22 * 40.0
+
+
+def _mixed(rng, n, reach):
+    """Clumps of triangles (a, a, c), whose distance exists on one side of them only, and of
+    ordinary triangles within `reach` of them."""
+    a = np.repeat(rng.uniform(8.0, 28.0, (n, 3)), 16, 0) + rng.uniform(-0.7, 0.7, (16 * n, 3))
+    e = np.concatenate([a, a, a + rng.uniform(-0.9, 0.9, (16 * n, 3))], 1)
+    c = np.repeat(rng.uniform(8.0, 28.0, (n, 3)), 8, 0)
+    b = (c + rng.uniform(-reach, reach, (8 * n, 3)))[:, None] + rng.uniform(-1.0, 1.0, (8 * n, 3, 3))
+    t = np.concatenate([e, b.reshape(-1, 9)])
+    return np.concatenate([t, np.zeros((len(t), 3))], 1).astype(np.float32)
+
+
+@pytest.mark.parametrize("n,reach", [(1, 0.0), (1, 6.0), (3, 6.0), (20, 3.0), (200, 2.0)])
+def test_limits_that_do_not_hold(engine, n, reach):
+    # a centre on the side where such a triangle has a distance, voxels on the other: each voxel
+    # still gets the least distance over every triangle
+    for seed in range(4):
+        tris = _mixed(np.random.default_rng(seed), n, reach)
+        mn, mx = (0, 0, 0), (37, 38, 36)
+        a, ra = engine.compute_mesh_sdf(tris, 1.0, mn, mx, path=engine.PATH_LEGACY, winding_eval=0)
+        b, rb = engine.compute_mesh_sdf(tris, 1.0, mn, mx, path=engine.PATH_LEGACY, winding_eval=1)
+        assert ra.ok and rb.ok
+        assert np.abs(np.abs(a) - np.abs(b)).max() <= 2.0 ** -22 * 40.0
