@@ -447,10 +447,9 @@ __global__ void __launch_bounds__(kSplatThreads, 4) splat_kernel(FwnView f, cons
         float u = tn < f.T ? sqrtf(leaf_dist_sq(f.leaf + 5 * tn, oc)) : inf;
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1) u = fminf(u, __shfl_xor_sync(0xffffffffu, u, o));
-        const float reach = fminf((u + 2.0f * rho) * 1.00002f + slop, out), reach_sq = reach * reach;
         int x[2], y[2], z[2];
         f3 p[2];
-        float best[2] = {inf, inf}, lim_sq[2];
+        float best[2], lim_sq[2], reach_sq;
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
             const int v = morton_voxel(k * 32 + lane);
@@ -458,8 +457,6 @@ __global__ void __launch_bounds__(kSplatThreads, 4) splat_kernel(FwnView f, cons
             y[k] = y0 + ((v >> 3) & 7);
             z[k] = z0 + (v >> 6);
             p[k] = lattice_point(L.mn[0], L.mn[1], L.mn[2], x[k], y[k], z[k], h);
-            const float lim = fminf(u + rho, bw) * 1.00002f + slop;
-            lim_sq[k] = lim * lim;
         }
         auto take = [&](int m) {  // the listed clusters, voxel by voxel
             __syncwarp();
@@ -521,25 +518,41 @@ __global__ void __launch_bounds__(kSplatThreads, 4) splat_kernel(FwnView f, cons
                 nt = 0;
             }
         };
-        list_tri(tn, lane < 8 && tn < f.T);  // the nearest cluster first: it sets the voxels' limits
-        for (int base = 0; base < n; base += 32) {
-            const int e = base + lane;
-            const unsigned k = e < n ? mine[e] : 0u;
-            unsigned near = __ballot_sync(0xffffffffu, e < n && k != (unsigned)kn &&
-                                                           !(box_dist_sq(f.box[0] + 2 * (size_t)k, oc) > reach_sq));
-            while (near) {  // four clusters of eight triangles at a time
-                int src[4];
+        // The limits hold for the distances as computed, unless the triangle they come from is one
+        // without area (it has no distance for some points) or a sliver: a voxel left above its
+        // limit shows it, and the octant is taken again with the band as its only limit.
+        for (;;) {
+            const float reach = fminf((u + 2.0f * rho) * 1.00002f + slop, out);
+            const float lim = fminf(u + rho, bw) * 1.00002f + slop, held = lim * lim;
+            reach_sq = reach * reach;
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    src[q] = __ffs(near) - 1;
-                    near &= near - 1u;
-                }
-                const int sl = lane < 8 ? src[0] : lane < 16 ? src[1] : lane < 24 ? src[2] : src[3];
-                const long long t = (long long)__shfl_sync(0xffffffffu, k, sl & 31) * kFwnLeaf + (lane & 7);
-                list_tri(t, sl >= 0 && t < f.T);
+            for (int k = 0; k < 2; ++k) {
+                best[k] = inf;
+                lim_sq[k] = held;
             }
+            list_tri(tn, lane < 8 && tn < f.T);  // the nearest cluster first: it sets the voxels' limits
+            for (int base = 0; base < n; base += 32) {
+                const int e = base + lane;
+                const unsigned k = e < n ? mine[e] : 0u;
+                unsigned near = __ballot_sync(0xffffffffu, e < n && k != (unsigned)kn &&
+                                                               !(box_dist_sq(f.box[0] + 2 * (size_t)k, oc) > reach_sq));
+                while (near) {  // four clusters of eight triangles at a time
+                    int src[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        src[q] = __ffs(near) - 1;
+                        near &= near - 1u;
+                    }
+                    const int sl = lane < 8 ? src[0] : lane < 16 ? src[1] : lane < 24 ? src[2] : src[3];
+                    const long long t = (long long)__shfl_sync(0xffffffffu, k, sl & 31) * kFwnLeaf + (lane & 7);
+                    list_tri(t, sl >= 0 && t < f.T);
+                }
+            }
+            take(nt);
+            nt = 0;
+            if (!(u + rho < bw) || !__any_sync(0xffffffffu, fmaxf(best[0], best[1]) > held)) break;
+            u = inf;
         }
-        take(nt);
 #pragma unroll
         for (int k = 0; k < 2; ++k)
             if (best[k] != inf && x[k] < L.dims[0] && y[k] < L.dims[1] && z[k] < L.dims[2]) {

@@ -52,3 +52,17 @@ def test_limits_that_do_not_hold(engine, n, reach):
         b, rb = engine.compute_mesh_sdf(tris, 1.0, mn, mx, path=engine.PATH_LEGACY, winding_eval=1)
         assert ra.ok and rb.ok
         assert np.abs(np.abs(a) - np.abs(b)).max() <= 2.0 ** -22 * 40.0
+
+
+@pytest.mark.parametrize("n,reach", [(1, 0.0), (1, 6.0), (3, 6.0), (20, 3.0), (200, 2.0)])
+def test_band_limits_that_do_not_hold(engine, oracle, n, reach):
+    # the same in the band splat (8 voxels), against the oracle's
+    for seed in range(3):
+        tris = _mixed(np.random.default_rng(seed), n, reach)
+        mn, mx = (0, 0, 0), (37, 38, 36)
+        out, res = engine.compute_mesh_sdf(tris, 1.0, mn, mx, mode=engine.MODE_EXACT_SIGNS, path=engine.PATH_FAST,
+                                           raise_on_error=False)
+        st, ref, _, ost = oracle.fast_sdf(tris, 1.0, mn, mx, fsm_mode=0, gwn_mode=1, signed_parity=True)
+        assert res.status == st and res.stats["band_voxels"] == ost["band_voxels"] > 0
+        if st == oracle.OK:
+            assert np.array_equal(np.abs(out).view(np.uint32), np.abs(ref).view(np.uint32))
