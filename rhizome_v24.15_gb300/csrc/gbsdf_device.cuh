@@ -124,8 +124,10 @@ __device__ __forceinline__ float solid_angle_fast(f3 p, f3 v0, f3 v1, f3 v2, boo
     return 2.0f * atan2f(det, denom);
 }
 
-// The same formula in FP64 from the FP32 inputs (used only for re-checks).
-__device__ __forceinline__ double solid_angle_f64(f3 pf, f3 v0, f3 v1, f3 v2) {
+// The same formula in FP64 from the FP32 inputs (used only for re-checks), with the two terms of
+// its tangent and the product of the lengths they scale with (all 0 next to a vertex).
+__device__ __forceinline__ double solid_angle_f64(f3 pf, f3 v0, f3 v1, f3 v2, double& det, double& denom,
+                                                  double& labc) {
     double px = pf.x, py = pf.y, pz = pf.z;
     double ax = v0.x - px, ay = v0.y - py, az = v0.z - pz;
     double bx = v1.x - px, by = v1.y - py, bz = v1.z - pz;
@@ -133,11 +135,17 @@ __device__ __forceinline__ double solid_angle_f64(f3 pf, f3 v0, f3 v1, f3 v2) {
     double la = sqrt(ax * ax + ay * ay + az * az);
     double lb = sqrt(bx * bx + by * by + bz * bz);
     double lc = sqrt(cx * cx + cy * cy + cz * cz);
+    det = denom = labc = 0.0;
     if (la <= 1e-6 || lb <= 1e-6 || lc <= 1e-6) return 0.0;
-    double det = ax * (by * cz - bz * cy) - ay * (bx * cz - bz * cx) + az * (bx * cy - by * cx);
-    double denom = la * lb * lc + (ax * bx + ay * by + az * bz) * lc + (bx * cx + by * cy + bz * cz) * la +
-                   (cx * ax + cy * ay + cz * az) * lb;
+    labc = la * lb * lc;
+    det = ax * (by * cz - bz * cy) - ay * (bx * cz - bz * cx) + az * (bx * cy - by * cx);
+    denom = labc + (ax * bx + ay * by + az * bz) * lc + (bx * cx + by * cy + bz * cz) * la +
+            (cx * ax + cy * ay + cz * az) * lb;
     return 2.0 * atan2(det, denom);
+}
+__device__ __forceinline__ double solid_angle_f64(f3 pf, f3 v0, f3 v1, f3 v2) {
+    double det, denom, labc;
+    return solid_angle_f64(pf, v0, v1, v2, det, denom, labc);
 }
 
 // x / 3, correctly rounded, without a general division: q = RN(x * RN(1/3)), the exact

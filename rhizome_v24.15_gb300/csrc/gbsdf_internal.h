@@ -240,8 +240,9 @@ void launch_winding_blocks(const Fwn& f, const float* tri9, long long T, const L
 // blocks it can (as launch_winding_blocks does; f: the caps' clusters) and leaves the others
 // marked.
 struct Crossings {
-    const uint32_t* k;    // the voxels with a nonzero crossing number (sign-word layout)
-    const unsigned* bad;  // the columns to leave out, a bit per column (x fastest)
+    const uint32_t* k;       // the voxels with a nonzero crossing number (sign-word layout)
+    const uint32_t* unsure;  // the voxels on a crossing, to leave out (the same layout)
+    const unsigned* bad;     // the columns to leave out, a bit per column (x fastest)
 };
 constexpr long long kCapsMinVoxels = 32768;  // marked voxels from which the pass pays off
 size_t edge_table_bytes(long long T);

@@ -16,12 +16,15 @@
 // boundary of a chain is closed, and so is each connected part of it); a fan from one vertex of
 // each component.
 //
-// The crossings: vertical rays 3.7e-4 h / 5.1e-4 h beside the lattice columns (the exact-signs
-// mode's); a voxel farther than the step from the mesh and the caps has the ray start's winding
-// number. Edge functions are FP32 with an error bound and FP64 inside it (FP32 coordinates'
-// differences and their products are exact there); a ray that meets an edge within FP64's own
-// rounding, or a column whose crossings do not sum to zero, is left out. Each crossing adds
-// its sign at its height in an integer grid, and a pass up the columns sums it.
+// The crossings: a voxel's ray goes straight down its own column, moved by an infinitesimal
+// (e, e^2) where it meets an edge, so that the crossing number below a voxel is the voxel's own and
+// nothing has to be known about its distance to the mesh. The edge functions and the height are
+// FP32 with a bound of their rounding, which grows with the triangle and not with the voxel, and
+// FP64 where a sign or the voxel above is not certain within it (all but a few in 10^4; a sliver's
+// height follows from its area by the same bound). The two triangles of an edge take its ends
+// in one order, so they agree on its side. A voxel that a crossing's height cannot be told
+// from even in FP64, and a column whose crossings do not sum to zero, are left out. Each
+// crossing adds its sign at its height in an integer grid, and a pass up the columns sums it.
 #include <algorithm>
 
 #include "gwn_device.cuh"
@@ -193,21 +196,30 @@ __global__ void caps_kernel(const float* __restrict__ t9, const uint2* __restric
     }
 }
 
-constexpr float kRayX = 3.7e-4f, kRayY = 5.1e-4f;
-
-// Edge function of the ray (rx, ry) and the directed edge (a, b) in xy, its sign certain: 1, -1,
-// or 0 where even FP64 cannot tell.
-__device__ __forceinline__ double edge_fn(const float* a, const float* b, double rx, double ry) {
-    const double ux = (double)b[0] - a[0], uy = (double)b[1] - a[1], wx = rx - a[0], wy = ry - a[1];
+// Edge function of a column (x, y) and the directed edge (a, b) in xy: d, the magnitude m of its
+// terms (its rounding is within 4e-16 m), and the side s of the column moved by (e, e^2), 0 for an
+// edge without extent. Differences of FP32 coordinates and their products are exact in FP64 but for
+// far apart magnitudes; with the ends in order both triangles of an edge get the same.
+struct EdgeFn {
+    double d, m;
+    int s;
+};
+__device__ __forceinline__ EdgeFn edge_fn(const float* a, const float* b, double x, double y) {
+    const bool turn = b[0] < a[0] || (b[0] == a[0] && b[1] < a[1]);
+    const float *lo = turn ? b : a, *hi = turn ? a : b;
+    const double ux = (double)hi[0] - lo[0], uy = (double)hi[1] - lo[1], wx = x - lo[0], wy = y - lo[1];
     const double p = ux * wy, q = uy * wx, d = p - q;
-    return fabs(d) > 1e-14 * (fabs(p) + fabs(q)) ? d : 0.0;
+    int s = (d > 0.0) - (d < 0.0);
+    if (s == 0) s = (uy < 0.0) - (uy > 0.0);
+    if (s == 0) s = (ux > 0.0) - (ux < 0.0);
+    return turn ? EdgeFn{-d, fabs(p) + fabs(q), -s} : EdgeFn{d, fabs(p) + fabs(q), s};
 }
 
 // One warp per (triangle, row slice): the lanes take the columns of the triangle's xy box. A
 // crossing adds its sign to its column's sum and, at the first voxel above it, to the grid.
 __global__ void __launch_bounds__(256) crossings_kernel(const float* __restrict__ t9, long long T, Lattice L,
                                                         int slices, int* __restrict__ grid, int* __restrict__ colsum,
-                                                        unsigned* __restrict__ colbad) {
+                                                        unsigned* __restrict__ colbad, uint32_t* __restrict__ unsure) {
     const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const long long t = w / slices;
@@ -215,57 +227,77 @@ __global__ void __launch_bounds__(256) crossings_kernel(const float* __restrict_
     if (t >= T) return;
     const float* v = t9 + 9 * t;
     const float h = L.h;
+    const int dz = L.dims[2];
     const float x0 = fminf(v[0], fminf(v[3], v[6])), x1 = fmaxf(v[0], fmaxf(v[3], v[6]));
     const float y0 = fminf(v[1], fminf(v[4], v[7])), y1 = fmaxf(v[1], fmaxf(v[4], v[7]));
-    // the columns whose rays can lie in the box, one more on each side for the rounding
-    const int ix0 = (int)fmaxf(floorf(fmaxf(x0 / h - (float)L.mn[0], -2.0f)) - 1.0f, 0.0f),
-              iy0 = (int)fmaxf(floorf(fmaxf(y0 / h - (float)L.mn[1], -2.0f)) - 1.0f, 0.0f);
-    const int ix1 = (int)fminf(ceilf(fminf(x1 / h - (float)L.mn[0], (float)L.dims[0])) + 1.0f, (float)(L.dims[0] - 1)),
-              iy1 = (int)fminf(ceilf(fminf(y1 / h - (float)L.mn[1], (float)L.dims[1])) + 1.0f, (float)(L.dims[1] - 1));
+    const float z0 = fminf(v[2], fminf(v[5], v[8])), z1 = fmaxf(v[2], fmaxf(v[5], v[8]));
+    const float zabs = fmaxf(fabsf(z0), fabsf(z1));
+    // the columns in the box, at least one more on each side for the rounding
+    auto column = [&](float c, int a, float side) {
+        const float q = c / h, far = 1.0f + 3e-7f * (fabsf(q) + fabsf((float)L.mn[a]));
+        return fminf(fmaxf(floorf(q - (float)L.mn[a] + side * far), -1.0f), (float)L.dims[a]);
+    };
+    const int ix0 = max(0, (int)column(x0, 0, -1.0f)), ix1 = min(L.dims[0] - 1, (int)column(x1, 0, 1.0f));
+    const int iy0 = max(0, (int)column(y0, 1, -1.0f)), iy1 = min(L.dims[1] - 1, (int)column(y1, 1, 1.0f));
     if (ix1 < ix0 || iy1 < iy0) return;
     const int nx = ix1 - ix0 + 1;
     const long long n = (long long)nx * (iy1 - iy0 + 1);
-    const double jx = (double)kRayX * h, jy = (double)kRayY * h;
+    auto height = [&](int z) { return (float)(L.mn[2] + z) * h; };
+    auto above = [&](auto zh) {  // the first voxel higher than zh
+        int z = (int)fminf(fmaxf(floorf((float)zh / h) - (float)L.mn[2], 0.0f), (float)dz);
+        while (z > 0 && height(z - 1) > zh) --z;
+        while (z < dz && height(z) <= zh) ++z;
+        return z;
+    };
     for (long long c = (long long)sl * 32 + lane; c < n; c += (long long)slices * 32) {
         const int x = ix0 + (int)(c % nx), y = iy0 + (int)(c / nx);
         const float qx = (float)(L.mn[0] + x) * h, qy = (float)(L.mn[1] + y) * h;
-        // a cheap look first: outside the box, or outside an edge by more than FP32's rounding
-        const float rxf = qx + kRayX * h, ryf = qy + kRayY * h;
-        const float tol = 4e-7f * (fabsf(qx) + fabsf(qy) + fabsf(x0) + fabsf(x1) + fabsf(y0) + fabsf(y1));
-        if (rxf < x0 - tol || rxf > x1 + tol || ryf < y0 - tol || ryf > y1 + tol) continue;
+        if (qx < x0 || qx > x1 || qy < y0 || qy > y1) continue;
         int pos = 0, neg = 0;
-        float df[3];
+        float df[3], e = 0.0f;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
+            // four roundings of each product at most (2^-24 each), of FP32 inputs taken as exact
             const float *a = v + 3 * k, *b = v + 3 * (k == 2 ? 0 : k + 1);
-            const float ux = b[0] - a[0], uy = b[1] - a[1], wx = rxf - a[0], wy = ryf - a[1];
-            const float d = __fmaf_rn(ux, wy, -(uy * wx));
-            const float e = tol * (fabsf(ux) + fabsf(uy) + fabsf(wx) + fabsf(wy));
-            pos += d > e;
-            neg += d < -e;
+            const float ux = b[0] - a[0], uy = b[1] - a[1], wx = qx - a[0], wy = qy - a[1];
+            const float q = uy * wx, d = __fmaf_rn(ux, wy, -q);
+            const float ek = __fmaf_rn(4e-7f, fabsf(ux * wy) + fabsf(q), 1e-36f);
+            pos += d > ek;
+            neg += d < -ek;
             df[k] = d;
+            e += ek;
         }
         if (pos && neg) continue;
         const size_t col = (size_t)y * L.dims[0] + x;
-        auto add = [&](int sg, float zh) {
-            atomicAdd(&colsum[col], sg);
-            int z = (int)fminf(fmaxf(floorf(zh / h) - (float)L.mn[2] - 1.0f, 0.0f), (float)L.dims[2]);
-            while (z < L.dims[2] && (float)(L.mn[2] + z) * h <= zh) ++z;
-            if (z < L.dims[2]) atomicAdd(&grid[((size_t)z * L.dims[1] + y) * L.dims[0] + x], sg);
-        };
-        if (pos == 3 || neg == 3) {  // certain in FP32 (FP64 issues at 1/64 of its rate here)
-            add(neg ? 1 : -1, __fmaf_rn(df[0], v[8], __fmaf_rn(df[1], v[2], df[2] * v[5])) / (df[0] + df[1] + df[2]));
-            continue;
+        auto voxel = [&](int z) { return ((size_t)z * L.dims[1] + y) * L.dims[0] + x; };
+        if (pos == 3 || neg == 3) {  // inside for certain (FP64 issues at 1/64 of FP32's rate here)
+            const float sum = df[0] + df[1] + df[2], area = fabsf(sum);
+            const float zh = __fmaf_rn(df[0], v[8], __fmaf_rn(df[1], v[2], df[2] * v[5])) / sum;
+            // the weights are off by e in all, of a true sum of at least area / 2
+            const float ez = 2.1f * e * (z1 - z0) / area + 6e-7f * zabs;
+            const int z = above(zh);
+            if (e < 0.4f * area && (z == dz || height(z) - zh > ez) && (z == 0 || zh - height(z - 1) > ez)) {
+                const int sg = neg ? 1 : -1;
+                atomicAdd(&colsum[col], sg);
+                if (z < dz) atomicAdd(&grid[voxel(z)], sg);
+                continue;
+            }
         }
-        const double rx = (double)qx + jx, ry = (double)qy + jy;
-        const double d0 = edge_fn(v, v + 3, rx, ry), d1 = edge_fn(v + 3, v + 6, rx, ry), d2 = edge_fn(v + 6, v, rx, ry);
-        const bool any_pos = d0 > 0.0 || d1 > 0.0 || d2 > 0.0, any_neg = d0 < 0.0 || d1 < 0.0 || d2 < 0.0;
-        if (any_pos && any_neg) continue;
-        if (d0 == 0.0 || d1 == 0.0 || d2 == 0.0) {  // on an edge, a vertex, or in the plane of the triangle
+        const EdgeFn f0 = edge_fn(v, v + 3, qx, qy), f1 = edge_fn(v + 3, v + 6, qx, qy), f2 = edge_fn(v + 6, v, qx, qy);
+        if (f0.s == 0 || f0.s != f1.s || f0.s != f2.s) continue;
+        const double sum = f0.d + f1.d + f2.d;
+        const double zh = (f0.d * v[8] + f1.d * v[2] + f2.d * v[5]) / sum;
+        const double ez = 1e-15 * ((f0.m + f1.m + f2.m) * ((double)z1 - z0) / fabs(sum) + zabs);
+        if (!(ez < 0.25 * h)) {
             atomicOr(&colbad[col >> 5], 1u << (col & 31));
             continue;
         }
-        add(any_neg ? 1 : -1, (float)((d0 * v[8] + d1 * v[2] + d2 * v[5]) / (d0 + d1 + d2)));
+        const int sg = f0.s < 0 ? 1 : -1, z = above(zh);
+        atomicAdd(&colsum[col], sg);
+        if (z < dz) atomicAdd(&grid[voxel(z)], sg);
+        auto leave = [&](int k) { atomicOr(&unsure[word_of(L, x, y, k)], 1u << (x & 31)); };
+        for (int k = z; k < dz && height(k) - zh <= ez; ++k) leave(k);
+        for (int k = z - 1; k >= 0 && zh - height(k) <= ez; --k) leave(k);
     }
 }
 
@@ -375,7 +407,7 @@ const float* launch_caps(const float* tri9, long long T, const void* table, long
 
 size_t crossing_bytes(const Lattice& L) {
     const size_t cols = (size_t)L.dims[0] * L.dims[1];
-    return up256(cols * 4) + up256((cols + 31) / 32 * 4) + up256((size_t)L.nwords * 4);
+    return up256(cols * 4) + up256((cols + 31) / 32 * 4) + 2 * up256((size_t)L.nwords * 4);
 }
 
 Crossings launch_crossings(const float* tri9, long long T, const float* caps9, long long B, const Lattice& L,
@@ -384,21 +416,24 @@ Crossings launch_crossings(const float* tri9, long long T, const float* caps9, l
     char* p = static_cast<char*>(scratch);
     auto* colsum = reinterpret_cast<int*>(p);
     auto* colbad = reinterpret_cast<unsigned*>(p + up256(cols * 4));
-    auto* K = reinterpret_cast<uint32_t*>(p + up256(cols * 4) + up256((cols + 31) / 32 * 4));
-    cudaMemsetAsync(p, 0, up256(cols * 4) + up256((cols + 31) / 32 * 4), st);
+    const size_t zeroed = up256(cols * 4) + up256((cols + 31) / 32 * 4) + up256((size_t)L.nwords * 4);
+    auto* unsure = reinterpret_cast<uint32_t*>(p + up256(cols * 4) + up256((cols + 31) / 32 * 4));
+    auto* K = reinterpret_cast<uint32_t*>(p + zeroed);
+    cudaMemsetAsync(p, 0, zeroed, st);
     cudaMemsetAsync(grid, 0, (size_t)L.N * 4, st);
     auto cross = [&](const float* t9, long long n) {
         // few triangles are large ones: several warps share a triangle's columns
         const int slices = (int)std::max<long long>(1, std::min<long long>(64, 152ll * 64 / n));
         GBSDF_COUNT_LAUNCH();
-        crossings_kernel<<<(unsigned)((n * slices + 7) / 8), 256, 0, st>>>(t9, n, L, slices, grid, colsum, colbad);
+        crossings_kernel<<<(unsigned)((n * slices + 7) / 8), 256, 0, st>>>(t9, n, L, slices, grid, colsum, colbad,
+                                                                             unsure);
     };
     cross(tri9, T);
     if (B > 0) cross(caps9, B);
     const long long warps = (long long)L.wx * L.dims[1];
     GBSDF_COUNT_LAUNCH();
     crossing_bits_kernel<<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(grid, colsum, colbad, L, K);
-    return Crossings{K, colbad};
+    return Crossings{K, unsure, colbad};
 }
 
 }  // namespace gbsdf

@@ -408,8 +408,10 @@ __device__ __forceinline__ bool cell_far(const float4* __restrict__ cell, const 
 
 // Solid angle of a triangle in FP32, or in FP64 where FP32 cannot be trusted: the point's side of
 // the triangle is uncertain (as in solid_angle_fast's users), or the point is so near the
-// triangle's edges that the two terms of the angle's tangent cancel.
-__device__ __forceinline__ float tri_angle(const f3& p, const f3& v0, const f3& v1, const f3& v2) {
+// triangle's edges that the two terms of the angle's tangent cancel. CAPS: a point on the triangle, to
+// within FP64's rounding of its side, sets `near`.
+template <bool CAPS>
+__device__ __forceinline__ float tri_angle(const f3& p, const f3& v0, const f3& v1, const f3& v2, bool& near) {
     const float ax = v0.x - p.x, ay = v0.y - p.y, az = v0.z - p.z;
     const float bx = v1.x - p.x, by = v1.y - p.y, bz = v1.z - p.z;
     const float cx = v2.x - p.x, cy = v2.y - p.y, cz = v2.z - p.z;
@@ -424,16 +426,18 @@ __device__ __forceinline__ float tri_angle(const f3& p, const f3& v0, const f3& 
     const float labc = la * lb * lc;
     const float denom = __fmaf_rn(ca, lb, __fmaf_rn(bc, la, __fmaf_rn(ab, lc, labc)));
     if ((fabsf(det) < kCoplanarRel * labc && denom < 0.0f) || !(fabsf(det) + fabsf(denom) >= 0.01f * labc) ||
-        la <= 1e-6f || lb <= 1e-6f || lc <= 1e-6f)
-        return (float)solid_angle_f64(p, v0, v1, v2);
+        la <= 1e-6f || lb <= 1e-6f || lc <= 1e-6f) {
+        double det64, denom64, labc64;
+        const float angle = (float)solid_angle_f64(p, v0, v1, v2, det64, denom64, labc64);
+        if (CAPS) near |= fabs(det64) <= 1e-9 * labc64 && denom64 <= 1e-9 * labc64;
+        return angle;
+    }
     return 2.0f * atan2f(det, denom);
 }
 
-// A triangle's term: by its dipole when d > beta r, else the exact solid angle. CAPS: a point
-// within sqrt(near_sq) of the triangle sets `near`.
+// A triangle's term: by its dipole when d > beta r, else the exact solid angle.
 template <bool CAPS = false>
-__device__ __forceinline__ void leaf_term(const float4* __restrict__ leaf, const f3& p, float beta, Sum& a,
-                                          float near_sq = 0.0f) {
+__device__ __forceinline__ void leaf_term(const float4* __restrict__ leaf, const f3& p, float beta, Sum& a) {
     const float4 c0 = __ldg(leaf);
     const float dx = c0.x - p.x, dy = c0.y - p.y, dz = c0.z - p.z;
     const float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx));
@@ -447,10 +451,7 @@ __device__ __forceinline__ void leaf_term(const float4* __restrict__ leaf, const
     } else {
         const float4 u = __ldg(leaf + 2), v = __ldg(leaf + 3);
         const float w = __ldg(&leaf[4].x);
-        const f3 v0 = mk(u.x, u.y, u.z), v1 = mk(u.w, v.x, v.y), v2 = mk(v.z, v.w, w);
-        term = tri_angle(p, v0, v1, v2);
-        // (NaN, a triangle without area: a fan's first and last edges, which are the mesh's own)
-        if (CAPS) a.near |= ptd_sq(p, v0, v1, v2) <= near_sq;
+        term = tri_angle<CAPS>(p, mk(u.x, u.y, u.z), mk(u.w, v.x, v.y), mk(v.z, v.w, w), a.near);
     }
     kahan_add(a.s, a.c, term);
     a.mag += fabsf(term);
@@ -752,8 +753,9 @@ __device__ __forceinline__ int cta_list(int n, unsigned* list, int cap, unsigned
 
 // The marked voxels of the listed blocks (list null: of every block). Persistent CTAs.
 // CAPS: f holds the mesh's caps (k_caps.cu) and a voxel with |w(caps)| < 1/2 is inside iff its
-// bit of X.k is set, when its column is not left out and it lies farther than the ray's step
-// from the mesh and the caps; the others keep their marks.
+// bit of X.k is set, when neither it nor its column is left out and it lies on no cap; the
+// others keep their marks, and so do those next to the mesh, whose side the FP64 sum defines
+// where they are on it.
 // What bounds it: the FP32 work of the near clusters and triangles of dense bricks, and the
 // cluster tests of a block for sparse ones; nothing but a few bits a voxel goes to memory.
 template <int BB, bool CAPS>
@@ -793,8 +795,7 @@ __global__ void __launch_bounds__(kBqThreads) winding_blocks_kernel(
         // half the diagonal of the block's (brick's) points
         const float rho_b = (BB == 2 ? 12.9904f : 6.0622f) * L.h * 1.0002f + slop;
         const float rho = 6.0622f * L.h * 1.0002f + slop;
-        // CAPS: the ray's step (6.3e-4 h) and the rounding of positions and distances
-        const float step = 7e-4f * L.h + 2.0f * slop, step_sq = step * step;
+        const float next = 7e-4f * L.h + 2.0f * slop, next_sq = next * next;  // CAPS: "next to the mesh"
         int n2, n1 = 0;
         {
             Local a{};
@@ -851,7 +852,8 @@ __global__ void __launch_bounds__(kBqThreads) winding_blocks_kernel(
                         pend = false;
                     } else if (CAPS) {
                         const size_t col = (size_t)y * L.dims[0] + x;
-                        if (!(dist_sq ? (d > step_sq) : (d > step)) || ((X.bad[col >> 5] >> (col & 31)) & 1u)) {
+                        if (!(dist_sq ? (d > next_sq) : (d > next)) || ((X.bad[col >> 5] >> (col & 31)) & 1u) ||
+                            ((X.unsure[word_of(L, x, y, z)] >> (x & 31)) & 1u)) {
                             atomicOr(&s_keep[v >> 5], 1u << (v & 31));
                             pend = false;
                         }
@@ -916,7 +918,7 @@ __global__ void __launch_bounds__(kBqThreads) winding_blocks_kernel(
                             }
                             const long long t0 = (long long)k * kFwnLeaf;
                             const int m = (int)min((long long)kFwnLeaf, f.T - t0);
-                            for (int t = 0; t < m; ++t) leaf_term<CAPS>(f.leaf + 5 * (t0 + t), p, beta, a, step_sq);
+                            for (int t = 0; t < m; ++t) leaf_term<CAPS>(f.leaf + 5 * (t0 + t), p, beta, a);
                         }
                     }
                     __syncwarp();
