@@ -250,8 +250,8 @@ __global__ void __launch_bounds__(kStatThreads) fwn_leaf_kernel(const float* __r
         const double dx = (double)v[3 * q] - fg[0], dy = (double)v[3 * q + 1] - fg[1], dz = (double)v[3 * q + 2] - fg[2];
         rt2 = fmax(rt2, dx * dx + dy * dy + dz * dz);
     }
-    // the record's centroid is rounded to FP32; the dipole's first moment about it, at most
-    // a |g - fg|, is far below the rounding slack
+    // the record's centroid is rounded to FP32: the second moment is the one about it, the first
+    // one enters the bound where the dipole is used (leaf_term)
     const double qt = a * (l2 / 36.0 + off2);
     if (on) {
         float4* o = leaf + 5 * t;
@@ -445,9 +445,13 @@ __device__ __forceinline__ void leaf_term(const float4* __restrict__ leaf, const
     float term;
     if (d > beta * c0.w) {
         const float4 c1 = __ldg(leaf + 1);
-        term = __fmaf_rn(c1.z, dz, __fmaf_rn(c1.y, dy, c1.x * dx)) * ir * ir * ir;
+        const float ir3 = ir * ir * ir;
+        term = __fmaf_rn(c1.z, dz, __fmaf_rn(c1.y, dy, c1.x * dx)) * ir3;
         const float e = (d - c0.w) * 0.9999f, e2 = e * e;
-        a.err += __fdividef(3.0f * c1.w, e2 * e2);
+        // the record's centroid is off by up to 2^-24 of itself, and a first moment s from it adds at
+        // most 2 |D| |s| / d^3
+        const float g = fabsf(c0.x) + fabsf(c0.y) + fabsf(c0.z), D = fabsf(c1.x) + fabsf(c1.y) + fabsf(c1.z);
+        a.err += __fmaf_rn(1.2e-7f * g, D * ir3, __fdividef(3.0f * c1.w, e2 * e2));
     } else {
         const float4 u = __ldg(leaf + 2), v = __ldg(leaf + 3);
         const float w = __ldg(&leaf[4].x);
