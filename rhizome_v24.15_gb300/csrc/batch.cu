@@ -138,7 +138,8 @@ struct gbsdf_batch {
     std::vector<cudaEvent_t> joins;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    unsigned long long launches_per_run = 0;
+    unsigned long long launches_per_run = 0;  // recorded in the graph
+    unsigned long long launched = 0;          // by the current run: its graphs and from the host
     gbsdf::CapScratch cap_scratch;  // patch rounds: crossings and caps of one member at a time
     // learned mode: the network's parameters (device memory, the caller's), the proposal
     // threshold as a logit and the budget (0: 1/16 of each lattice's bricks)
@@ -388,6 +389,7 @@ int plan(gbsdf_batch& b, BErr& e) {
             if (ws_opt >= kWCpAsync && ws_opt <= kWTmaNarrow) j.wsched = j.wsched1 = ws_opt;
         }
     // counting pass
+    const unsigned long long counts0 = launch_counter();
     for (Job& j : b.jobs) {
         if (j.pre_status != GBSDF_OK) continue;
         if (!b.tris_dev) std::memcpy(j.hin, j.tris, (size_t)j.T * 48);
@@ -434,6 +436,7 @@ int plan(gbsdf_batch& b, BErr& e) {
                      cudaGetErrorString(cap_err != cudaSuccess ? cap_err : end_err));
     }
     b.launches_per_run = launch_counter() - l0;
+    b.launched += l0 - counts0;
     GBB_CK(cudaGraphInstantiate(&b.exec, b.graph, 0));
     return GBSDF_OK;
 }
@@ -510,8 +513,10 @@ int run_once(gbsdf_batch& b, bool& any_overflow, float& ms, BErr& e) {
     GBB_CK(cudaEventRecord(b.t0, b.origin));
     GBB_CK(cudaGraphLaunch(b.exec, b.origin));
     GBB_CK(cudaStreamSynchronize(b.origin));
+    const unsigned long long host0 = launch_counter();
     for (Job& j : b.jobs)
         if (j.pre_status == GBSDF_OK) GBB_CK(finish_job(b, j));
+    b.launched += b.launches_per_run + (launch_counter() - host0);
     GBB_CK(cudaEventRecord(b.t1, b.origin));
     GBB_CK(cudaStreamSynchronize(b.origin));
     GBB_CK(cudaEventElapsedTime(&ms, b.t0, b.t1));
@@ -665,6 +670,7 @@ int gbsdf_batch_run(gbsdf_batch* b, int32_t* statuses, gbsdf_stats* stats, char*
     GBB_CK(cudaSetDevice(b->device));
     bool overflow = false;
     float ms = 0.0f;
+    b->launched = 0;
     int rc = gbsdf::run_once(*b, overflow, ms, e);
     if (rc != GBSDF_OK) return rc;
     if (overflow) {  // new contents outgrew the planned lists: plan again, run again
@@ -681,7 +687,7 @@ int gbsdf_batch_run(gbsdf_batch* b, int32_t* statuses, gbsdf_stats* stats, char*
         const int s = gbsdf::status_of(*b, j, ov);
         if (s == GBSDF_OK && !b->out_dev) gbsdf::parallel_copy(j.out, j.hout, (size_t)j.L.N * 4);
         if (statuses) statuses[i] = s;
-        if (stats) gbsdf::fill_stats(j, s, ms, i == 0 ? b->launches_per_run : 0, &stats[i]);
+        if (stats) gbsdf::fill_stats(j, s, ms, i == 0 ? b->launched : 0, &stats[i]);
         if (s != GBSDF_OK && first == GBSDF_OK) {
             first = s;
             e.set(s, "mesh %zu failed with status %d", i, s);
