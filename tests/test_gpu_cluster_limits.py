@@ -18,7 +18,7 @@ def _soup(rng, flat, whole):
     return np.concatenate([t, np.zeros((flat + whole, 3))], 1).astype(np.float32)
 
 
-@pytest.mark.parametrize("flat,whole", [(8, 8), (8, 1), (8, 40), (64, 8), (1, 8), (128, 2048), (24, 0)])
+@pytest.mark.parametrize("flat,whole", [(8, 256), (8, 249), (8, 4000), (64, 200), (1, 256), (128, 2048), (264, 0)])
 def test_nearest_cluster_without_area(engine, flat, whole):
     tris = _soup(np.random.default_rng(7), flat, whole)
     mn, mx = (0, 0, 0), (37, 38, 36)
@@ -31,13 +31,14 @@ def test_nearest_cluster_without_area(engine, flat, whole):
 
 
 def _mixed(rng, n, reach):
-    """Clumps of triangles (a, a, c), whose distance exists on one side of them only, and of
-    ordinary triangles within `reach` of them."""
+    """Clumps of triangles (a, a, c), whose distance exists on one side of them only, of ordinary
+    triangles within `reach` of the lattice's middle part, and one of many at its far corner."""
     a = np.repeat(rng.uniform(8.0, 28.0, (n, 3)), 16, 0) + rng.uniform(-0.7, 0.7, (16 * n, 3))
     e = np.concatenate([a, a, a + rng.uniform(-0.9, 0.9, (16 * n, 3))], 1)
     c = np.repeat(rng.uniform(8.0, 28.0, (n, 3)), 8, 0)
     b = (c + rng.uniform(-reach, reach, (8 * n, 3)))[:, None] + rng.uniform(-1.0, 1.0, (8 * n, 3, 3))
-    t = np.concatenate([e, b.reshape(-1, 9)])
+    far = rng.uniform(33.0, 36.0, (256, 1, 3)) + rng.uniform(-0.3, 0.3, (256, 3, 3))  # so many that clusters are used
+    t = np.concatenate([e, b.reshape(-1, 9), far.reshape(-1, 9)])
     return np.concatenate([t, np.zeros((len(t), 3))], 1).astype(np.float32)
 
 
