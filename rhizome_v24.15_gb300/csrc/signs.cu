@@ -75,7 +75,7 @@ cudaError_t decide_marked(SignWork& w, uint32_t* E, bool patching) {
         const long long n = std::min<long long>((long long)w.hs->listed, w.cap);
         if (n <= 0) return cudaSuccess;
         if (w.fwn) {
-            if (!w.tried && w.hs->listed_voxels >= (unsigned long long)kCapsMinVoxels) SG_CK(make_capped(w));
+            if (!w.tried && w.hs->listed_voxels >= (unsigned long long)caps_min_voxels(w.L.N)) SG_CK(make_capped(w));
             if (w.capped)
                 launch_capped_blocks(w.capf, w.B, w.L, w.x, w.U, w.S, E, w.list, w.cap, only, w.dist, w.dist_sq, w.stol,
                                      w.ds, w.num_sms, w.st);
