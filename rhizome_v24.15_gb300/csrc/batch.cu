@@ -275,12 +275,20 @@ void enqueue_build(gbsdf_batch& b, Job& j, cudaStream_t st) {
     if (learned) cudaMemsetAsync(j.E, 0, (size_t)L.nwords * 4, st);
     // (a lattice of at most the list's capacity cannot leave more than the list holds)
     const long long passes = N <= j.list_cap ? 1 : std::min<long long>(64, (N + j.list_cap - 1) / j.list_cap + 1);
+    // the marks are not known here: at most half of the voxels are taken to be marked
+    const bool walks = by_voxels(N / 2, T);
     auto fixup_passes = [&](uint32_t* ebits) {
         for (long long p = 0; p < passes; ++p) {
             cudaMemsetAsync(&j.ds->listed, 0, kPassCounters, st);
-            launch_list_blocks(j.U, L, j.list, j.list_cap, j.ds, 0, st);
-            launch_winding_blocks(j.fwn, j.t9, T, L, j.U, j.S, ebits, j.list, j.list_cap, 0, j.recheck, j.list_cap,
-                                  j.A, 0, stol, j.ds, b.num_sms, st);
+            if (walks) {
+                launch_list_unknown(j.U, j.S, L, j.list, j.list_cap, j.ds, 0, st, ebits);
+                launch_winding(&j.fwn, j.t9, T, L, j.list, j.list_cap, kGwnFixup, 0, j.S, j.recheck, j.list_cap, j.A, 0,
+                               stol, j.ds, b.num_sms, st);
+            } else {
+                launch_list_blocks(j.U, L, j.list, j.list_cap, j.ds, 0, st);
+                launch_winding_blocks(j.fwn, j.t9, T, L, j.U, j.S, ebits, j.list, j.list_cap, 0, j.recheck, j.list_cap,
+                                      j.A, 0, stol, j.ds, b.num_sms, st);
+            }
             launch_gwn_recheck(j.t9, T, L, j.recheck, j.list_cap, kGwnFixup, j.S, j.ds, b.num_sms, st);
         }
     };

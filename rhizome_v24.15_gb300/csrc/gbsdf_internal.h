@@ -244,13 +244,11 @@ struct Crossings {
     const uint32_t* unsure;  // the voxels on a crossing, to leave out (the same layout)
     const unsigned* bad;     // the columns to leave out, a bit per column (x fastest)
 };
-// Marked voxels from which the pass pays off. It costs 0.07 ms and 2e-9 ms a voxel of the lattice (an
-// integer grid cleared and summed); the clusters alone 0.1 to 1.5 ms for the first few hundred
-// voxels, by the triangles near them, and more with each. Clusters alone / with the pass, ms (voxels
-// marked): vessel trees of 16k and 101k triangles on 64^3 0.17 / 0.25 (192) and 1.43 / 0.31 (448), on
-// 128^3 0.72 / 0.34 (3,840) and 1.73 / 0.33 (4,608); blob of 632k triangles on 64^3 3.8 / 0.64
-// (1,728), on 128^3 13.3 / 4.3 (22,656); 860 x 860 x 880 mug without three triangles 2.8 / 1.4 (11,440).
-constexpr long long caps_min_voxels(long long N) { return 256 + N / 65536; }
+// Marked voxels from which the pass can pay off. It costs 0.1 ms and 2e-9 ms a voxel of the lattice
+// (an integer grid cleared and summed), a voxel's own walk about 25e-6 ms. Walks / with the pass, ms
+// (voxels marked): 256^3 mug of 23k triangles 0.16 / 0.28 (2,048), 0.48 / 0.31 (7,168), 1.85 / 1.43
+// (55,808); vessel tree of 101k on 64^3 0.16 / 0.30 (448), on 128^3 0.46 / 0.32 (4,608).
+constexpr long long caps_min_voxels(long long N) { return 4096 + N / 16384; }
 size_t edge_table_bytes(long long T);
 void launch_edge_table(const float* tri9, long long T, void* table, cudaStream_t st);
 size_t caps_bytes(long long B);

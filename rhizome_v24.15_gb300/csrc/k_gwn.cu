@@ -34,6 +34,8 @@ __global__ void list_unknown_kernel(uint32_t* __restrict__ ubits, uint32_t* __re
     long long stride = (long long)gridDim.x * blockDim.x;
     for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < L.nwords; w += stride) {
         uint32_t u = ubits[w];
+        const int left = L.dims[0] - (int)(w % L.wx) * 32;  // the last word's pad bits are no voxels
+        if (left < 32) u &= (1u << left) - 1u;
         if (u == 0u) continue;
         int n = __popc(u);
         unsigned long long pos = atomicAdd(&ds->listed, (unsigned long long)n);
