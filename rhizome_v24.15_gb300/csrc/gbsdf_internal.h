@@ -224,7 +224,7 @@ void launch_nearest(const Fwn& f, long long T, const Lattice& L, float* d2, cuda
 // marked in U (DevState::listed; listed_voxels counts the marks); launch_winding_blocks
 // decides their marked voxels (U, S and E as launch_list_unknown treats them; a voxel that
 // finds no room in the leftover list stays marked and counts in list_overflow) and hands the
-// undecided ones to the refining stage and the exact sum. ubits null: every voxel.
+// undecided ones to the refining stage and the exact sum.
 void launch_list_blocks(const uint32_t* ubits, const Lattice& L, long long* list, long long cap, DevState* ds,
                         int only_if, cudaStream_t st);
 void launch_winding_blocks(const Fwn& f, const float* tri9, long long T, const Lattice& L, uint32_t* ubits,

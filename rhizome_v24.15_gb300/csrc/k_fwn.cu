@@ -564,7 +564,9 @@ constexpr int kBqCap0 = 2048;    // near clusters of a brick
 constexpr float kBqRatio = 0.25f; // largest brick radius / distance of a far cluster
 
 // A block's pending flags: BB = 2 (16^3 voxels) on large lattices, BB = 1 (8^3) where 16^3
-// blocks would be too few to fill the chip.
+// blocks would be too few to fill the chip, four an SM. Blocks of 16^3 / 8^3, every voxel, ms: watertight mug of 23k
+// triangles, mostly by its crossings, 120^3 (512 blocks) 0.39 / 0.29, 144^3 (729) 0.41 / 0.33, 160^3 (1,000)
+// 0.34 / 0.36, 256^3 0.89 / 1.00; by the clusters alone 120^3 26 / 12, 144^3 31 / 19, 256^3 131 / 116.
 __host__ __device__ inline long long block_count(const Lattice& L, int BB) {
     return (long long)((L.nb[0] + BB - 1) / BB) * ((L.nb[1] + BB - 1) / BB) * ((L.nb[2] + BB - 1) / BB);
 }
@@ -755,7 +757,7 @@ __device__ __forceinline__ int cta_list(int n, unsigned* list, int cap, unsigned
     return total;
 }
 
-// The marked voxels of the listed blocks (list null: of every block). Persistent CTAs.
+// The marked voxels of the listed blocks. Persistent CTAs.
 // CAPS: f holds the mesh's caps (k_caps.cu) and a voxel with |w(caps)| < 1/2 is inside iff its
 // bit of X.k is set, when neither it nor its column is left out and it lies on no cap; the
 // others keep their marks, and so do those next to the mesh, whose side the FP64 sum defines
@@ -776,21 +778,11 @@ __global__ void __launch_bounds__(kBqThreads) winding_blocks_kernel(
     const int tid = threadIdx.x, lane = tid & 31;
     const float tau = surf_tol_vox * L.h;
     const int gx = (L.nb[0] + BB - 1) / BB, gy = (L.nb[1] + BB - 1) / BB;
-    const long long nblk = list ? min((long long)ds->listed, cap) : block_count(L, BB);
+    const long long nblk = min((long long)ds->listed, cap);
     unsigned certified = 0, taken = 0;
     for (long long it = blockIdx.x; it < nblk; it += gridDim.x) {
-        const long long blk = list ? list[it] : it;
+        const long long blk = list[it];
         const int Bx = (int)(blk % gx) * BB, By = (int)(blk / gx % gy) * BB, Bz = (int)(blk / ((long long)gx * gy)) * BB;
-        if (U) {  // an earlier stage may have left no mark
-            constexpr int R = 8 * BB;
-            bool mine = false;
-            if (tid < R * R) {
-                const int y = By * 8 + tid % R, z = Bz * 8 + tid / R;
-                if (y < L.dims[1] && z < L.dims[2])
-                    mine = (U[((size_t)z * L.dims[1] + y) * L.wx + (Bx >> 2)] >> ((Bx * 8) & 31)) & ((1u << R) - 1u);
-            }
-            if (!__syncthreads_or(mine)) continue;
-        }
         // ---- the block: far clusters of the upper levels into its polynomial, the others listed
         const float bcx = lattice_mid(L.mn[0], Bx * 8, 4.0f * BB - 0.5f, L.h),
                     bcy = lattice_mid(L.mn[1], By * 8, 4.0f * BB - 0.5f, L.h),
@@ -827,7 +819,7 @@ __global__ void __launch_bounds__(kBqThreads) winding_blocks_kernel(
                 for (int r = 0; r < 4; ++r) {
                     const int y = by * 8 + ((tid * 4 + r) & 7), z = bz * 8 + ((tid * 4 + r) >> 3);
                     if (y >= L.dims[1] || z >= L.dims[2]) continue;
-                    const unsigned b = U ? U[((size_t)z * L.dims[1] + y) * L.wx + (bx >> 2)] >> shift : 0xffu;
+                    const unsigned b = U[((size_t)z * L.dims[1] + y) * L.wx + (bx >> 2)] >> shift;
                     m |= (b & row) << (8 * r);
                 }
                 s_mark[tid] = m;
@@ -980,7 +972,7 @@ __global__ void __launch_bounds__(kBqThreads) winding_blocks_kernel(
                 const unsigned in = (s_in[tid >> 2] >> (8 * (tid & 3))) & 0xffu;
                 if (done) {
                     const size_t w = ((size_t)(bz * 8 + (tid >> 3)) * L.dims[1] + by * 8 + (tid & 7)) * L.wx + (bx >> 2);
-                    if (U) atomicAnd(&U[w], ~(done << shift));
+                    atomicAnd(&U[w], ~(done << shift));
                     atomicAnd(&S[w], ~(done << shift));
                     if (in) atomicOr(&S[w], in << shift);
                     if (E) atomicOr(&E[w], done << shift);

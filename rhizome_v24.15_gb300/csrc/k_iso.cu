@@ -754,7 +754,7 @@ static int extract_iso(const float* grid, int32_t grid_on_device, const int32_t 
         return e.set(GBSDF_ECUDA, "cudaSetDevice failed");
     }
     const long long N = (long long)dx * dy * dz;
-    const long long groups = (long long)((dy + 3) / 4) * dz;
+    const long long groups = (long long)((dy + 3) / 4) * dz;  // the call's limit on dims: groups of four rows
     if (groups > 0x7fffffffLL) return e.set(GBSDF_EINVAL, "lattice too large (%lld row groups)", groups);
     const int wpr = (dx + 31) / 32;
     const IsoGeom G{dx, dy, dz, wpr, (long long)dy * dz, (long long)dy * dz * wpr, iso_value, iso_value + voxel_size,
