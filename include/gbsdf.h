@@ -130,9 +130,10 @@ typedef struct gbsdf_options {
     int32_t host_output;    /* host outputs: 0 = a page-locked output is written by the sign-apply
                                kernel through its device mapping (no staging copy), others are
                                staged in device memory and copied; 1 = always stage and copy */
-    int32_t winding_eval;   /* exact winding decisions: 0 = clustered (far clusters by a dipole
-                               with a rigorous error bound, undecided voxels summed exactly;
-                               same decisions), 1 = every voxel summed triangle by triangle */
+    int32_t winding_eval;   /* exact winding decisions: 0 = clustered (clusters of triangles by
+                               their moments, and crossings with caps over the mesh's boundary,
+                               with a rigorous error bound, undecided voxels summed exactly; same
+                               decisions), 1 = every voxel summed triangle by triangle */
     int32_t splat_dense_cut; /* binned triangles (eight to a cluster) per 8^3 brick above which the
                                 band splat takes the brick before the others, so that the longest
                                 work starts first: 0 = 256, > 0 = that cut

@@ -245,8 +245,8 @@ struct Crossings {
     const unsigned* bad;     // the columns to leave out, a bit per column (x fastest)
 };
 // Marked voxels from which the pass can pay off. It costs 0.1 ms and 2e-9 ms a voxel of the lattice
-// (an integer grid cleared and summed), a voxel's own walk about 25e-6 ms. Walks / with the pass, ms
-// (voxels marked): 256^3 mug of 23k triangles 0.16 / 0.28 (2,048), 0.48 / 0.31 (7,168), 1.85 / 1.43
+// (an integer grid cleared and summed), a voxel's own walk about 25e-6 ms. Walks / with the pass,
+// ms (voxels marked): 256^3 mug of 23k triangles 0.16 / 0.28 (2,048), 0.48 / 0.31 (7,168), 1.85 / 1.43
 // (55,808); vessel tree of 101k on 64^3 0.16 / 0.30 (448), on 128^3 0.46 / 0.32 (4,608).
 constexpr long long caps_min_voxels(long long N) { return 4096 + N / 16384; }
 size_t edge_table_bytes(long long T);

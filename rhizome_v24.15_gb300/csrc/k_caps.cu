@@ -8,8 +8,8 @@
 // triangles missing has a few caps for every hundred triangles, each as small as its hole.
 // Where |w(caps)| < 1/2, a voxel is inside (|w| >= 1/2) iff k != 0: one bit, read off the
 // crossings of its column. On the 512^3 vessel tree (2,062 triangles missing) it
-// decides all but a few thousand of 3.2M voxels; the fixup and the proposals' decisions fell
-// from 61 ms with the clusters alone to 15, on the 181 x 135 x 156 mug (watertight) from 29 to 0.6.
+// decides all but some hundred of 3.2M voxels; the fixup and the proposals' decisions fell
+// from 61 ms with the clusters alone to 12, on the 181 x 141 x 171 mug (watertight) from 29 to 0.4.
 //
 // The caps: unmatched edges from a table of position-keyed undirected edges (exact comparison
 // of the positions); connected components by union-find over the boundary's vertices (the

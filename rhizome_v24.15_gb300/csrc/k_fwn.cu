@@ -7,8 +7,8 @@
 // triangles themselves as the last one (a far triangle by its dipole, about a quarter of the
 // solid angle's work) leave the few triangles next to a voxel to the exact formula.
 //
-// A voxel-by-voxel query walks the levels for each voxel. Where whole bricks are asked for
-// (columns through holes, patch boxes, proposed bricks, the legacy path's every voxel) one CTA
+// A voxel-by-voxel query walks the levels for each voxel. Where many voxels are asked for (the
+// legacy path's every voxel, patch boxes, proposed bricks; signs.h has the line) one CTA
 // takes a block of BB^3 bricks instead and looks at the clusters in steps:
 //   * a cluster far from the block enters a polynomial about the block's centre;
 //   * the others are looked at again for each brick with marked voxels: far ones enter a
@@ -20,8 +20,8 @@
 // the per-triangle sum.
 //
 // Measured (voxels decided, before -> after, with k_caps.cu's pass in front): legacy path,
-// 181 x 135 x 156 mug, 3.8M voxels: 102 -> 0.56 ms; 512^3 vessel tree, 5,161 proposed bricks and
-// 0.52M fixup voxels: 160 -> 14 ms; 640^3 blob with holes, 3.96M fixup voxels: 307 -> 19 ms.
+// 181 x 141 x 171 mug, 4.4M voxels: 102 -> 0.4 ms; 512^3 vessel tree, 5,161 proposed bricks and
+// 0.52M fixup voxels: 160 -> 12 ms; 640^3 blob with holes, 3.96M fixup voxels: 307 -> 19 ms.
 #include <algorithm>
 
 #include "gwn_device.cuh"
@@ -467,8 +467,9 @@ __device__ __forceinline__ void leaf_term(const float4* __restrict__ leaf, const
 // time. What a walk leaves undecided is walked again with a wider near range (smaller truncation
 // bounds, more exact terms): beta0, 8, 32; then the voxel is handed to the sum over every
 // triangle. The blocks' leftovers start at 32: most come from 8 undecided (512^3 vessel tree, its
-// two queries 3.6 + 3.1 ms from 8, 3.1 + 3.0 from 16, 2.9 + 2.7 so; 640^3 blob 5.1, 6.1, 4.2). Latency-bound: a walk is a chain of some tens of
-// loads and ballots; the lists are short (4,096 probes, the block kernel's leftovers).
+// two queries 3.6 + 3.1 ms from 8, 3.1 + 3.0 from 16, 2.9 + 2.7 so; 640^3 blob 5.1, 6.1, 4.2).
+// Latency-bound: a walk is a chain of some tens of loads and ballots, and one of beta 32 some
+// thousand triangles long (29% of the issue slots).
 __global__ void __launch_bounds__(kQueryThreads) fwn_query_kernel(
     FwnView f, Lattice L, const long long* __restrict__ list, const unsigned long long* __restrict__ list_n,
     long long cap, int consumer, int only_if, uint32_t* __restrict__ sbits, const float* __restrict__ dist, int dist_sq,
@@ -564,9 +565,10 @@ constexpr int kBqCap0 = 2048;    // near clusters of a brick
 constexpr float kBqRatio = 0.25f; // largest brick radius / distance of a far cluster
 
 // A block's pending flags: BB = 2 (16^3 voxels) on large lattices, BB = 1 (8^3) where 16^3
-// blocks would be too few to fill the chip, four an SM. Blocks of 16^3 / 8^3, every voxel, ms: watertight mug of 23k
-// triangles, mostly by its crossings, 120^3 (512 blocks) 0.39 / 0.29, 144^3 (729) 0.41 / 0.33, 160^3 (1,000)
-// 0.34 / 0.36, 256^3 0.89 / 1.00; by the clusters alone 120^3 26 / 12, 144^3 31 / 19, 256^3 131 / 116.
+// blocks would be too few to fill the chip, four an SM. Blocks of 16^3 / 8^3, every voxel, ms:
+// watertight mug of 23k triangles, by its crossings, 120^3 (512 blocks) 0.39 / 0.29, 144^3 (729)
+// 0.41 / 0.33, 160^3 (1,000) 0.34 / 0.36, 256^3 0.89 / 1.00; by the clusters alone 120^3 26 / 12,
+// 144^3 31 / 19, 256^3 131 / 116.
 __host__ __device__ inline long long block_count(const Lattice& L, int BB) {
     return (long long)((L.nb[0] + BB - 1) / BB) * ((L.nb[1] + BB - 1) / BB) * ((L.nb[2] + BB - 1) / BB);
 }
@@ -1045,11 +1047,12 @@ __device__ __forceinline__ float walk_near(const FwnView& f, int level, int n, c
 // keeps, most is near none of its voxels. The tests are widened by the rounding of both sides, so the
 // minimum is that over all triangles. (Boxes, not spheres: a run of a mug wall's long
 // triangles is flat, and a voxel within its sphere's radius of the wall would keep it.)
-// Bound by the FP32 work of the tests and exact distances (57% of the issue slots, 24 lanes of
-// 32; 80 registers, three CTAs an SM: with the 97 the compiler takes, two, 3.5 ms below).
-// Replaces a walk of 128-triangle tiles in input order for each voxel: 181 x 135 x 156 mug,
-// 24,000 triangles, 56.5 -> 3.0 ms (3.4 without the pairs and the order); 48 x 48 x 52, 2,712
-// triangles, 0.72 -> 0.32 (0.46).
+// Bound by the FP32 work of the tests and exact distances (71% of the issue slots while active, 26
+// lanes of 32; 80 registers, three CTAs an SM: with the 97 the compiler takes, two, 3.5 ms below).
+// Replaces a walk of 128-triangle tiles in input order for each voxel: 181 x 141 x 171 mug,
+// 24,000 triangles, 56.5 -> 3.1 ms (3.4 without the pairs and the order); 48 x 48 x 52, 2,712
+// triangles, 0.72 -> 0.33 (0.46); where bricks are too crowded to list, 179,840 triangles, 215 x
+// 215 x 220 558 -> 43 and 48 x 48 x 52 20.5 -> 10.1.
 // One CTA a brick and no persistent loop: the bricks' work differs by more than ten times (on
 // a mug's axis the whole wall is equally near), and the hardware's own order balances it.
 __global__ void __launch_bounds__(kBqThreads, 3) nearest_bricks_kernel(FwnView f, Lattice L, float* __restrict__ d2out) {

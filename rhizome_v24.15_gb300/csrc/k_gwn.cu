@@ -16,8 +16,8 @@
 //  * every voxel whose FP32 |w| lies within 0.05 of 0.5 is re-evaluated in FP64 by a
 //    CTA (deterministic tree reduction), so each inside/outside decision is the
 //    exact-arithmetic one: inside iff |w| >= 0.5, the reference's rule;
-//  * the probe / patch control runs on the device (state in DevState), so the loop
-//    needs no host round trip per probe.
+//  * a probe's verdict and patch sites are found on the device (state in DevState); the host
+//    reads them once a probe and runs the patch rounds (signs.cu), which few builds need.
 #include "gwn_device.cuh"
 
 namespace gbsdf {

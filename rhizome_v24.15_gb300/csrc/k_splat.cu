@@ -400,9 +400,9 @@ __device__ __forceinline__ bool splat_admits(const float4* __restrict__ leaf, co
 // within its best so far; the tests are widened by the rounding of both sides. Fine meshes are
 // pruned by the cluster boxes, coarse ones by the masks and the triangle boxes. Bound by the
 // FP32 work of the box tests and exact distances. Against one exact distance per (voxel,
-// triangle binned to its brick), splat stage: 860 x 860 x 880 mug 9.8 -> 7.3 ms, 640^3 blob
-// 21.4 -> 9.2, 512^3 vessel tree 10.2 -> 3.9, 128^3 mug 1.0 -> 0.38; summed over the kernels of
-// a 16-mesh batch (2k to 150k triangles on 64^3 to 224^3) 27 -> 13 ms.
+// triangle binned to its brick), splat stage: 860 x 860 x 880 mug 9.8 -> 7.2 ms, 640^3 blob
+// 21.4 -> 9.4, 512^3 vessel tree 10.2 -> 4.0, 128^3 mug 1.0 -> 0.39; summed over the kernels of
+// a 16-mesh batch (2k to 150k triangles on 64^3 to 224^3) 27 -> 13.6 ms.
 __global__ void __launch_bounds__(kSplatThreads, 4) splat_kernel(FwnView f, const unsigned long long* __restrict__ off,
                                                                  const unsigned* __restrict__ cnt,
                                                                  const unsigned* __restrict__ list,

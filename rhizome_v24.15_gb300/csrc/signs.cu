@@ -36,10 +36,11 @@ namespace {
 // Makes the crossings and caps of the build. Two kinds of mesh keep to their own clusters: those whose
 // boundary is long (unwelded soups; more than one unmatched edge for every four triangles), whose
 // caps are wide fans over one another and decide little, and those with more than one cap for
-// every eight marked voxels, where a brick's caps cost more than its voxels' walks. So does a build that
-// finds no memory for them. Without / with them, ms: sphere of 10k triangles on 64^3, every voxel, 8% of the triangles
-// missing (0.24 unmatched edges a triangle) 0.9 / 0.9, 12% 1.7 / 2.8, 20% 1.6 / 7.8, 40% 1.4 / 31; of 88k and 352k
-// triangles, 8% missing, on 64^3, walks / caps and walks: 4.6 / 4.4 (13 voxels a cap), 6.9 / 11.6 (3.3).
+// every eight marked voxels, where a brick's caps cost more than its voxels' walks. So does a
+// build that finds no memory for them. Without / with them, ms, every voxel of 64^3: sphere of 10k triangles,
+// 8% missing (0.24 unmatched edges a triangle) 0.9 / 0.9, 12% 1.7 / 2.8, 20% 1.6 / 7.8, 40%
+// 1.4 / 31; of 88k and 352k triangles, 8% missing, walks / caps and walks: 4.6 / 4.4 (13 voxels a
+// cap), 6.9 / 11.6 (3.3).
 cudaError_t make_capped(SignWork& w, long long marks) {
     CapScratch& s = *w.scratch;
     if (!w.counted) {

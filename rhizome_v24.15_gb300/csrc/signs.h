@@ -45,11 +45,12 @@ struct SignWork {
 
 // Whether `marks` voxels of a mesh of T triangles are walked one by one rather than taken by blocks
 // of bricks. A block looks at its clusters once for all its voxels, which pays where they are many
-// and the triangles in a brick few. Blocks / walks, ms (voxels marked): in columns through holes, vessel trees
-// of 16k and 101k triangles 0.72 / 0.25 (3,840) and 1.73 / 0.45 (4,608), blob of 632k 13.2 / 1.3 (22,656) and
-// 15.8 / 12.2 (234,496), sphere of 71k without a fifth of its triangles 5.2 / 7.5 (355,968), of 287k
-// 35 / 12 (355,328) and 34 / 45 (1.5M); every voxel, sphere of 3k on 64^3 1.2 / 1.3 and on 96^3 2.5 / 4.5, of 90k
-// 27 / 4.6 and 9.0 / 16, of 360k 248 / 23 (96^3) and 103 / 218 (200^3).
+// and the triangles in a brick few. Blocks / walks, ms (voxels marked): in columns through holes,
+// vessel trees of 16k and 101k triangles 0.72 / 0.25 (3,840) and 1.73 / 0.45 (4,608), blob of 632k
+// 13.2 / 1.3 (22,656) and 15.8 / 12.2 (234,496), sphere of 71k without a fifth of its triangles
+// 5.2 / 7.5 (355,968), of 287k 35 / 12 (355,328) and 34 / 45 (1.5M); every voxel, sphere of 3k on
+// 64^3 1.2 / 1.3 and on 96^3 2.5 / 4.5, of 90k 27 / 4.6 and 9.0 / 16, of 360k 248 / 23 (96^3) and
+// 103 / 218 (200^3).
 inline bool by_voxels(long long marks, long long T) { return marks <= (4 * T > (1ll << 18) ? 4 * T : (1ll << 18)); }
 
 // Decides every voxel marked in U (its marks are cleared; E, when given, records them).
