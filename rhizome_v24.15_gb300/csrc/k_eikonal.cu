@@ -1697,10 +1697,11 @@ void launch_sweep_t(int axis, int round, const float* src, float* dst, const Lat
     GBSDF_COUNT_LAUNCH();
     // four lines per thread: 16-byte stores need an aligned destination (rows already are)
     if ((wsched == kWTmaVec || wsched == kWTmaVec2) && (reinterpret_cast<uintptr_t>(dst) & 15)) wsched = kWTmaPipe;
-    // packed pairs: the reference's update, at least two rows across the walk, and a voxel
-    // size whose square-root operands stay where nsqrt2_rn is exact
+    // packed pairs: the reference's update and a voxel size whose square-root operands stay where
+    // nsqrt2_rn is exact; the walk's also at least two voxels along x and two rows across it (its
+    // minima take no clamp, so a voxel needs a neighbour inside the lattice along each)
     const bool pair_ok = (RULE == 0) && pair_sqrt_ok(L.h);
-    if (wsched == kWTmaVec2 && (!pair_ok || (axis == 2 ? dy : dz) < 2)) wsched = kWTmaVec;
+    if (wsched == kWTmaVec2 && (!pair_ok || dx < 2 || (axis == 2 ? dy : dz) < 2)) wsched = kWTmaVec;
     if (axis != 0 && wsched == kWTmaNarrow) {
         const int n_rows = (axis == 2) ? dy : dz;
         dim3 grid((dx + kWX - 1) / kWX, (n_rows + kWNR - 1) / kWNR);
