@@ -40,8 +40,13 @@ constexpr float kSurfaceTolVoxels = 1e-5f;
 // voxels within 1e-3 voxel of the surface as on it.
 constexpr float kSurfaceTolExactSigns = 1e-3f;
 // A triangle term's sign is uncertain when |det| < this * |a||b||c| and the point
-// projects inside the triangle (denominator < 0): such voxels are decided in FP64.
+// projects inside the triangle (denominator < 0), and so is the angle itself next to an edge, where
+// both terms of its tangent cancel: such voxels are decided in FP64.
 constexpr float kCoplanarRel = 1e-4f;
+constexpr float kEdgeRel = 0.01f;  // (|det| + |denominator|) / |a||b||c|
+__device__ __forceinline__ bool angle_uncertain(float det, float denom, float labc) {
+    return (fabsf(det) < kCoplanarRel * labc && denom < 0.0f) || !(fabsf(det) + fabsf(denom) >= kEdgeRel * labc);
+}
 constexpr unsigned long long kFastMinVoxels = 32ull * 1024ull * 1024ull;
 
 // Brick edge of the band splat and lattice strip width of the parity pass.
@@ -120,7 +125,7 @@ __device__ __forceinline__ float solid_angle_fast(f3 p, f3 v0, f3 v1, f3 v2, boo
     float ca = __fmaf_rn(cz, az, __fmaf_rn(cy, ay, cx * ax));
     float labc = la * lb * lc;
     float denom = __fmaf_rn(ca, lb, __fmaf_rn(bc, la, __fmaf_rn(ab, lc, labc)));
-    amb |= (fabsf(det) < kCoplanarRel * labc) && (denom < 0.0f);
+    amb |= angle_uncertain(det, denom, labc);
     return 2.0f * atan2f(det, denom);
 }
 

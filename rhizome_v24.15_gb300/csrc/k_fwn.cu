@@ -406,9 +406,7 @@ __device__ __forceinline__ bool cell_far(const float4* __restrict__ cell, const 
     return true;
 }
 
-// Solid angle of a triangle in FP32, or in FP64 where FP32 cannot be trusted: the point's side of
-// the triangle is uncertain (as in solid_angle_fast's users), or the point is so near the
-// triangle's edges that the two terms of the angle's tangent cancel. CAPS: a point on the triangle, to
+// Solid angle of a triangle in FP32, or in FP64 where FP32 cannot be trusted. CAPS: a point on the triangle, to
 // within FP64's rounding of its side, sets `near`.
 template <bool CAPS>
 __device__ __forceinline__ float tri_angle(const f3& p, const f3& v0, const f3& v1, const f3& v2, bool& near) {
@@ -425,8 +423,7 @@ __device__ __forceinline__ float tri_angle(const f3& p, const f3& v0, const f3& 
     const float ca = __fmaf_rn(cz, az, __fmaf_rn(cy, ay, cx * ax));
     const float labc = la * lb * lc;
     const float denom = __fmaf_rn(ca, lb, __fmaf_rn(bc, la, __fmaf_rn(ab, lc, labc)));
-    if ((fabsf(det) < kCoplanarRel * labc && denom < 0.0f) || !(fabsf(det) + fabsf(denom) >= 0.01f * labc) ||
-        la <= 1e-6f || lb <= 1e-6f || lc <= 1e-6f) {
+    if (angle_uncertain(det, denom, labc) || la <= 1e-6f || lb <= 1e-6f || lc <= 1e-6f) {
         double det64, denom64, labc64;
         const float angle = (float)solid_angle_f64(p, v0, v1, v2, det64, denom64, labc64);
         if (CAPS) near |= fabs(det64) <= 1e-9 * labc64 && denom64 <= 1e-9 * labc64;
